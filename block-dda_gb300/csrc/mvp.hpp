@@ -5,6 +5,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "fx_fft.cuh"
 
 namespace bdda {
 
@@ -92,12 +93,21 @@ template <typename T> struct MvpPrec {
   const C* twz;
   const C* ghat;  // [Px][Py][6 or 9][Pz] (digit-reversed frequencies), divided by Px*Py*Pz
   const float4* twzp = nullptr;  // complex FP32: z twiddle pairs {wx, wx, wy, wy} (packed z pass)
-  // staged tables (stage_twiddles) of the compile-time-plan kernels: x, y, z
-  // (complex FP32), z pairs (packed z pass), z (double-float z pass)
+  // staged tables (stage_twiddles) of the compile-time-plan kernels: x, y, z, z pairs (packed z pass)
   const C* twxs = nullptr;
   const C* twys = nullptr;
   const C* twzs = nullptr;
   const float4* twzps = nullptr;
+};
+
+// Tables of the fixed-point MVP (FP64 and double-float, mvp_fx.cu): axis plans,
+// Q62 twiddles, and the Green spectrum [Px][Py][6 or 9][Pz] / (Px Py Pz) as Q62
+// over one power of two per (x, y) line.
+struct FxTables {
+  fx::Plan plan[3];
+  const fx::Fac* tw[3];
+  const fx::Fac* ghat;
+  const int* gexp;
 };
 
 // Timed kernel classes: the five MVP passes per precision (FP32 first), then
@@ -272,18 +282,33 @@ bool packed_z_available(int Pz, int f);
 // L (an autotuner candidate; the default rule also wants two CTAs per SM).
 bool pipe_z_available(int Pz, int f, int nzp, int L);
 
-// Pass C of a double-float block MVP (f = 3) with the compile-time z plan of
-// g.Pz; false (nothing launched) when g.Pz has none or f = 6.
-bool launch_pass_c_static_df(const MvpGeom& g, dfzc* t2, int L, const dfzc* twz, const dfzc* ghat, cudaStream_t st,
-                             const int* done, cudaError_t* err);
+// Workspace of the fixed-point MVP: T1 and T2 (16 bytes per element) and the
+// exponents of their lines: after pass A [f L][ny][nzp], after B and D
+// [f L][Px][nzp], after C [L][Px][Py], carved in that order from one array.
+struct FxWork {
+  void *t1, *t2;
+  int *ea, *eb, *ec;
+  static size_t exp_elems(const MvpGeom& g, int L) {
+    return (size_t)g.f * L * (g.ny + g.Px) * g.nzp + (size_t)L * g.Px * g.Py;
+  }
+  FxWork(void* t1_, void* t2_, int* e, const MvpGeom& g, int L)
+      : t1(t1_), t2(t2_), ea(e), eb(e + (size_t)g.f * L * g.ny * g.nzp), ec(eb + (size_t)g.f * L * g.Px * g.nzp) {}
+};
+// Block MVP in FP64 or double-float (df) storage of x, y, diag and jpre.
+cudaError_t launch_block_mvp_fx(const MvpGeom& g, const FxTables& t, bool df, const void* x, int ldx, void* y, int ldy, int L,
+                                const void* diag, const void* jpre, const FxWork& w, cudaStream_t st, KernelTimer* timer,
+                                const int* done = nullptr);
+// Forward 3-D transform in place of data[nc][Px][Py][Pz], and the packing of its result for the fixed-point MVP.
+cudaError_t fx_green_transform(double2* data, int nc, const FxTables& t, cudaStream_t st);
+cudaError_t fx_green_pack(const double2* data, int nc, const FxTables& t, fx::Fac* ghat, int* gexp, double scale, cudaStream_t st);
 
-// Green tensor: build Ghat (FP64 evaluation + FP64 3-D FFT), layout
-// [Px][Py][nc][Pz] with nc = 6 (g.f = 3) or 9 (g.f = 6), for any of the
-// precisions (null pointers skipped); the complex FP32 output in the z layout
-// gperm (green_pos), the others natural.  work: c128 [nc*Px*Py*Pz].
-cudaError_t build_green_hat(const MvpGeom& g, double lf, double k_re, double k_im,
-                            const double2* twx, const double2* twy, const double2* twz,
-                            double2* work, double2* ghat_d, float2* ghat_f, dfc* ghat_df, int gperm, cudaStream_t st);
+// Green tensor: build Ghat (FP64 evaluation, fixed-point 3-D FFT), layout
+// [Px][Py][nc][Pz] with nc = 6 (g.f = 3) or 9 (g.f = 6): ghat_f complex FP32 in
+// the frequency order of g's plans and the z layout g.gperm (green_pos), pos
+// [3][kMaxLine] mapping that order to the fixed-point plans' (null: skipped);
+// ghat_x / gexp for the fixed-point MVP (null: skipped).  work: c128 [nc*Px*Py*Pz].
+cudaError_t build_green_hat(const MvpGeom& g, double lf, double k_re, double k_im, const FxTables& t, double2* work,
+                            float2* ghat_f, const int* pos, fx::Fac* ghat_x, int* gexp, cudaStream_t st);
 
 // Radix schedule and shared-memory layout for a 5-smooth 2 <= N <= kMaxLine.
 // three: the fused z pass (three lines per warp), else the single-line tile
@@ -294,6 +319,12 @@ cudaError_t build_green_hat(const MvpGeom& g, double lf, double k_re, double k_i
 // prefers.  The skew shift and line pitch of both element widths come from the
 // same bank model (cached per plan).
 bool make_axis_plan(int N, AxisPlan* p, bool three, bool wide);
+// Plan of the fixed-point transforms (any 5-smooth 2 <= N <= kMaxLine), and its
+// Q62 twiddles: stage s, factor k = 1 .. R_s - 1, n1 < M_s at two[s] + (k - 1) M_s + n1.
+bool make_fx_plan(int N, fx::Plan* p);
+void make_fx_twiddles(const fx::Plan& p, std::vector<fx::Fac>* out);
+// Position in the fixed-point transform's output order of each position of plan a's (same length).
+void fx_positions(const AxisPlan& a, const fx::Plan& p, int* pos);
 // FP64 twiddle table exp(-2 pi i t / N), t < N.
 void make_twiddles(int N, std::vector<double2>* out);
 // Staged twiddle table of a plan, for the compile-time-plan kernels: stage s

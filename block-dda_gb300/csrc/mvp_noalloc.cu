@@ -6,7 +6,8 @@
 // own pool or arena, and latency-critical serving loops that must never enter
 // the CUDA allocator (cudaMalloc/cudaFree can synchronise the device).  This
 // variant runs the same five kernels with their two workspace buffers carved
-// out of one file-scope __device__ array of kNoAllocScratchBytes.  A GPU
+// out of one file-scope __device__ array of kNoAllocScratchBytes (plus the
+// FP64 path's line exponents).  A GPU
 // reserves that array when this file's device code is loaded on it -- under
 // CUDA's default lazy module loading, at the first call of the entry point
 // there -- and keeps it until the process exits.  Only complex FP64 and FP32
@@ -33,7 +34,10 @@ namespace {
 constexpr size_t kNoAllocScratchBytes = 64ull << 20;  // 64 MiB per device
 constexpr int kMaxDevices = 64;
 
-__device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratchBytes];
+// Line exponents of the FP64 workspace (FxWork), behind the two workspace buffers.  At 16 bytes an element they are at most
+// 1/8 of T1 (Px >= 2) and of T2 (Py >= 2) and, per right-hand side, 1/48 of T2 (f >= 3, nzp >= 4).
+constexpr size_t kNoAllocExpBytes = kNoAllocScratchBytes / 8 + kNoAllocScratchBytes / 48 + 256;
+__device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratchBytes + kNoAllocExpBytes];
 
 std::mutex g_scratch_mu;
 void* g_scratch_ptr[kMaxDevices] = {};
@@ -80,7 +84,7 @@ int mvp_noalloc(Op* op, const void* x, int ldx, void* y, int ldy, int L, const v
     set_error("bad L or leading dimension");
     return BDDA_ERR_INVALID;
   }
-  const MvpGeom g = op->geom<T>(o);
+  const MvpGeom g = op->geom(o);
   const size_t b1 = align256(mvp_t1_elems(g, L) * sizeof(C));
   const size_t b2 = align256(mvp_t2_elems(g, L) * sizeof(C));
   if (b1 + b2 > kNoAllocScratchBytes) {
@@ -94,9 +98,14 @@ int mvp_noalloc(Op* op, const void* x, int ldx, void* y, int ldy, int L, const v
   if (rc != BDDA_OK) return rc;
   C* t1 = static_cast<C*>(base);
   C* t2 = reinterpret_cast<C*>(static_cast<unsigned char*>(base) + b1);
-  const cudaError_t e = launch_block_mvp<T>(g, op->tables<T>(), static_cast<const C*>(x), ldx, static_cast<C*>(y), ldy, L,
-                                            static_cast<const C*>(diag), static_cast<const C*>(jpre), t1, t2, st,
-                                            nullptr, nullptr);
+  cudaError_t e;
+  if constexpr (std::is_same<T, float>::value)
+    e = launch_block_mvp<float>(g, op->tables32(), static_cast<const C*>(x), ldx, static_cast<C*>(y), ldy, L,
+                                static_cast<const C*>(diag), static_cast<const C*>(jpre), t1, t2, st, nullptr, nullptr);
+  else
+    e = launch_block_mvp_fx(g, op->tables_fx(), false, x, ldx, y, ldy, L, diag, jpre,
+                            FxWork(t1, t2, reinterpret_cast<int*>(static_cast<unsigned char*>(base) + b1 + b2), g, L), st, nullptr,
+                            nullptr);
   if (e != cudaSuccess) {
     set_error(std::string("no-allocation MVP launch: ") + cudaGetErrorString(e));
     return BDDA_ERR_CUDA;

@@ -82,12 +82,13 @@ Op::~Op() {
   solver.reset();
   for (auto* o : {&dip, &cub}) { o->occ.release(); o->tiles.release(); o->tmask.release(); }
   for (int i = 0; i < 3; ++i) {
-    tw64[i].release(); tw32[i].release(); twdf[i].release(); tw32p[i].release(); tws32[i].release();
+    tw32[i].release(); twfx[i].release(); tw32p[i].release(); tws32[i].release();
   }
-  tws32p.release(); twsdf.release();
-  ghat64.release(); ghat32.release(); ghatdf.release();
+  tws32p.release(); fxpos.release();
+  ghat32.release(); ghatfx.release(); gexpfx.release();
   kstat.release();
-  for (int i = 0; i < 3; ++i) { t1[i].release(); t2[i].release(); }
+  for (int i = 0; i < 2; ++i) { t1[i].release(); t2[i].release(); }
+  texp.release();
   if (stream) {
     wait_stream(stream);
     cudaStreamDestroy(stream);
@@ -276,20 +277,18 @@ int op_block_mvp(Op* op, const Occupancy& o, const typename cplx<T>::type* x, in
     set_error("bad L or leading dimension");
     return BDDA_ERR_INVALID;
   }
-  MvpGeom g = op->geom<T>(o);
-  const bool grow = op->t1[pi].bytes < mvp_t1_elems(g, L) * sizeof(C) || op->t2[pi].bytes < mvp_t2_elems(g, L) * sizeof(C);
+  MvpGeom g = op->geom(o);
+  const size_t eb = std::is_same<T, float>::value ? 0 : FxWork::exp_elems(g, L) * sizeof(int);
+  const bool grow = op->t1[pi].bytes < mvp_t1_elems(g, L) * sizeof(C) || op->t2[pi].bytes < mvp_t2_elems(g, L) * sizeof(C) ||
+                    op->texp.bytes < eb;
   if (grow && st != op->stream) BDDA_TRY_CUDA(order_after(op->stream, st));  // old buffers may be in use on st
   BDDA_CUDA(op->t1[pi].ensure(mvp_t1_elems(g, L) * sizeof(C), op->stream));
   BDDA_CUDA(op->t2[pi].ensure(mvp_t2_elems(g, L) * sizeof(C), op->stream));
+  if (eb) BDDA_CUDA(op->texp.ensure(eb, op->stream));
   if (grow && st != op->stream) BDDA_TRY_CUDA(order_after(st, op->stream));  // new buffers exist before st uses them
-  // the kernels' arithmetic: dfz (unrenormalised) for the double-float tables
-  using A = typename MvpArith<T>::type;
-  using CA = typename cplx<A>::type;
-  static_assert(sizeof(CA) == sizeof(C), "storage layouts agree");
-  const MvpPrec<T> tb = op->tables<T>();
-  MvpPrec<A> ta{(const CA*)tb.twx, (const CA*)tb.twy, (const CA*)tb.twz, (const CA*)tb.ghat, tb.twzp,
-                (const CA*)tb.twxs, (const CA*)tb.twys, (const CA*)tb.twzs, tb.twzps};
+  cudaError_t e;
   if constexpr (std::is_same<T, float>::value) {
+    const MvpPrec<float> ta = op->tables32();
     auto it = op->tuned.find(L);
     if (it != op->tuned.end()) {
       g.tune = it->second.tune;
@@ -315,9 +314,12 @@ int op_block_mvp(Op* op, const Occupancy& o, const typename cplx<T>::type* x, in
       }
     }
     if (op->zkern_force >= 0) g.tune.zkern = op->zkern_force;
+    e = launch_block_mvp<float>(g, ta, x, ldx, y, ldy, L, diag, jpre, op->t1[pi].as<float2>(), op->t2[pi].as<float2>(), st,
+                                &op->timer, done);
+  } else {
+    e = launch_block_mvp_fx(g, op->tables_fx(), std::is_same<T, dfl>::value, x, ldx, y, ldy, L, diag, jpre,
+                            FxWork(op->t1[pi].p, op->t2[pi].p, op->texp.as<int>(), g, L), st, &op->timer, done);
   }
-  cudaError_t e = launch_block_mvp<A>(g, ta, (const CA*)x, ldx, (CA*)y, ldy, L, (const CA*)diag, (const CA*)jpre,
-                                      op->t1[pi].as<CA>(), op->t2[pi].as<CA>(), st, &op->timer, done);
   if (e != cudaSuccess) return cuda_fail(e, "block MVP launch");
   return BDDA_OK;
 }
@@ -343,23 +345,14 @@ static int build_spectrum(Op* op, double k_re, double k_im) {
   DevBuf work;
   const size_t nc = f == 6 ? 9 : 6;  // Green components (symmetric A; f = 6 adds antisymmetric B)
   BDDA_CUDA(work.ensure(nc * ng * sizeof(double2), op->stream));
-  if (prec & BDDA_PREC_FP64) BDDA_CUDA(op->ghat64.ensure(nc * ng * sizeof(double2), op->stream));
-  if (prec & BDDA_PREC_FP32) BDDA_CUDA(op->ghat32.ensure(nc * ng * sizeof(float2), op->stream));
-  if (prec & BDDA_PREC_DF64) BDDA_CUDA(op->ghatdf.ensure(nc * ng * sizeof(dfc), op->stream));
-  // one spectrum per distinct digit order (radix sequences) of the plan sets
-  bool same = true;
-  for (int i = 0; i < 3; ++i) {
-    const AxisPlan &a = op->plan[0][i], &b = op->plan[1][i];
-    same = same && a.nst == b.nst && std::equal(a.radix, a.radix + a.nst, b.radix);
+  if (prec & (BDDA_PREC_FP64 | BDDA_PREC_DF64)) {
+    BDDA_CUDA(op->ghatfx.ensure(nc * ng * sizeof(fx::Fac), op->stream));
+    BDDA_CUDA(op->gexpfx.ensure((size_t)Px * Py * sizeof(int), op->stream));
   }
-  const double2 *tx = op->tw64[0].as<double2>(), *ty = op->tw64[1].as<double2>(), *tz = op->tw64[2].as<double2>();
-  const int gperm = green_perm_radix(f, op->plan[0][2]);  // FP32 / double-float spectra for the fused z pass
-  BDDA_CUDA(build_green_hat(op->geom(op->dip, 1), lf, k_re, k_im, tx, ty, tz, work.as<double2>(),
-                            op->ghat64.as<double2>(), same ? op->ghat32.as<float2>() : nullptr,
-                            op->ghatdf.as<dfc>(), gperm, op->stream));
-  if (!same && op->ghat32.p)
-    BDDA_CUDA(build_green_hat(op->geom(op->dip, 0), lf, k_re, k_im, tx, ty, tz, work.as<double2>(), nullptr,
-                              op->ghat32.as<float2>(), nullptr, gperm, op->stream));
+  if (prec & BDDA_PREC_FP32) BDDA_CUDA(op->ghat32.ensure(nc * ng * sizeof(float2), op->stream));
+  // one transform, packed for each precision in the order of its plans
+  BDDA_CUDA(build_green_hat(op->geom(op->dip), lf, k_re, k_im, op->tables_fx(), work.as<double2>(), op->ghat32.as<float2>(),
+                            op->fxpos.as<int>(), op->ghatfx.as<fx::Fac>(), op->gexpfx.as<int>(), op->stream));
   BDDA_CUDA(wait_stream(op->stream));
   op->kr = k_re;
   op->ki = k_im;
@@ -394,8 +387,7 @@ int bdda_op_create(bdda_op** out, const int n[3], int f, double lf, double k_re,
     op->n[i] = n[i];
     op->P[i] = smooth235(2 * n[i]);
     // z lines: the fused pass (three lines per warp); x / y: the tile passes
-    if (!make_axis_plan(op->P[i], &op->plan[0][i], i == 2, false) ||
-        !make_axis_plan(op->P[i], &op->plan[1][i], i == 2, true)) {
+    if (!make_axis_plan(op->P[i], &op->plan[i], i == 2, false) || !make_fx_plan(op->P[i], &op->fxplan[i])) {
       set_error("no FFT plan for the padded grid");
       return BDDA_ERR_INVALID;
     }
@@ -408,8 +400,11 @@ int bdda_op_create(bdda_op** out, const int n[3], int f, double lf, double k_re,
   for (int i = 0; i < 3; ++i) {
     std::vector<double2> tw;
     make_twiddles(op->P[i], &tw);
-    BDDA_CUDA(op->tw64[i].ensure(tw.size() * sizeof(double2), op->stream));
-    BDDA_CUDA(cudaMemcpyAsync(op->tw64[i].p, tw.data(), tw.size() * sizeof(double2), cudaMemcpyHostToDevice, op->stream));
+    std::vector<fx::Fac> tx;
+    make_fx_twiddles(op->fxplan[i], &tx);
+    if (tx.empty()) tx.push_back(fx::Fac{0, 0, 0, 0});
+    BDDA_CUDA(op->twfx[i].ensure(tx.size() * sizeof(fx::Fac), op->stream));
+    BDDA_CUDA(cudaMemcpyAsync(op->twfx[i].p, tx.data(), tx.size() * sizeof(fx::Fac), cudaMemcpyHostToDevice, op->stream));
     std::vector<float2> tf(tw.size());
     for (size_t t = 0; t < tw.size(); ++t) tf[t] = make_float2((float)tw[t].x, (float)tw[t].y);
     BDDA_CUDA(op->tw32[i].ensure(tf.size() * sizeof(float2), op->stream));
@@ -420,13 +415,9 @@ int bdda_op_create(bdda_op** out, const int n[3], int f, double lf, double k_re,
       BDDA_CUDA(op->tw32p[i].ensure(tp.size() * sizeof(float4), op->stream));
       BDDA_CUDA(cudaMemcpyAsync(op->tw32p[i].p, tp.data(), tp.size() * sizeof(float4), cudaMemcpyHostToDevice, op->stream));
     }
-    std::vector<dfc> td(tw.size());
-    for (size_t t = 0; t < tw.size(); ++t) td[t] = cmake(dfl(tw[t].x), dfl(tw[t].y));
-    BDDA_CUDA(op->twdf[i].ensure(td.size() * sizeof(dfc), op->stream));
-    BDDA_CUDA(cudaMemcpyAsync(op->twdf[i].p, td.data(), td.size() * sizeof(dfc), cudaMemcpyHostToDevice, op->stream));
-    // staged tables of the complex FP32 compile-time-plan kernels (plan set 0)
+    // staged tables of the complex FP32 compile-time-plan kernels
     std::vector<double2> ts;
-    stage_twiddles(op->plan[0][i], &ts);
+    stage_twiddles(op->plan[i], &ts);
     const size_t nts = std::max<size_t>(ts.size(), 1);
     std::vector<float2> tsf(nts, make_float2(1.f, 0.f));
     std::vector<float4> tsp(nts, make_float4(1.f, 1.f, 0.f, 0.f));
@@ -434,30 +425,27 @@ int bdda_op_create(bdda_op** out, const int n[3], int f, double lf, double k_re,
       tsf[t] = make_float2((float)ts[t].x, (float)ts[t].y);
       tsp[t] = make_float4(tsf[t].x, tsf[t].x, tsf[t].y, tsf[t].y);
     }
-    // the double-float z pass runs the 16-byte z table's plan (plan set 1)
-    std::vector<double2> tsw;
-    stage_twiddles(op->plan[1][i], &tsw);
-    const size_t ntw = std::max<size_t>(tsw.size(), 1);
-    std::vector<dfc> tsd(ntw, cmake(dfl(1.0), dfl(0.0)));
-    for (size_t t = 0; t < tsw.size(); ++t) tsd[t] = cmake(dfl(tsw[t].x), dfl(tsw[t].y));
     BDDA_CUDA(op->tws32[i].ensure(nts * sizeof(float2), op->stream));
     BDDA_CUDA(cudaMemcpyAsync(op->tws32[i].p, tsf.data(), nts * sizeof(float2), cudaMemcpyHostToDevice, op->stream));
     if (i == 2) {
       BDDA_CUDA(op->tws32p.ensure(nts * sizeof(float4), op->stream));
       BDDA_CUDA(cudaMemcpyAsync(op->tws32p.p, tsp.data(), nts * sizeof(float4), cudaMemcpyHostToDevice, op->stream));
-      BDDA_CUDA(op->twsdf.ensure(ntw * sizeof(dfc), op->stream));
-      BDDA_CUDA(cudaMemcpyAsync(op->twsdf.p, tsd.data(), ntw * sizeof(dfc), cudaMemcpyHostToDevice, op->stream));
     }
     BDDA_CUDA(wait_stream(op->stream));  // tw / tf / ts die at the end of this iteration
+  }
+  {
+    std::vector<int> pos(3 * kMaxLine, 0);
+    for (int i = 0; i < 3; ++i) fx_positions(op->plan[i], op->fxplan[i], pos.data() + i * kMaxLine);
+    BDDA_CUDA(op->fxpos.ensure(pos.size() * sizeof(int), op->stream));
+    BDDA_CUDA(cudaMemcpyAsync(op->fxpos.p, pos.data(), pos.size() * sizeof(int), cudaMemcpyHostToDevice, op->stream));
+    BDDA_CUDA(wait_stream(op->stream));  // pos dies here
   }
   {
     // kernel attributes sized for the largest line, so every live operator fits; once per process
     static std::once_flag once;
     static cudaError_t cfg = cudaSuccess;
     std::call_once(once, [] {
-      cfg = configure_mvp_kernels<double>();
-      if (cfg == cudaSuccess) cfg = configure_mvp_kernels<float>();
-      if (cfg == cudaSuccess) cfg = configure_mvp_kernels<dfz>();
+      cfg = configure_mvp_kernels<float>();
     });
     BDDA_CUDA(cfg);
   }

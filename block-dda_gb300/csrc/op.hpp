@@ -83,23 +83,25 @@ struct Op {
   int f = 3;
   double lf = 0, kr = 0, ki = 0;
   int prec = 0;  // bit mask BDDA_PREC_FP64 | BDDA_PREC_FP32
-  // Axis plans per element width: [0] complex FP32 (the compile-time plan
-  // tables' radix sequences, first-stage radices up to 32 along z), [1]
-  // 16-byte FP64 / double-float (the 16-byte z table, radices <= 8 on the
-  // single-line x / y axes).  Each set has its own Green spectrum order.
-  AxisPlan plan[2][3];
-  DevBuf tw64[3], tw32[3], twdf[3];
+  // Axis plans of the complex FP32 MVP (the compile-time plan tables' radix
+  // sequences, first-stage radices up to 32 along z) and of the fixed-point
+  // one (FP64 and double-float, mvp_fx.cu).  Each has its own spectrum order.
+  AxisPlan plan[3];
+  fx::Plan fxplan[3];
+  DevBuf tw32[3], twfx[3];
+  DevBuf fxpos;     // int [3][kMaxLine]: the complex FP32 order's positions in the fixed-point order
   DevBuf tw32p[3];  // complex FP32 twiddle pairs {wx, wx, wy, wy} of the packed z pass ([2] only)
   // staged twiddles (stage_twiddles) of the compile-time-plan kernels: complex
-  // FP32 per axis, the packed z pass's pairs, the double-float z pass.  Every
-  // DevBuf of the operator is released in ~Op, before its stream is destroyed.
-  DevBuf tws32[3], tws32p, twsdf;
-  DevBuf ghat64, ghat32, ghatdf;
+  // FP32 per axis, the packed z pass's pairs.  Every DevBuf of the operator is
+  // released in ~Op, before its stream is destroyed.
+  DevBuf tws32[3], tws32p;
+  DevBuf ghat32, ghatfx, gexpfx;  // Green spectra: complex FP32; Q62 with its exponents
   DevBuf kstat;     // int: status word of the pipelined z pass (take_kernel_status)
   Occupancy dip;    // dipole occupancy (set_dipoles)
   unsigned long long dip_epoch = 0;  // bumped whenever dip is rebuilt (captured MVPs hold its sizes)
   Occupancy cub;    // every cuboid site (the reference's MBT_fft_mvp vector)
-  DevBuf t1[3], t2[3];   // MVP workspace per precision (0 = FP64, 1 = FP32, 2 = double-float)
+  DevBuf t1[2], t2[2];   // MVP workspace (0 = FP64 and double-float, 1 = FP32)
+  DevBuf texp;           // line exponents of workspace 0 (FxWork)
   cudaStream_t stream = nullptr;
   KernelTimer timer;
   std::mutex mu;
@@ -119,23 +121,25 @@ struct Op {
   // signature of every buffer a block MVP's kernels are launched with
   unsigned long long buffer_sig() const {
     unsigned long long h = 0;
-    for (int i = 0; i < 3; ++i) {
-      for (const DevBuf* b : {&tw64[i], &tw32[i], &twdf[i], &tw32p[i], &tws32[i], &t1[i], &t2[i]}) h = sig_add(h, *b);
-    }
-    for (const DevBuf* b : {&ghat64, &ghat32, &ghatdf, &tws32p, &twsdf, &kstat, &dip.occ, &dip.tiles, &dip.tmask})
+    for (int i = 0; i < 3; ++i)
+      for (const DevBuf* b : {&tw32[i], &twfx[i], &tw32p[i], &tws32[i]}) h = sig_add(h, *b);
+    for (int i = 0; i < 2; ++i)
+      for (const DevBuf* b : {&t1[i], &t2[i]}) h = sig_add(h, *b);
+    for (const DevBuf* b : {&texp, &ghat32, &ghatfx, &gexpfx, &tws32p, &kstat, &dip.occ, &dip.tiles, &dip.tmask})
       h = sig_add(h, *b);
     return h;
   }
 
-  MvpGeom geom(const Occupancy& o, int set) const {
+  // gperm: the complex FP32 Green spectrum is in the fused z pass's layout
+  MvpGeom geom(const Occupancy& o) const {
     MvpGeom g;
     g.f = f;
     g.nx = n[0]; g.ny = n[1]; g.nz = n[2];
     g.nzp = (n[2] + 3) & ~3;  // 32-byte rows of complex FP32: aligned tile segments and column pairs
     g.Px = P[0]; g.Py = P[1]; g.Pz = P[2];
-    g.px = plan[set][0]; g.py = plan[set][1]; g.pz = plan[set][2];
+    g.px = plan[0]; g.py = plan[1]; g.pz = plan[2];
     g.nzt = (n[2] + kTZ - 1) / kTZ;
-    g.gperm = 0;
+    g.gperm = green_perm_radix(f, plan[2]);
     g.kstat = kstat.as<int>();
     g.zstall = zstall;
     g.ntiles = o.ntiles;
@@ -145,38 +149,24 @@ struct Op {
     g.tmask = o.tmask.as<unsigned char>();
     return g;
   }
-  // complex FP32 tables: the Green spectrum is in the fused z pass's layout
-  // (green_perm_radix); FP64 and double-float keep the natural one
-  template <typename T> MvpGeom geom(const Occupancy& o) const {
-    MvpGeom g = geom(o, sizeof(T) == sizeof(float) ? 0 : 1);
-    g.gperm = sizeof(T) == sizeof(float) ? green_perm_radix(f, plan[0][2]) : 0;
-    return g;
+  MvpPrec<float> tables32() const {
+    return {tw32[0].as<float2>(), tw32[1].as<float2>(), tw32[2].as<float2>(), ghat32.as<float2>(), tw32p[2].as<float4>(),
+            tws32[0].as<float2>(), tws32[1].as<float2>(), tws32[2].as<float2>(), tws32p.as<float4>()};
   }
-  template <typename T> MvpPrec<T> tables() const;
+  FxTables tables_fx() const {
+    return {{fxplan[0], fxplan[1], fxplan[2]},
+            {twfx[0].as<fx::Fac>(), twfx[1].as<fx::Fac>(), twfx[2].as<fx::Fac>()},
+            ghatfx.as<fx::Fac>(),
+            gexpfx.as<int>()};
+  }
   ~Op();
 };
 
-template <> inline MvpPrec<double> Op::tables<double>() const {
-  return {tw64[0].as<double2>(), tw64[1].as<double2>(), tw64[2].as<double2>(), ghat64.as<double2>()};
-}
-template <> inline MvpPrec<float> Op::tables<float>() const {
-  return {tw32[0].as<float2>(), tw32[1].as<float2>(), tw32[2].as<float2>(), ghat32.as<float2>(), tw32p[2].as<float4>(),
-          tws32[0].as<float2>(), tws32[1].as<float2>(), tws32[2].as<float2>(), tws32p.as<float4>()};
-}
-template <> inline MvpPrec<dfl> Op::tables<dfl>() const {
-  return {twdf[0].as<dfc>(), twdf[1].as<dfc>(), twdf[2].as<dfc>(), ghatdf.as<dfc>(), nullptr,
-          nullptr, nullptr, twsdf.as<dfc>(), nullptr};
-}
-
-// Arithmetic of the block-MVP kernels for each table precision.
-template <typename T> struct MvpArith { using type = T; };
-template <> struct MvpArith<dfl> { using type = dfz; };
-
-// Workspace slot and precision bit of each arithmetic type.
+// Workspace slot and precision bit of each vector type (FP64 and double-float share the fixed-point MVP's workspace).
 template <typename T> struct PrecInfo;
 template <> struct PrecInfo<double> { static constexpr int slot = 0, bit = 1; };
 template <> struct PrecInfo<float> { static constexpr int slot = 1, bit = 2; };
-template <> struct PrecInfo<dfl> { static constexpr int slot = 2, bit = 4; };
+template <> struct PrecInfo<dfl> { static constexpr int slot = 0, bit = 4; };
 
 // Make stream 'later' wait for the work enqueued so far on 'earlier'.
 cudaError_t order_after(cudaStream_t later, cudaStream_t earlier);

@@ -258,6 +258,128 @@ bool make_axis_plan(int N, AxisPlan* p, bool three, bool wide) {
   return p->lw[0] <= kMaxLineWords && p->lw[1] <= kMaxLineWords;
 }
 
+// Cost of one radix-R butterfly stage per point, in SM clocks: 32 x 32 -> 64
+// multiplies at 32 per clock (butterfly constants, and 12 per twiddle product
+// unless it is the last stage), other instructions at 110, the shared-memory
+// round trip; times the idle lanes of a warp's NL N / R butterflies.
+static double fx_stage_cost(int N, int R, bool last) {
+  struct Row { int R; double wide, alu; };
+  static const Row rows[] = {{2, 0, 4}, {3, 2, 17}, {4, 0, 8}, {5, 6, 26}, {6, 2, 21}, {8, 1.5, 17}, {9, 9.3, 43}, {10, 6, 30}};
+  double wide = 0, alu = 0;
+  for (const Row& r : rows)
+    if (r.R == R) { wide = r.wide; alu = r.alu; }
+  const double tw = last ? 0.0 : (R - 1.0) / R;
+  double fill = 0;
+  for (int nl : {2, 3}) fill += 0.5 * 32.0 * std::ceil(nl * (N / R) / 32.0) / (nl * (double)(N / R));
+  return fill * ((wide + 12 * tw) / 32 + (alu + 16 * tw + 14) / 110 + 0.25);
+}
+
+static void fx_sequences(int rem, int lo, std::vector<int>& cur, std::vector<std::vector<int>>& out) {
+  if (rem == 1) { out.push_back(cur); return; }
+  for (int r : {2, 3, 4, 5, 6, 8, 9, 10}) {
+    if (r < lo || rem % r) continue;
+    cur.push_back(r);
+    fx_sequences(rem / r, r, cur, out);
+    cur.pop_back();
+  }
+}
+
+bool make_fx_plan(int N, fx::Plan* p) {
+  if (N < 2 || N > kMaxLine) return false;
+  std::vector<std::vector<int>> seqs;
+  std::vector<int> cur;
+  fx_sequences(N, 2, cur, seqs);  // ascending radices: the largest last, where no twiddles are needed
+  const std::vector<int>* best = nullptr;
+  double bc = 0;
+  for (const auto& s : seqs) {
+    if ((int)s.size() > fx::kMaxFxStages) continue;
+    double c = 0;
+    for (size_t i = 0; i < s.size(); ++i) c += fx_stage_cost(N, s[i], i + 1 == s.size());
+    if (!best || c < bc) { best = &s; bc = c; }
+  }
+  if (!best) return false;
+  *p = fx::Plan{};
+  p->N = N;
+  p->nst = (int)best->size();
+  int Ls = N, off = 0;
+  double grow = 1, early = 1;  // bound of a value after each butterfly and division, in units of the largest input
+  for (int s = 0; s < p->nst; ++s) {
+    const int R = (*best)[s];
+    p->radix[s] = R;
+    p->M[s] = Ls / R;
+    p->mM[s] = ((1 << 21) + p->M[s] - 1) / p->M[s];
+    p->mB[s] = ((1 << 21) + N / R - 1) / (N / R);
+    p->two[s] = off;
+    off += (R - 1) * p->M[s];
+    Ls = p->M[s];
+    grow *= R;
+    if (s + 1 < p->nst) early = std::max(early, grow);
+    if (s + 1 < p->nst) {
+      p->D += fx::flog2(R);
+      grow /= 1 << fx::flog2(R);
+    }
+  }
+  auto bits = [](double v) { return (int)std::ceil(std::log2(v) - 1e-9); };
+  p->early[0] = bits(early);
+  p->head[0] = bits(std::max(early, grow));
+  // the inverse divides before each butterfly: grows towards its end
+  p->early[1] = p->nst > 1 ? bits(grow / p->radix[0] * (1 << fx::flog2(p->radix[0]))) : 0;
+  p->head[1] = bits(grow);
+  p->Rl = best->back();
+  p->mRl = ((1 << 21) + p->Rl - 1) / p->Rl;
+  p->S = p->Rl | 1;
+  p->LW = (N / p->Rl * p->S) | 1;
+  return true;
+}
+
+void make_fx_twiddles(const fx::Plan& p, std::vector<fx::Fac>* out) {
+  out->clear();
+  // cos / sin of 2 pi t / N in extended precision, reduced to the first octant by integer symmetry
+  auto q62 = [](long double v) { return (long long)std::llroundl(v * 4611686018427387904.0L); };
+  auto factor = [&](long long t, long long N) {
+    const long long o = 8 * t / N;
+    const bool odd = o & 1;
+    const long long r = odd ? (o + 1) * N - 8 * t : 8 * t - o * N;  // angle (pi / 4) r / N past or before the octant's edge
+    const long double a = 0.785398163397448309615660845819875721L * (long double)r / (long double)N;
+    long double c = std::cos(a), s = std::sin(a);
+    if (odd) std::swap(c, s);
+    long double re, im;
+    switch ((o / 2) & 3) {
+      case 0: re = c; im = s; break;
+      case 1: re = -s; im = c; break;
+      case 2: re = -c; im = -s; break;
+      default: re = s; im = -c; break;
+    }
+    fx::Fac f;
+    fx::split(q62(re), f.rh, f.rl);
+    fx::split(q62(-im), f.ih, f.il);  // exp(-2 pi i t / N)
+    return f;
+  };
+  int Ls = p.N;
+  for (int s = 0; s < p.nst; ++s) {
+    const int R = p.radix[s], M = p.M[s];
+    for (int k = 1; k < R; ++k)
+      for (int n1 = 0; n1 < M; ++n1) out->push_back(factor((long long)k * n1, Ls));
+    Ls = M;
+  }
+}
+
+// Frequency held at output position q of a forward transform with the given radices.
+template <class P> static int freq_at(const P& p, int q) {
+  int k = 0, w = 1;
+  for (int s = 0; s < p.nst; ++s) {
+    k += w * (q / p.M[s]);
+    q %= p.M[s];
+    w *= p.radix[s];
+  }
+  return k;
+}
+void fx_positions(const AxisPlan& a, const fx::Plan& p, int* pos) {
+  std::vector<int> at(p.N);
+  for (int q = 0; q < p.N; ++q) at[freq_at(p, q)] = q;
+  for (int q = 0; q < a.N; ++q) pos[q] = at[freq_at(a, q)];
+}
+
 void make_twiddles(int N, std::vector<double2>* out) {
   out->resize(N);
   const double two_pi = 6.283185307179586476925286766559;
@@ -298,7 +420,9 @@ extern "C" {
 // Runs the device FFT core (one "lane") on a host line: forward (natural ->
 // digit-reversed) or inverse (digit-reversed -> natural, unnormalised).
 // data: N interleaved complex values; prec 1 = FP64, 2 = FP32, 3 = double-float arithmetic
-// (values are rounded to float and back).  nvalid in (0, N): the forward
+// (values are rounded to float and back), 4 = the fixed-point core of the FP64 and
+// double-float MVPs (its own schedule; the forward transform is pruned for 0 < nvalid <=
+// N / 2, the inverse gives the first N / 2 values, as the MVP's, and zeros after them).  nvalid in (0, N): the forward
 // transform reads only the first nvalid inputs and takes the rest as zero
 // (the pad slots hold poison values to prove it).  radix[0] > 8 on input: the
 // z-axis schedule, else the x / y one, each for the element width of prec;
@@ -306,6 +430,50 @@ extern "C" {
 // Green spectrum is transformed in FP64).  Returns the number of stages, or a
 // negative value for an unsupported N.  Radices are written to radix (<= 32).
 int bdda_host_fft_line(int N, int inverse, int prec, int nvalid, double* data, int* radix) {
+  if (prec == 4) {
+    bdda::fx::Plan fp;
+    if (!bdda::make_fx_plan(N, &fp)) return -1;
+    std::vector<bdda::fx::Fac> ft;
+    bdda::make_fx_twiddles(fp, &ft);
+    const bool prune = !inverse && nvalid > 0 && 2 * nvalid <= N;
+    const int n = prune ? nvalid : N;
+    const long long poison = 0x3fffffffffffffffll;
+    std::vector<bdda::fx::Val> s(fp.LW, bdda::fx::Val{poison, poison});
+    for (int i = 0; i < n; ++i)
+      s[fp.addr(i)] = bdda::fx::Val{bdda::fx::double_to_bits(data[2 * i]), bdda::fx::double_to_bits(data[2 * i + 1])};
+    auto largest = [&] {
+      int k = 0;
+      for (int i = 0; i < n; ++i)
+        k = std::max(k, std::max(bdda::fx::key(s[fp.addr(i)].x), bdda::fx::key(s[fp.addr(i)].y)));
+      return k;
+    };
+    int key = largest();
+    const bool tiny = bdda::fx::tiny(key);
+    if (tiny) {
+      for (int i = 0; i < n; ++i) s[fp.addr(i)] = bdda::fx::lift_tiny(s[fp.addr(i)]);
+      key = largest();
+    }
+    unsigned sum = 0;
+    for (int i = 0; i < n; ++i)
+      sum += bdda::fx::sum_unit(s[fp.addr(i)].x, key >> 20) + bdda::fx::sum_unit(s[fp.addr(i)].y, key >> 20);
+    bdda::fx::Scale sc = bdda::fx::make_scale(key, fp.headroom(inverse != 0, bdda::fx::sum_head(sum, n)));
+    if (tiny) sc.ebase -= 200;
+    const int rsh[1] = {sc.rsh0};
+    const bdda::fx::InArgs in{rsh, nullptr, 0};
+    int used[1] = {0};
+    if (inverse) bdda::fx::inverse<1, bdda::fx::kRaw, true>(s.data(), fp, ft.data(), 0, 1, N / 2, in, used);
+    else if (prune) bdda::fx::forward<1, bdda::fx::kRaw, true, true>(s.data(), fp, ft.data(), 0, 1, n, in, used);
+    else bdda::fx::forward<1, bdda::fx::kRaw, false, true>(s.data(), fp, ft.data(), 0, 1, N, in, used);
+    for (int i = 0; i < N; ++i) {
+      bdda::fx::Val v{0, 0};
+      if (!inverse || i < N / 2) v = bdda::fx::to_bits(s[fp.addr(i)], sc.ebase + fp.D, sc.bad);
+      data[2 * i] = bdda::fx::bits_to_double(v.x);
+      data[2 * i + 1] = bdda::fx::bits_to_double(v.y);
+    }
+    if (radix)
+      for (int i = 0; i < fp.nst; ++i) radix[i] = fp.radix[i];
+    return fp.nst;
+  }
   bdda::AxisPlan p;
   const bool three = radix && radix[0] > 8;
   const bool wide = (radix && radix[1] == 1) ? false : prec != 2;

@@ -41,28 +41,6 @@ bool dispatch_z(const MvpGeom& g, float2* t2, int L, const float2* twz, const fl
   return false;
 }
 
-// The double-float z pass of f = 3 operators with the 16-byte z table's
-// compile-time plans (the double-float Green spectrum is in their digit order).
-template <int PART>
-bool dispatch_z_df(const MvpGeom& g, dfzc* t2, int L, const dfzc* twz, const dfzc* ghat, cudaStream_t st,
-                   const int* done, cudaError_t* err) {
-  if (g.f != 3) return false;
-  switch (g.Pz) {
-#define BDDA_ZWPLAN(I, N, S, LW, ...)                                                                 \
-  case N:                                                                                             \
-    if constexpr ((I) % kParts == PART) {                                                             \
-      *err = zstatic::launch_f<sfft::Plan<N, S, LW, __VA_ARGS__>, false, dfzc>(g, t2, L, twz, ghat, st, done); \
-      return true;                                                                                    \
-    }                                                                                                 \
-    return false;
-#include "zwplans.inc"
-#undef BDDA_ZWPLAN
-    default:
-      break;
-  }
-  return false;
-}
-
 template <int PART>
 bool dispatch_tile(int pass, const TileArgs& a, cudaError_t* err) {
   if (pass == kTileA || pass == kTileE) {
