@@ -57,9 +57,11 @@ BDDA_FX_FN Fac ldfac(const Fac* p) {
 }
 BDDA_FX_FN Val add(Val a, Val b) { return {a.x + b.x, a.y + b.y}; }
 BDDA_FX_FN Val sub(Val a, Val b) { return {a.x - b.x, a.y - b.y}; }
-// 32 x 32 -> 64-bit product (and sum) as one instruction: from plain C++ the
-// compiler widens the factors and multiplies 64 x 64 (36 instead of 12
-// multiplies per complex product, 0.95 -> 0.51 clocks).
+// 32 x 32 -> 64-bit product as one instruction: from plain C++ the compiler
+// widens the factors and multiplies 64 x 64 (36 instead of 12 multiplies per
+// complex product, 0.95 -> 0.49 clocks).  Products are added with 64-bit adds:
+// the multiply-add form takes 2.75 slots of the multiplier pipe, which bounds
+// these kernels, instead of 2.
 BDDA_FX_FN long long mw(int a, int b) {
 #if defined(__CUDA_ARCH__)
   long long d;
@@ -67,15 +69,6 @@ BDDA_FX_FN long long mw(int a, int b) {
   return d;
 #else
   return (long long)a * b;
-#endif
-}
-BDDA_FX_FN long long mwadd(int a, int b, long long c) {
-#if defined(__CUDA_ARCH__)
-  long long d;
-  asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(d) : "r"(a), "r"(b), "l"(c));
-  return d;
-#else
-  return (long long)a * b + c;
 #endif
 }
 BDDA_FX_FN long long shl(long long v, int s) { return (long long)((unsigned long long)v << s); }
@@ -93,7 +86,7 @@ constexpr int lo_of(long long q) { return (int)q; }
 template <long long Q> BDDA_FX_FN long long mulk(long long v) {
   int h, l;
   split(v, h, l);
-  const long long c = mwadd(h, lo_of(Q), 1ll << 29) + mw(l, hi_of(Q));
+  const long long c = mw(h, lo_of(Q)) + mw(l, hi_of(Q)) + (1ll << 29);
   return shl(mw(h, hi_of(Q)), 2) + (c >> 30);
 }
 
@@ -104,8 +97,8 @@ template <int D, bool CJ> BDDA_FX_FN Val cmul(Val z, int rh, int rl, int ih, int
   split(z.y, yh, yl);
   const long long rnd = D >= 2 ? (1ll << 31) : (1ll << (29 + D));
   // real: x r -+ y i; imaginary: y r +- x i
-  const long long a = mwadd(xh, rl, rnd) + mw(xl, rh), b = mw(yh, il) + mw(yl, ih);
-  const long long c = mwadd(yh, rl, rnd) + mw(yl, rh), d = mw(xh, il) + mw(xl, ih);
+  const long long a = mw(xh, rl) + mw(xl, rh) + rnd, b = mw(yh, il) + mw(yl, ih);
+  const long long c = mw(yh, rl) + mw(yl, rh) + rnd, d = mw(xh, il) + mw(xl, ih);
   const long long e = mw(xh, rh), f = mw(yh, ih), g = mw(yh, rh), k = mw(xh, ih);
   const long long cr = CJ ? a + b : a - b, ci = CJ ? c - d : c + d;
   const long long mr = CJ ? e + f : e - f, mi = CJ ? g - k : g + k;
@@ -157,8 +150,8 @@ BDDA_FX_FN void rot5(long long a, long long b, long long& p, long long& q) {
   split(a, ah, al);
   split(b, bh, bl);
   constexpr int sh = hi_of(kS72), sl = lo_of(kS72), th = hi_of(kS36), tl = lo_of(kS36);
-  const long long c = mwadd(ah, sl, 1ll << 29) + mw(al, sh) + mw(bh, tl) + mw(bl, th);
-  const long long d = mwadd(ah, tl, 1ll << 29) + mw(al, th) + mw(bh, -sl) + mw(bl, -sh);
+  const long long c = mw(ah, sl) + mw(al, sh) + (mw(bh, tl) + mw(bl, th)) + (1ll << 29);
+  const long long d = mw(ah, tl) + mw(al, th) + (mw(bh, -sl) + mw(bl, -sh)) + (1ll << 29);
   p = shl(mw(ah, sh) + mw(bh, th), 2) + (c >> 30);
   q = shl(mw(ah, th) + mw(bh, -sh), 2) + (d >> 30);
 }

@@ -46,6 +46,17 @@ constexpr int kFxLines = kTZ / kFxWarps;       // lines per warp
 constexpr int kFxRows = kFxThreads / kTZ;      // rows a tile copy moves at once
 constexpr int kBadAlign = 1 << 24;             // stands in for the exponent of a line that is not finite
 
+// CTAs per SM the kernels are compiled for: registers against resident warps.
+// Measured at one CTA fewer / more: y passes N=16384, L=16 (Py=160) 1.97 /
+// 1.89 ms for both, N=65536, L=16 (Py=270, 43 KB of lines per CTA) 10.5 /
+// 10.9 ms; pass C 4.39 / 3.89 (Pz=150) and 20.4 / 20.9 ms (Pz=250, where only
+// two CTAs fit).  So the larger count where that many fit in shared memory.
+constexpr int kXMany = 6, kXFew = 5;  // passes A, B, D, E
+constexpr int kCMany = 3, kCFew = 2;  // pass C, f = 3
+constexpr int kCSix = 2;              // pass C, f = 6
+constexpr int kSmemPerSm = 228 * 1024, kSmemReserved = 1024;  // shared memory of an SM, and what each CTA takes of it beside its own
+bool fits(int ctas, int smem) { return ctas * (smem + kSmemReserved) <= kSmemPerSm; }
+
 __device__ __forceinline__ bool skip(const int* done) { return done && *(volatile const int*)done; }
 __device__ __forceinline__ int clog2(int n) { return n <= 1 ? 0 : 32 - __clz(n - 1); }
 __device__ __forceinline__ Val raw(double2 v) { return {__double_as_longlong(v.x), __double_as_longlong(v.y)}; }
@@ -153,8 +164,8 @@ __device__ __forceinline__ void fill_tile(Val* lines, const fx::Plan& p, const v
 }
 
 // ---------------------------------------------------------------- pass A
-template <class Io>
-__global__ void __launch_bounds__(kFxThreads)
+template <class Io, int MB>
+__global__ void __launch_bounds__(kFxThreads, MB)
 k_fx_a(const typename Io::E* __restrict__ x, int ldx, int nfield, int fpg, int fc, const int* __restrict__ occ,
        const int* __restrict__ tiles, int nx, int ny, int nz, int nzp, int nzt, fx::Plan p, const Fac* __restrict__ tw,
        Val* __restrict__ t1, int* __restrict__ ea, const int* done) {
@@ -204,8 +215,8 @@ k_fx_a(const typename Io::E* __restrict__ x, int ldx, int nfield, int fpg, int f
 }
 
 // ---------------------------------------------------------------- pass B / D
-template <bool INV>
-__global__ void __launch_bounds__(kFxThreads)
+template <bool INV, int MB>
+__global__ void __launch_bounds__(kFxThreads, MB)
 k_fx_y(const Val* __restrict__ src, Val* __restrict__ dst, const unsigned char* __restrict__ tmask, int fc, int Px, int ny,
        int nz, int nzp, int nzt, fx::Plan p, const Fac* __restrict__ tw, const int* __restrict__ ein, int* __restrict__ eout,
        const int* done) {
@@ -247,8 +258,8 @@ k_fx_y(const Val* __restrict__ src, Val* __restrict__ dst, const unsigned char* 
 }
 
 // ---------------------------------------------------------------- pass E
-template <class Io>
-__global__ void __launch_bounds__(kFxThreads)
+template <class Io, int MB>
+__global__ void __launch_bounds__(kFxThreads, MB)
 k_fx_e(const Val* __restrict__ t1, const int* __restrict__ ein, int nfield, int fpg, int fc, const int* __restrict__ occ,
        const int* __restrict__ tiles, int nx, int ny, int nz, int nzp, int nzt, fx::Plan p, const Fac* __restrict__ tw,
        const typename Io::E* __restrict__ x, int ldx, const typename Io::E* __restrict__ diag,
@@ -311,19 +322,18 @@ struct Acc {
   long long cr = 1ll << 29, ci = 1ll << 29, mr = 0, mi = 0;
   __device__ __forceinline__ void mad(const Fac& g, const Split& s) {
     using fx::mw;
-    using fx::mwadd;
-    cr = mwadd(s.xh, g.rl, cr) + mw(s.xl, g.rh) - (mw(s.yh, g.il) + mw(s.yl, g.ih));
-    mr = mwadd(s.xh, g.rh, mr) - mw(s.yh, g.ih);
-    ci = mwadd(s.xh, g.il, ci) + mw(s.xl, g.ih) + mw(s.yh, g.rl) + mw(s.yl, g.rh);
-    mi = mwadd(s.xh, g.ih, mi) + mw(s.yh, g.rh);
+    cr += (mw(s.xh, g.rl) + mw(s.xl, g.rh)) - (mw(s.yh, g.il) + mw(s.yl, g.ih));
+    mr += mw(s.xh, g.rh) - mw(s.yh, g.ih);
+    ci += (mw(s.xh, g.il) + mw(s.xl, g.ih)) + (mw(s.yh, g.rl) + mw(s.yl, g.rh));
+    mi += mw(s.xh, g.ih) + mw(s.yh, g.rh);
   }
   __device__ __forceinline__ void msub(const Fac& g, const Split& s) { mad(Fac{-g.rh, -g.rl, -g.ih, -g.il}, s); }
   __device__ __forceinline__ Val get() const { return {fx::shl(mr, 2) + (cr >> 30), fx::shl(mi, 2) + (ci >> 30)}; }
 };
 
 // One warp per (x = q, y = qy, rhs l): fc component lines, blockDim.x / 32 warps per CTA.
-template <bool SIX>
-__global__ void __launch_bounds__(kZWarps * 32)
+template <bool SIX, int MB>
+__global__ void __launch_bounds__(kZWarps * 32, MB)
 k_fx_c(Val* __restrict__ t2, int L, int Px, int Py, int nz, int nzp, fx::Plan p, const Fac* __restrict__ tw,
        const Fac* __restrict__ ghat, const int* __restrict__ gexp, const int* __restrict__ ein, int* __restrict__ eout,
        const int* done) {
@@ -544,14 +554,21 @@ cudaError_t configure() {
     auto set = [&](const void* k) {
       if (cfg == cudaSuccess) cfg = cudaFuncSetAttribute(k, attr, kZSmemMax);
     };
-    set((const void*)k_fx_a<Io64>);
-    set((const void*)k_fx_a<IoDf>);
-    set((const void*)k_fx_y<false>);
-    set((const void*)k_fx_y<true>);
-    set((const void*)k_fx_e<Io64>);
-    set((const void*)k_fx_e<IoDf>);
-    set((const void*)k_fx_c<false>);
-    set((const void*)k_fx_c<true>);
+    set((const void*)k_fx_a<Io64, kXMany>);
+    set((const void*)k_fx_a<IoDf, kXMany>);
+    set((const void*)k_fx_a<Io64, kXFew>);
+    set((const void*)k_fx_a<IoDf, kXFew>);
+    set((const void*)k_fx_y<false, kXMany>);
+    set((const void*)k_fx_y<true, kXMany>);
+    set((const void*)k_fx_y<false, kXFew>);
+    set((const void*)k_fx_y<true, kXFew>);
+    set((const void*)k_fx_e<Io64, kXMany>);
+    set((const void*)k_fx_e<IoDf, kXMany>);
+    set((const void*)k_fx_e<Io64, kXFew>);
+    set((const void*)k_fx_e<IoDf, kXFew>);
+    set((const void*)k_fx_c<false, kCMany>);
+    set((const void*)k_fx_c<false, kCFew>);
+    set((const void*)k_fx_c<true, kCSix>);
     set((const void*)k_fx_contig);
     set((const void*)k_fx_strided);
   });
@@ -588,11 +605,15 @@ cudaError_t launch(const MvpGeom& g, const FxTables& t, const void* xv, int ldx,
   auto begin = [&](int id) { if (timer) timer->begin(id, st); };
   auto end = [&](int id) { if (timer) timer->end(id, st); };
   begin(kPassA64);
-  k_fx_a<Io><<<xgrid, kFxThreads, fx_smem(px, kTZ * g.nx), st>>>(x, ldx, nfield, fpg, g.f, g.occ, g.tiles, g.nx, g.ny, g.nz,
+  const int asm_ = fx_smem(px, kTZ * g.nx), bsm = fx_smem(py, kTZ * g.ny), dsm = fx_smem(py, g.Py),
+            esm = fx_smem(px, kTZ * (g.nx + g.Px));
+  auto* ka = fits(kXMany, asm_) ? k_fx_a<Io, kXMany> : k_fx_a<Io, kXFew>;
+  ka<<<xgrid, kFxThreads, asm_, st>>>(x, ldx, nfield, fpg, g.f, g.occ, g.tiles, g.nx, g.ny, g.nz,
                                                                  g.nzp, g.nzt, px, t.tw[0], t1, w.ea, done);
   end(kPassA64);
   begin(kPassB64);
-  k_fx_y<false><<<ygrid, kFxThreads, fx_smem(py, kTZ * g.ny), st>>>(t1, t2, g.tmask, g.f, g.Px, g.ny, g.nz, g.nzp, g.nzt, py,
+  auto* kb = fits(kXMany, bsm) ? k_fx_y<false, kXMany> : k_fx_y<false, kXFew>;
+  kb<<<ygrid, kFxThreads, bsm, st>>>(t1, t2, g.tmask, g.f, g.Px, g.ny, g.nz, g.nzp, g.nzt, py,
                                                                     t.tw[1], w.ea, w.eb, done);
   end(kPassB64);
   begin(kPassC64);
@@ -601,20 +622,18 @@ cudaError_t launch(const MvpGeom& g, const FxTables& t, const void* xv, int ldx,
     const int wpc = z_warps_per_cta(per_warp);
     const long long ntask = (long long)g.Px * g.Py * L;
     const unsigned grid = (unsigned)((ntask + wpc - 1) / wpc);
-    if (g.f == 6)
-      k_fx_c<true><<<grid, wpc * 32, wpc * per_warp, st>>>(t2, L, g.Px, g.Py, g.nz, g.nzp, pz, t.tw[2], t.ghat, t.gexp, w.eb,
-                                                            w.ec, done);
-    else
-      k_fx_c<false><<<grid, wpc * 32, wpc * per_warp, st>>>(t2, L, g.Px, g.Py, g.nz, g.nzp, pz, t.tw[2], t.ghat, t.gexp, w.eb,
-                                                            w.ec, done);
+    auto* kc = g.f == 6 ? k_fx_c<true, kCSix> : fits(kCMany, wpc * per_warp) ? k_fx_c<false, kCMany> : k_fx_c<false, kCFew>;
+    kc<<<grid, wpc * 32, wpc * per_warp, st>>>(t2, L, g.Px, g.Py, g.nz, g.nzp, pz, t.tw[2], t.ghat, t.gexp, w.eb, w.ec, done);
   }
   end(kPassC64);
   begin(kPassD64);
-  k_fx_y<true><<<ygrid, kFxThreads, fx_smem(py, g.Py), st>>>(t2, t1, g.tmask, g.f, g.Px, g.ny, g.nz, g.nzp, g.nzt, py, t.tw[1],
+  auto* kd = fits(kXMany, dsm) ? k_fx_y<true, kXMany> : k_fx_y<true, kXFew>;
+  kd<<<ygrid, kFxThreads, dsm, st>>>(t2, t1, g.tmask, g.f, g.Px, g.ny, g.nz, g.nzp, g.nzt, py, t.tw[1],
                                                              w.ec, w.eb, done);
   end(kPassD64);
   begin(kPassE64);
-  k_fx_e<Io><<<xgrid, kFxThreads, fx_smem(px, kTZ * (g.nx + g.Px)), st>>>(t1, w.eb, nfield, fpg, g.f, g.occ, g.tiles, g.nx, g.ny,
+  auto* ke = fits(kXMany, esm) ? k_fx_e<Io, kXMany> : k_fx_e<Io, kXFew>;
+  ke<<<xgrid, kFxThreads, esm, st>>>(t1, w.eb, nfield, fpg, g.f, g.occ, g.tiles, g.nx, g.ny,
                                                                           g.nz, g.nzp, g.nzt, px, t.tw[0], x, ldx, diag, jpre,
                                                                           y, ldy, done);
   end(kPassE64);
