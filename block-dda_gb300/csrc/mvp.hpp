@@ -58,8 +58,8 @@ struct MvpTune {
   // three 8-warp CTAs fit, else scalar), 0 scalar, 1 packed, 2 pipelined (zpass_pipe.cuh)
   int zkern = -1;
   int ywaves = 4;    // passes B, D: grid of this many waves of the CTAs resident per SM
-  int ybuf = 2;      // passes B, D: tile buffers per CTA (2: prefetch the next task; 1: twice the CTAs)
-  int ybufd = 0;     // pass D's own buffers and waves when > 0 (the autotuner times it separately)
+  int ybuf = 2;      // passes B, D: buffers per CTA (2: the next task's rows are prefetched; 1: more CTAs)
+  int ybufd = 1;     // pass D's own buffers and waves when > 0 (the autotuner times it separately)
   int ywavesd = 0;
   int xcta = 10;     // passes A, E: aim at this many CTAs per SM (fields split into groups)
 };
@@ -93,9 +93,9 @@ template <typename T> struct MvpPrec {
   const C* twz;
   const C* ghat;  // [Px][Py][6 or 9][Pz] (digit-reversed frequencies), divided by Px*Py*Pz
   const float4* twzp = nullptr;  // complex FP32: z twiddle pairs {wx, wx, wy, wy} (packed z pass)
-  // staged tables (stage_twiddles) of the compile-time-plan kernels: x, y, z, z pairs (packed z pass)
+  // staged tables (stage_twiddles) of the compile-time-plan kernels: x, y pairs, z, z pairs (packed z pass)
   const C* twxs = nullptr;
-  const C* twys = nullptr;
+  const float4* twyps = nullptr;
   const C* twzs = nullptr;
   const float4* twzps = nullptr;
 };
@@ -234,8 +234,8 @@ struct TileArgs {
   const float2* jpre;
   float2* t1;
   float2* t2;
-  const float2* twx;
-  const float2* twy;
+  const float2* twx;   // staged x twiddles
+  const float4* twyp;  // staged y twiddle pairs {wx, wx, wy, wy}
   int sms;              // multiprocessors of the device
   cudaStream_t st;
   const int* done;

@@ -4,6 +4,7 @@
 #pragma once
 
 #include "tile_static.cuh"
+#include "ypass_cols.cuh"
 #include "zpass_packed.cuh"
 #include "zpass_pipe.cuh"
 #include "zpass_static.cuh"
@@ -63,7 +64,7 @@ bool dispatch_tile(int pass, const TileArgs& a, cudaError_t* err) {
 #define BDDA_YPLAN(I, N, S, LW, ...)                                                     \
   case N:                                                                                \
     if constexpr ((I) % kParts == PART) {                                                \
-      *err = tstatic::launch_y<sfft::Plan<N, S, LW, __VA_ARGS__>>(pass, a);              \
+      *err = ycol::launch<sfft::Plan<N, S, LW, __VA_ARGS__>>(pass, a);                   \
       return true;                                                                       \
     }                                                                                    \
     return false;

@@ -5,10 +5,10 @@
 // layout of the plan; every precision).  A CTA stages 8 z-columns (one line
 // per warp) of one tile in shared memory; forward transforms read only the
 // first nv inputs.
-// k_pass_a2i / k_pass_y2i / k_pass_e2i: compile-time plans (static_fft.cuh,
-// padded layout; complex FP32).  Each warp transforms two adjacent z-columns
-// at once, interleaved element by element in shared memory, so the padded
-// T1 / T2 rows are staged and stored one 16-byte column pair per copy;
+// k_pass_a2i / k_pass_e2i: compile-time plans (static_fft.cuh, padded layout;
+// complex FP32; the y passes are in ypass_cols.cuh).  Each warp transforms two
+// adjacent z-columns at once, interleaved element by element in shared memory,
+// so the padded T1 rows are stored and staged one 16-byte column pair per copy;
 // inverse transforms write only the first nv outputs.
 #pragma once
 
@@ -173,89 +173,9 @@ k_pass_y(const typename cplx<T>::type* __restrict__ src, typename cplx<T>::type*
   }
 }
 
-// ---------------------------------------------------------------- static-plan tiles
-// The complex FP32 passes with compile-time plans process 16 z-columns (y
-// passes) or 8 (x passes) per task as column pairs.
-constexpr int kTZ2 = 2 * kTZ;
-
 // ---------------------------------------------------------------- pass E
 // One CTA per listed (y, z-tile); loops over fields with the next field's
 // tile prefetched by cp.async; scatters the occupied sites.
-// ---------------------------------------------------------------- pass B / D, column pairs
-// Persistent CTAs over tasks (field, x, 16-column z tile); lines along y.
-// Warp w transforms columns 2w and 2w + 1 as one line pair interleaved
-// element by element in shared memory (sfft::stage_il), so the tile is
-// staged and stored one column pair -- 16 contiguous bytes, since rows are
-// padded to a multiple of 4 elements -- per copy (a copy per column left the
-// warps stalled on the shared-memory queue).  A pair whose second column is
-// row padding transforms it and never stores it.  NBUF = 2: the next task's
-// tile is prefetched by cp.async into the second buffer while the current one
-// is transformed; NBUF = 1: one buffer, so twice the CTAs fit on an SM
-// (the autotuner picks; N=65536, Py=270: 3.28 -> 2.57 ms forward with one
-// buffer, Py=160: 0.254 -> 0.267 ms).
-constexpr int kPairsY = kTZ2 / 2;
-constexpr int kRowStepP = kTileThreads / kPairsY;
-
-template <bool INV, class P, int NBUF = 2>
-__global__ void __launch_bounds__(kTileThreads)
-k_pass_y2i(const float2* __restrict__ src, float2* __restrict__ dst, const unsigned char* __restrict__ tmask, int ny,
-           int nz, int nzp, int nzt, int ntask, const float2* __restrict__ twy, const int* done) {
-  if (skip(done)) return;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  constexpr int Py = P::N, lw = P::LW;
-  float2* tile = reinterpret_cast<float2*>(smem_raw);  // [NBUF][kPairsY][lw][2]
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int nin = INV ? Py : ny;
-  const int nout = INV ? ny : Py;
-  const int nzt2 = (nz + kTZ2 - 1) / kTZ2;
-  const int tp = tid & (kPairsY - 1), ty = tid / kPairsY;  // column pair and first row of this thread
-  auto issue = [&](int task, int buf) {
-    const int zt2 = task % nzt2;
-    const int r = task / nzt2;  // f * Px + q
-    const int z = zt2 * kTZ2 + 2 * tp;
-    const bool zval = z < nz;
-    const float2* g = src + (size_t)r * nin * nzp + z + (size_t)ty * nzp;
-    const unsigned char* tm = tmask + (zval ? z / kTZ : 0) + (size_t)ty * nzt;
-    float2* lb = tile + (size_t)(buf * kPairsY + tp) * lw * 2;
-    for (int yy = ty; yy < nin; yy += kRowStepP, g += (size_t)kRowStepP * nzp, tm += (size_t)kRowStepP * nzt) {
-      const bool valid = zval && (INV || *tm);
-      cp_async<16>(lb + 2 * P::addr(yy), valid ? g : src, valid);
-    }
-    cp_commit();
-  };
-  int task = blockIdx.x;
-  if (NBUF == 2 && task < ntask) issue(task, 0);
-  for (int it = 0; task < ntask; ++it, task += gridDim.x) {
-    const int buf = NBUF == 2 ? (it & 1) : 0;
-    const int next = task + gridDim.x;
-    if (NBUF == 1) {
-      issue(task, 0);
-      cp_wait<0>();
-    } else if (next < ntask) {
-      issue(next, buf ^ 1);
-      cp_wait<1>();
-    } else {
-      cp_wait<0>();
-    }
-    __syncthreads();
-    float2* wl = tile + (size_t)(buf * kPairsY + warp) * lw * 2;
-    if (!INV) sfft::forward_il<P>(wl, twy, lane, ny);
-    else sfft::inverse_il<P>(wl, twy, lane, ny);
-    __syncthreads();
-    const int zt2 = task % nzt2;
-    const int r = task / nzt2;
-    const int z = zt2 * kTZ2 + 2 * tp;
-    if (z < nz) {
-      float4* ob = reinterpret_cast<float4*>(dst + (size_t)r * nout * nzp + z + (size_t)ty * nzp);
-      const unsigned char* tm = tmask + z / kTZ + (size_t)ty * nzt;
-      const float4* lb = reinterpret_cast<const float4*>(tile + (size_t)(buf * kPairsY + tp) * lw * 2);
-      for (int yy = ty; yy < nout; yy += kRowStepP, ob += (size_t)kRowStepP * nzp / 2, tm += (size_t)kRowStepP * nzt)
-        if (!INV || *tm) *ob = lb[P::addr(yy)];
-    }
-    __syncthreads();  // buffer 'buf' is the cp.async target of the next-but-one task (next task, NBUF = 1)
-  }
-}
-
 template <typename T, class Line>
 __global__ void __launch_bounds__(kTileThreads)
 k_pass_e(const typename cplx<T>::type* __restrict__ t1, int nfield, int fpg, int fc, const int* __restrict__ occ,
