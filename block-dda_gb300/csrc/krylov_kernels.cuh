@@ -12,6 +12,7 @@ namespace bdda {
 
 constexpr int kMaxL = 32;          // largest block width (nrhs) supported
 constexpr int kGramThreads = 256;
+constexpr int kGramSlices = 8;     // threads that share the rows of a sub-tile for one Gram entry, at most
 constexpr int kGramRows = 32;      // rows per shared-memory sub-tile
 constexpr int kRowRows = 64;       // rows per CTA of the row-transform kernel
 constexpr int kRowThreads = 256;   // its threads: kRowRows rows x 4 column groups
@@ -63,14 +64,25 @@ k_gram(const typename cplx<T>::type* __restrict__ A, int lda,
   if (ctl_skip(ctl)) return;
   __shared__ C sa[kMaxL][kGramRows + 1];
   __shared__ C sb[kMaxL][kGramRows + 1];
+  __shared__ P red[kGramThreads];
   const int tid = threadIdx.x;
   const int LL = L * L;
-  // entries owned by this thread: e = tid + k*256, k < 4  (L <= 32 -> LL <= 1024)
+  // Entry e of the LL (padded to a power of two E) and row slice sl of a thread.  With E < 256 the threads of an entry
+  // share a sub-tile's rows (L = 2, FP64: four threads walked 64 rows one after the other, 17.1 us; eight slices 7.2, 32 the
+  // same), with E > 256 a thread has up to four entries.
+  const int sh = LL <= 1 ? 0 : 32 - __clz(LL - 1);
+  const int nsl = sh < 8 ? min(kGramThreads >> sh, kGramSlices) : 1;
+  const int e0 = sh < 8 ? tid & ((1 << sh) - 1) : tid, sl = sh < 8 ? tid >> sh : 0;
+  int ei[4], ej[4];
   P acc[4], acc2[BOTH ? 4 : 1];
 #pragma unroll
-  for (int k = 0; k < 4; ++k) gp_zero(acc[k]);
-#pragma unroll
-  for (int k = 0; k < (BOTH ? 4 : 1); ++k) gp_zero(acc2[k]);
+  for (int k = 0; k < 4; ++k) {
+    const int e = e0 + k * kGramThreads;
+    gp_zero(acc[k]);
+    if (BOTH) gp_zero(acc2[BOTH ? k : 0]);
+    ej[k] = e / L;
+    ei[k] = e < LL && sl < nsl && (k == 0 || sh > 8) ? e - ej[k] * L : -1;
+  }
   const long long rows_per = ((long long)n + gridDim.x - 1) / gridDim.x;
   const long long r0 = (long long)blockIdx.x * rows_per;
   const long long r1 = min((long long)n, r0 + rows_per);
@@ -90,12 +102,10 @@ k_gram(const typename cplx<T>::type* __restrict__ A, int lda,
     __syncthreads();
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      const int e = tid + k * kGramThreads;
-      if (e < LL) {
-        const int i = e % L, j = e / L;
+      if (ei[k] >= 0) {
         C s = czero<C>(), s2 = czero<C>();
-        for (int rr = 0; rr < nr; ++rr) {
-          const C a = sa[i][rr], b = sb[j][rr];
+        for (int rr = sl; rr < nr; rr += nsl) {
+          const C a = sa[ei[k]][rr], b = sb[ej[k]][rr];
           s = CONJ ? cadd(s, cconjmul(a, b)) : cadd(s, cmul(a, b));
           if (BOTH) s2 = cadd(s2, cmul(a, b));
         }
@@ -105,12 +115,26 @@ k_gram(const typename cplx<T>::type* __restrict__ A, int lda,
     }
   }
   const int LLo = BOTH ? 2 * LL : LL;  // partial entries per CTA
+  P* out = partials + (size_t)blockIdx.x * LLo;
+  if (nsl > 1) {  // the slices' sums in a fixed tree
+#pragma unroll
+    for (int g = 0; g < (BOTH ? 2 : 1); ++g) {
+      __syncthreads();
+      red[tid] = g == 0 ? acc[0] : acc2[0];
+      __syncthreads();
+      for (int o = nsl >> 1; o > 0; o >>= 1) {
+        if (sl < o) gp_add(red[tid], red[tid + (o << sh)]);
+        __syncthreads();
+      }
+      if (sl == 0 && e0 < LL) out[g * LL + e0] = red[e0];
+    }
+    return;
+  }
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
-    const int e = tid + k * kGramThreads;
-    if (e < LL) {
-      partials[(size_t)blockIdx.x * LLo + e] = acc[k];
-      if (BOTH) partials[(size_t)blockIdx.x * LLo + LL + e] = acc2[BOTH ? k : 0];
+    if (ei[k] >= 0) {
+      out[e0 + k * kGramThreads] = acc[k];
+      if (BOTH) out[LL + e0 + k * kGramThreads] = acc2[BOTH ? k : 0];
     }
   }
 }

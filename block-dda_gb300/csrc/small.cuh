@@ -16,6 +16,8 @@
 // in global memory stay complex FP64 either way.
 #pragma once
 
+#include <type_traits>
+
 #include "common.cuh"
 #include "krylov_kernels.cuh"
 
@@ -32,10 +34,11 @@ template <> struct SmallMat<dfl> { using M = dfc; };
 // double-float (Dekker 1971; Hida, Li and Bailey 2001, "Algorithms for
 // quad-double precision floating point arithmetic").
 __device__ __forceinline__ dfl df_recip(dfl b) {
-  const float q1 = 1.0f / b.hi;
-  const dfl one(1.0f, 0.0f);
-  const dfl q = df_quick_two_sum(q1, (one - b * dfl(q1, 0.0f)).hi * q1);
-  return q + dfl((one - b * q).hi * q1, 0.0f);
+  const float q = __frcp_rn(b.hi);
+  // e = 1 - b q to about 2^-48 of 1 (the FMA of the leading part is exact but for its last rounding), then one Newton
+  // step with its second-order term: q (1 + e + e^2)
+  const float e = fmaf(-b.lo, q, fmaf(-b.hi, q, 1.0f));
+  return df_quick_two_sum(q, q * fmaf(e, e, e));
 }
 __device__ __forceinline__ dfl df_sqrt(dfl a) {
   if (!(a.hi > 0.0f)) return dfl(sqrtf(a.hi), 0.0f);  // zero, negative or NaN: the FP32 answer
@@ -49,31 +52,54 @@ __device__ __forceinline__ double r_recip(double a) { return 1.0 / a; }
 __device__ __forceinline__ dfl r_recip(dfl a) { return df_recip(a); }
 __device__ __forceinline__ double r_sqrt(double a) { return sqrt(a); }
 __device__ __forceinline__ dfl r_sqrt(dfl a) { return df_sqrt(a); }
-__device__ __forceinline__ bool r_gt(double a, double b) { return a > b; }
-__device__ __forceinline__ bool r_gt(dfl a, dfl b) { return a.hi > b.hi || (a.hi == b.hi && a.lo > b.lo); }
-__device__ __forceinline__ bool r_eq(double a, double b) { return a == b; }
-__device__ __forceinline__ bool r_eq(dfl a, dfl b) { return a.hi == b.hi && a.lo == b.lo; }
 __device__ __forceinline__ bool r_pos_finite(double a) { return a > 0.0 && isfinite(a); }
 __device__ __forceinline__ bool r_pos_finite(dfl a) { return a.hi > 0.0f && isfinite(a.hi) && isfinite(a.lo); }
 __device__ __forceinline__ double r_to_double(double a) { return a; }
-__device__ __forceinline__ double r_to_double(dfl a) { return df_to_double(a); }
-__device__ __forceinline__ double r_shfl_xor(double a, int o) { return __shfl_xor_sync(0xffffffffu, a, o); }
-__device__ __forceinline__ dfl r_shfl_xor(dfl a, int o) {
-  return dfl(__shfl_xor_sync(0xffffffffu, a.hi, o), __shfl_xor_sync(0xffffffffu, a.lo, o));
-}
+__device__ __forceinline__ double r_to_double(dfl a);
 template <typename R> __device__ __forceinline__ R r_const(float v) { return R(v); }
 template <> __device__ __forceinline__ dfl r_const<dfl>(float v) { return dfl(v, 0.0f); }
 
 __device__ __forceinline__ double2 m_to_double2(double2 a) { return a; }
-__device__ __forceinline__ double2 m_to_double2(dfc a) { return make_double2(df_to_double(a.x), df_to_double(a.y)); }
+// Double-float <-> FP64 with the values of dfl(v) and df_to_double(a), the conversions done on the bit patterns
+// (conversion instructions and FP64 additions issue at two per clock and SM).
+__device__ __forceinline__ dfl df_from_double(double v) {
+  const int h = __double2hiint(v);
+  const unsigned l = (unsigned)__double2loint(v);
+  const int e = (h >> 20) & 0x7ff;
+  if (e < 960 || e > 1140) return ((h << 1) | (int)l) == 0 ? dfl(0.0f, 0.0f) : dfl(v);
+  const int up = (int)((l >> 28) & 1u);  // the leading part is rounded to nearest (a tie away from zero)
+  const int r = (int)(l & 0x1fffffffu) - (up << 29);
+  const unsigned hb = ((unsigned)(e - 896) << 23 | ((unsigned)h & 0xfffffu) << 3 | l >> 29) + (unsigned)up;
+  const float lo = (float)r * __uint_as_float((unsigned)(e - 896 - 52) << 23);
+  const unsigned sg = (unsigned)h & 0x80000000u;
+  return dfl(__uint_as_float(hb | sg), __uint_as_float(__float_as_uint(lo) ^ sg));
+}
+__device__ __forceinline__ double d_from_float(float v) {
+  const unsigned b = __float_as_uint(v);
+  const unsigned e = (b >> 23) & 0xffu;
+  if (e == 0 || e == 0xff) return (b << 1) == 0 ? __hiloint2double((int)b, 0) : (double)v;
+  return __hiloint2double((int)((b & 0x80000000u) | ((e + 896) << 20) | ((b & 0x7fffffu) >> 3)), (int)(b << 29));
+}
+__device__ __forceinline__ double d_from_df(dfl a) { return d_from_float(a.hi) + d_from_float(a.lo); }
+__device__ __forceinline__ double r_to_double(dfl a) { return d_from_df(a); }
+__device__ __forceinline__ double2 m_to_double2(dfc a) { return make_double2(d_from_df(a.x), d_from_df(a.y)); }
 template <typename M> __device__ M m_from_double2(double2 a);
 template <> __device__ __forceinline__ double2 m_from_double2<double2>(double2 a) { return a; }
-template <> __device__ __forceinline__ dfc m_from_double2<dfc>(double2 a) { return cmake(dfl(a.x), dfl(a.y)); }
+template <> __device__ __forceinline__ dfc m_from_double2<dfc>(double2 a) { return cmake(df_from_double(a.x), df_from_double(a.y)); }
 
 template <typename M> __device__ __forceinline__ auto m_abs2(M a) { return a.x * a.x + a.y * a.y; }
 template <typename M> __device__ __forceinline__ M m_neg(M a) { return cmake(-a.x, -a.y); }
 template <typename M> __device__ __forceinline__ bool m_finite(M a) {
   return isfinite(r_to_double(a.x)) && isfinite(r_to_double(a.y));
+}
+// 1 / b; operands are O(1) pivots (no scaling against overflow)
+__device__ __forceinline__ double2 m_recip(double2 b) {
+  const double d = 1.0 / (b.x * b.x + b.y * b.y);
+  return make_double2(b.x * d, -b.y * d);
+}
+__device__ __forceinline__ dfc m_recip(dfc b) {
+  const dfl d = df_recip(b.x * b.x + b.y * b.y);
+  return cmake(b.x * d, -(b.y * d));
 }
 // a / b; operands are O(1) pivots (no scaling against overflow)
 __device__ __forceinline__ double2 m_div(double2 a, double2 b) {
@@ -93,70 +119,85 @@ __device__ __forceinline__ double cabs2(double2 a) { return a.x * a.x + a.y * a.
 __device__ __forceinline__ double2 cdiv(double2 a, double2 b) { return m_div(a, b); }
 __device__ __forceinline__ bool cfinite(double2 a) { return isfinite(a.x) && isfinite(a.y); }
 
-// dst[e] = sum over p of partials[p*LL + e] (complex FP64 partials).  16
-// independent accumulators (partial p goes to accumulator p mod 16), combined
-// in a fixed order: the loads of one round are in flight together and the
-// result is bitwise reproducible for a given nparts.
-template <typename R>
-__device__ void sm_reduce(typename SmallMat<R>::M* dst, const double2* __restrict__ partials, int nparts, int LL) {
-  constexpr int U = 16;
-  if (nparts == 1) {  // an already reduced matrix: convert only (FP64 adds are scarce on GB300)
-    for (int e = threadIdx.x; e < LL; e += blockDim.x) dst[e] = m_from_double2<typename SmallMat<R>::M>(__ldg(partials + e));
-    __syncthreads();
+// A Gram matrix as the row kernels leave it: n = 0: reduced, complex FP64 at p; else n partial matrices of type P (FP64 or
+// double-float), `stride` elements apart.
+struct GramRef {
+  const void* p;
+  int n, stride;
+};
+// dst = the matrix at element offset off.  Partials (LL <= 64, a separate reduction launch costs more than it saves there)
+// are summed by S threads per entry and a fixed tree.
+template <typename R, typename P>
+__device__ void sm_gram(typename SmallMat<R>::M* dst, GramRef g, int off, int LL) {
+  using M = typename SmallMat<R>::M;
+  if (g.n == 0) {
+    const double2* q = static_cast<const double2*>(g.p) + off;
+    for (int e = threadIdx.x; e < LL; e += blockDim.x) dst[e] = m_from_double2<M>(__ldg(q + e));
     return;
   }
-  for (int e = threadIdx.x; e < LL; e += blockDim.x) {
-    double2 acc[U];
+  __shared__ P red[kSmallThreads];
+  const P* q = static_cast<const P*>(g.p) + off;
+  const int sh = LL <= 1 ? 0 : 32 - __clz(LL - 1);
+  const int e = threadIdx.x & ((1 << sh) - 1), s = threadIdx.x >> sh, S = kSmallThreads >> sh;
+  P acc[4];
 #pragma unroll
-    for (int u = 0; u < U; ++u) acc[u] = make_double2(0.0, 0.0);
-    int p = 0;
-    for (; p + U <= nparts; p += U) {
-      double2 v[U];
+  for (int u = 0; u < 4; ++u) gp_zero(acc[u]);
+  if (e < LL) {
+    int p = s;
+    for (; p + 3 * S < g.n; p += 4 * S) {
+      P v[4];
 #pragma unroll
-      for (int u = 0; u < U; ++u) v[u] = __ldg(partials + (size_t)(p + u) * LL + e);
+      for (int u = 0; u < 4; ++u) v[u] = q[(size_t)(p + u * S) * g.stride + e];
 #pragma unroll
-      for (int u = 0; u < U; ++u) { acc[u].x += v[u].x; acc[u].y += v[u].y; }
+      for (int u = 0; u < 4; ++u) gp_add(acc[u], v[u]);
     }
-#pragma unroll
-    for (int u = 0; u < U; ++u)
-      if (p + u < nparts) {
-        const double2 v = __ldg(partials + (size_t)(p + u) * LL + e);
-        acc[u].x += v.x;
-        acc[u].y += v.y;
-      }
-    double2 s = acc[0];
-#pragma unroll
-    for (int u = 1; u < U; ++u) { s.x += acc[u].x; s.y += acc[u].y; }
-    dst[e] = m_from_double2<typename SmallMat<R>::M>(s);
+    for (; p < g.n; p += S) gp_add(acc[0], q[(size_t)p * g.stride + e]);
   }
+  gp_add(acc[0], acc[1]);
+  gp_add(acc[2], acc[3]);
+  gp_add(acc[0], acc[2]);
+  __syncthreads();  // red may still be read by a previous call's tree
+  red[threadIdx.x] = acc[0];
   __syncthreads();
+  for (int o = S >> 1; o > 0; o >>= 1) {
+    if (s < o) gp_add(red[threadIdx.x], red[threadIdx.x + (o << sh)]);
+    __syncthreads();
+  }
+  if (s == 0 && e < LL) {
+    if constexpr (std::is_same<M, P>::value) dst[e] = red[e];
+    else dst[e] = m_from_double2<M>(gp_d2(red[e]));
+  }
 }
 
-template <typename M> __device__ void sm_copy(M* dst, const M* src, int LL) {
-  for (int e = threadIdx.x; e < LL; e += blockDim.x) dst[e] = src[e];
-  __syncthreads();
-}
-// state slot (complex FP64, global) <-> shared matrix
+// state slot (complex FP64, global) <-> shared matrix; no barrier: the caller has one before the other side is used
 template <typename M> __device__ void sm_load(M* dst, const double2* src, int LL) {
   for (int e = threadIdx.x; e < LL; e += blockDim.x) dst[e] = m_from_double2<M>(src[e]);
-  __syncthreads();
 }
 template <typename M> __device__ void sm_store(double2* dst, const M* src, int LL, bool negate = false) {
   for (int e = threadIdx.x; e < LL; e += blockDim.x) dst[e] = m_to_double2(negate ? m_neg(src[e]) : src[e]);
-  __syncthreads();
 }
+
+// Element (i, j0 + s step) of an L-row matrix for thread `rank` of `size`: rows padded to a power of two, so that no
+// index needs an integer division (a runtime division is as long as the arithmetic it would feed).
+struct Cells {
+  int i, j0, step;
+  __device__ Cells(int rank, int size, int L) {
+    const int sh = L <= 2 ? 1 : 32 - __clz(L - 1);
+    i = rank & ((1 << sh) - 1);
+    j0 = rank >> sh;
+    step = size >> sh;
+  }
+};
 
 // C = op(A) * B with op = transpose (TA=1) or identity (TA=0); C must not alias.
 template <typename M> __device__ void sm_matmul(M* Cm, const M* A, const M* B, int L, bool TA) {
-  for (int e = threadIdx.x; e < L * L; e += blockDim.x) {
-    const int i = e % L, j = e / L;
-    M s = czero<M>();
-    for (int k = 0; k < L; ++k) {
-      const M a = TA ? A[k + i * L] : A[i + k * L];
-      s = cadd(s, cmul(a, B[k + j * L]));
+  const Cells c((int)threadIdx.x, (int)blockDim.x, L);
+  if (c.i < L)
+    for (int j = c.j0; j < L; j += c.step) {
+      M s = czero<M>();
+      for (int k = 0; k < L; ++k) s = cadd(s, cmul(TA ? A[k + c.i * L] : A[c.i + k * L], B[k + j * L]));
+      Cm[c.i + j * L] = s;
     }
-    Cm[e] = s;
-  }
   __syncthreads();
 }
 
@@ -178,112 +219,116 @@ struct WarpTeam {
   __device__ void sync() const { __syncwarp(); }
 };
 
+// Integer that orders values by |a|^2 (the top 32 bits of its FP64 or FP32 pattern; NaN is the largest).
+__device__ __forceinline__ unsigned mag_key(double2 a) { return (unsigned)__double2hiint(m_abs2(a)); }
+__device__ __forceinline__ unsigned mag_key(dfc a) { return __float_as_uint(a.x.hi * a.x.hi + a.y.hi * a.y.hi); }
+
+// Pivot of step k by one warp: the largest |a| (to the 20 or 23 bits of mag_key; the first in row order among equals, with
+// full in column order first) of the rows and columns not used yet.  Lane r holds row r.
+template <typename M>
+__device__ __forceinline__ void find_pivot(const M* A, int L, int k, bool full, unsigned rows, unsigned cols, int* pr, int* pc) {
+  const int lane = threadIdx.x & 31;
+  const bool row = lane < L && ((rows >> lane) & 1u);
+  unsigned best = 0;
+  int bc = k;
+  if (!full) {
+    best = row ? mag_key(A[lane + k * L]) : 0;
+  } else if (row) {
+    for (int c = 0; c < L; ++c)
+      if ((cols >> c) & 1u) {
+        const unsigned v = mag_key(A[lane + c * L]);
+        if (v > best) { best = v; bc = c; }
+      }
+  }
+  const unsigned mx = __reduce_max_sync(0xffffffffu, best);
+  const unsigned at = row && best == mx ? (unsigned)(bc * 32 + lane) : 0xffffffffu;
+  const unsigned w = __reduce_min_sync(0xffffffffu, at);
+  *pr = (int)(w & 31u);
+  *pc = full ? (int)((w >> 5) & 31u) : k;
+}
+
 // LU solve on a team (see sm_lu_solve); *bad (shared) set on a zero /
-// non-finite pivot or result.
-template <typename R, class Team>
+// non-finite pivot or result.  No rows or columns are moved: step k records the
+// row and column it eliminates with (prow, pcol) and updates the rows not used
+// yet.  A step is a chain -- pivot search, complex reciprocal, multiplier,
+// update -- so what its length is made of is cut:
+//  * in double-float, and on a single warp, every warp finds the pivot and
+//    every thread takes the reciprocal and its row's multiplier itself, and a
+//    step has one barrier (RED);
+//  * FP64 issues two operations per clock and SM, so on the whole CTA one warp
+//    does the search and the reciprocal and one thread per row the multiplier.
+// With the factor and inverse of ldl_team and the state loaded in one trip, the L x L steps of a mixed solve of N=8192,
+// L=16 went from 44.7 to 29.5 us per launch (event-timed).
+template <typename R, bool RED, class Team>
 __device__ void lu_solve_team(const Team tm, typename SmallMat<R>::M* A, typename SmallMat<R>::M* B, int L, int nrhs,
-                              bool full, int* colperm, int* piv, int* bad) {
+                              bool full, int* prow, typename SmallMat<R>::M* dinv, int* pcol, int* bad) {
   using M = typename SmallMat<R>::M;
-  const int tid = tm.rank, nt = tm.size;
-  for (int i = tid; i < L; i += nt) colperm[i] = i;
+  const Cells c(tm.rank, tm.size, L);
+  unsigned rows = L == 32 ? 0xffffffffu : (1u << L) - 1u, cols = rows;
+  const bool mine = c.i < L;
   tm.sync();
   for (int k = 0; k < L; ++k) {
-    // ---- pivot search by the first 32 ranks: lanes scan candidates, shuffle
-    // argmax (the largest |a|, first in column-major order on ties); |a|^2
-    // orders the candidates as |a| does, without a square root
-    if (tid < 32) {
-      const int m = L - k;
-      const int cnt = full ? m * m : m;
-      R best = r_const<R>(-1.0f);
-      int bidx = 0x7fffffff;
-      for (int t = tid; t < cnt; t += 32) {
-        const int ii = k + (t % m);
-        const int jj = full ? k + t / m : k;
-        const R v = m_abs2(A[ii + jj * L]);
-        const int lin = ii + jj * L;  // column-major order
-        if (r_gt(v, best) || (r_eq(v, best) && lin < bidx)) { best = v; bidx = lin; }
+    int pr = 0, pc = 0;
+    M f;
+    if constexpr (RED) {
+      find_pivot(A, L, k, full, rows, cols, &pr, &pc);
+      const M p = A[pr + pc * L];
+      if (full) tm.sync();  // the search read columns this step updates
+      if (!r_pos_finite(m_abs2(p))) { if (tm.rank == 0) *bad = 1; return; }
+      const M pi = m_recip(p);
+      if (tm.rank == 0) { prow[k] = pr; pcol[k] = pc; dinv[k] = pi; }
+      if (mine) f = cmul(A[c.i + pc * L], pi);
+    } else {
+      if (tm.rank < 32) {
+        find_pivot(A, L, k, full, rows, cols, &pr, &pc);
+        const M p = A[pr + pc * L];
+        const M pi = m_recip(p);
+        if (tm.rank == 0) {
+          prow[k] = pr; pcol[k] = pc; dinv[k] = pi;
+          if (!r_pos_finite(m_abs2(p))) *bad = 1;
+        }
+        if (tm.rank < L && tm.rank != pr && ((rows >> tm.rank) & 1u)) A[tm.rank + pc * L] = cmul(A[tm.rank + pc * L], pi);
       }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        const R v2 = r_shfl_xor(best, o);
-        const int i2 = __shfl_xor_sync(0xffffffffu, bidx, o);
-        if (r_gt(v2, best) || (r_eq(v2, best) && i2 < bidx)) { best = v2; bidx = i2; }
-      }
-      if (tid == 0) {
-        piv[0] = bidx % L;
-        piv[1] = bidx / L;
-        if (!r_pos_finite(best)) *bad = 1;
-      }
+      tm.sync();
+      if (*bad) return;
+      pr = prow[k]; pc = pcol[k];
+      if (mine) f = A[c.i + pc * L];
     }
-    tm.sync();
-    const int pr = piv[0], pc = piv[1];
-    // ---- row swap k <-> pr (A and B)
-    if (pr != k) {
-      for (int j = tid; j < L + nrhs; j += nt) {
-        M* Mt = j < L ? A : B;
-        const int jc = j < L ? j : j - L;
-        const M t = Mt[k + jc * L];
-        Mt[k + jc * L] = Mt[pr + jc * L];
-        Mt[pr + jc * L] = t;
-      }
-    }
-    if (full) tm.sync();  // the row and the column swap share elements
-    // ---- column swap k <-> pc (A only, record permutation)
-    if (full && pc != k) {
-      for (int i = tid; i < L; i += nt) {
-        const M t = A[i + k * L];
-        A[i + k * L] = A[i + pc * L];
-        A[i + pc * L] = t;
-      }
-      if (tid == 0) { const int t = colperm[k]; colperm[k] = colperm[pc]; colperm[pc] = t; }
-    }
-    tm.sync();
-    if (*bad) continue;
-    // ---- multipliers (one complex division per row), then the trailing update
-    const M pinv = m_div(m_one<R>(), A[k + k * L]);
-    for (int i = k + 1 + tid; i < L; i += nt) A[i + k * L] = cmul(A[i + k * L], pinv);
-    tm.sync();
-    const int rows = L - k - 1;
-    for (int t = tid; t < rows * (L - k - 1 + nrhs); t += nt) {
-      const int i = k + 1 + t % rows;
-      const int jj = t / rows;  // 0..(L-k-2) -> A columns k+1.., then B columns
-      const M f = A[i + k * L];
-      if (jj < L - k - 1) {
-        const int j = k + 1 + jj;
-        A[i + j * L] = csub(A[i + j * L], cmul(f, A[k + j * L]));
-      } else {
-        const int j = jj - (L - k - 1);
-        B[i + j * L] = csub(B[i + j * L], cmul(f, B[k + j * L]));
+    rows &= ~(1u << pr);
+    cols &= ~(1u << pc);
+    if (mine && ((rows >> c.i) & 1u)) {
+      for (int j = c.j0; j < L + nrhs; j += c.step) {
+        if (j < L && !((cols >> j) & 1u)) continue;
+        M* col = j < L ? A + j * L : B + (j - L) * L;
+        col[c.i] = csub(col[c.i], cmul(f, col[pr]));
       }
     }
     tm.sync();
   }
-  // ---- back substitution, right-looking: row k of X is final once the rows
-  // below were eliminated; then every remaining row sheds its row-k term in
-  // parallel (the serial chain per row is one product per step, not L)
-  for (int k = tid; k < L; k += nt) A[k + k * L] = m_div(m_one<R>(), A[k + k * L]);
-  tm.sync();  // the diagonal now holds 1 / pivot
-  for (int k = L - 1; k >= 0; --k) {
-    for (int j = tid; j < nrhs; j += nt) B[k + j * L] = cmul(B[k + j * L], A[k + k * L]);
-    tm.sync();
-    for (int t = tid; t < k * nrhs; t += nt) {
-      const int r = t % k, j = t / k;
-      B[r + j * L] = csub(B[r + j * L], cmul(A[r + k * L], B[k + j * L]));
+  // back substitution: the unknown of step k is its pivot row's right-hand side over the pivot once the later ones have
+  // been taken out; each step takes it out of the rows used before, one barrier a step
+  for (int k = L - 1; k > 0; --k) {
+    const int pr = prow[k], pc = pcol[k];
+    rows |= 1u << pr;  // rows used at step k and after
+    if (mine && !((rows >> c.i) & 1u)) {
+      const M u = cmul(A[c.i + pc * L], dinv[k]);
+      for (int j = c.j0; j < nrhs; j += c.step) {
+        M* col = B + j * L;
+        col[c.i] = csub(col[c.i], cmul(u, col[pr]));
+      }
     }
     tm.sync();
   }
-  if (full) {
-    // x[colperm[k]] = y[k]; use A as scratch (A no longer needed)
-    for (int e = tid; e < L * nrhs; e += nt) A[e] = B[e];
-    tm.sync();
-    for (int e = tid; e < L * nrhs; e += nt) {
-      const int k = e % L, j = e / L;
-      B[colperm[k] + j * L] = A[e];
+  // X[pcol[k]] = B[prow[k]] / pivot (through A, no longer needed)
+  if (mine)
+    for (int j = c.j0; j < nrhs; j += c.step) A[pcol[c.i] + j * L] = cmul(B[prow[c.i] + j * L], dinv[c.i]);
+  tm.sync();
+  if (mine)
+    for (int j = c.j0; j < nrhs; j += c.step) {
+      const M v = A[c.i + j * L];
+      if (!m_finite(v)) *bad = 1;
+      B[c.i + j * L] = v;
     }
-    tm.sync();
-  }
-  for (int e = tid; e < L * nrhs; e += nt)
-    if (!m_finite(B[e])) *bad = 1;
 }
 
 // Solve A X = B (L x L, nrhs columns) by LU; A and B are overwritten (B <- X).
@@ -292,14 +337,16 @@ __device__ void lu_solve_team(const Team tm, typename SmallMat<R>::M* A, typenam
 // first max in column-major order.  Returns false on a zero / non-finite pivot.
 template <typename R>
 __device__ bool sm_lu_solve(typename SmallMat<R>::M* A, typename SmallMat<R>::M* B, int L, int nrhs, bool full,
-                            int* colperm /*smem[L]*/, int* piv /*smem[2]*/) {
+                            int* colperm /*smem[L]*/, int* piv /*smem[L]*/) {
   __shared__ int bad;
+  __shared__ typename SmallMat<R>::M dinv[kMaxL];
   if (threadIdx.x == 0) bad = 0;
   __syncthreads();
   if (L <= kWarpL) {
-    if (threadIdx.x < 32) lu_solve_team<R>(WarpTeam{(int)threadIdx.x, 32}, A, B, L, nrhs, full, colperm, piv, &bad);
+    if (threadIdx.x < 32) lu_solve_team<R, true>(WarpTeam{(int)threadIdx.x, 32}, A, B, L, nrhs, full, piv, dinv, colperm, &bad);
   } else {
-    lu_solve_team<R>(CtaTeam{(int)threadIdx.x, (int)blockDim.x}, A, B, L, nrhs, full, colperm, piv, &bad);
+    lu_solve_team<R, !std::is_same<R, double>::value>(CtaTeam{(int)threadIdx.x, (int)blockDim.x}, A, B, L, nrhs, full, piv,
+                                                      dinv, colperm, &bad);
   }
   __syncthreads();
   const bool ok = !bad;
@@ -307,97 +354,82 @@ __device__ bool sm_lu_solve(typename SmallMat<R>::M* A, typename SmallMat<R>::M*
   return ok;
 }
 
-// Right-looking Cholesky on a team (see sm_cholesky), in place on Rm.  Every
-// rank takes the square root and reciprocal of the pivot itself (no broadcast
-// phase); rank 0 writes the diagonal after all ranks have read it.
-template <typename R, class Team>
-__device__ void cholesky_team(const Team tm, typename SmallMat<R>::M* Rm, int L, int* bad) {
+// Cholesky factor and inverse factor in one sweep on a team: H = L D L^H with L
+// unit lower triangular, so R = D^1/2 L^H and R^-1 = (L^-1)^H D^-1/2.  One array
+// holds both: U = D L^H above (and on) the diagonal, W = L^-1 below it; step k
+// takes L_ik U_k out of the rows i > k of U and L_ik W_k out of W's.  A step is a
+// reciprocal, a multiplier and an update (no square root in the chain; FP64 on a
+// whole CTA takes the multipliers once, see lu_solve_team), and there is no
+// second sweep for the inverse.
+template <typename R, bool RED, class Team>
+__device__ void ldl_team(const Team tm, typename SmallMat<R>::M* U, int L, R* dinv, int* bad) {
   using M = typename SmallMat<R>::M;
-  const int tid = tm.rank, nt = tm.size;
+  const Cells c(tm.rank, tm.size, L);
+  tm.sync();
   for (int k = 0; k < L; ++k) {
-    R d = Rm[k + k * L].x;
-    if (!r_pos_finite(d)) { if (tid == 0) *bad = 1; d = r_const<R>(1.0f); }
-    d = r_sqrt(d);
-    const R di = r_recip(d);
-    tm.sync();
-    if (tid == 0) Rm[k + k * L] = cmake(d, r_const<R>(0.0f));
-    for (int j = k + 1 + tid; j < L; j += nt) {
-      const M v = Rm[k + j * L];
-      Rm[k + j * L] = cmake(v.x * di, v.y * di);
+    R di;
+    const R d = U[k + k * L].x;
+    if (!r_pos_finite(d)) { if (tm.rank == 0) *bad = 1; return; }
+    if constexpr (RED) {
+      di = r_recip(d);
+    } else {
+      if (tm.rank < 32) {
+        di = r_recip(d);
+        if (tm.rank == 0) dinv[k] = di;
+      }
+      tm.sync();
+      di = dinv[k];
     }
-    tm.sync();
-    // trailing block (upper part, i <= j): H_ij -= conj(R_ki) R_kj
-    const int m = L - k - 1;
-    for (int t = tid; t < m * m; t += nt) {
-      const int i = k + 1 + t % m, j = k + 1 + t / m;
-      if (i <= j) Rm[i + j * L] = csub(Rm[i + j * L], cconjmul(Rm[k + i * L], Rm[k + j * L]));
+    if (c.i > k && c.i < L) {
+      const M u = U[k + c.i * L];
+      const M l = cmake(u.x * di, -(u.y * di));  // L_ik
+      for (int j = c.j0; j < L; j += c.step) {
+        if (j > k && j < c.i) continue;  // neither triangle has (i, j) at this step
+        M* col = U + j * L;
+        col[c.i] = j == k ? m_neg(l) : csub(col[c.i], cmul(l, col[k]));
+      }
     }
     tm.sync();
   }
 }
 
-// H = R^H R with R upper triangular, real positive diagonal.  R may alias H.
-// Right-looking: step k takes the square root of the (already updated)
-// diagonal, scales row k and subtracts its outer product from the trailing
-// block, every element in parallel.
+// H = R^H R with R upper triangular, real positive diagonal, and Ri = R^-1.
+// Rm, Ri and H are three arrays; H (its upper triangle is read) is overwritten.
 template <typename R>
-__device__ bool sm_cholesky(typename SmallMat<R>::M* Rm, const typename SmallMat<R>::M* H, int L) {
+__device__ bool sm_chol_inv(typename SmallMat<R>::M* Rm, typename SmallMat<R>::M* Ri, typename SmallMat<R>::M* H, int L) {
   using M = typename SmallMat<R>::M;
   __shared__ int bad;
-  const int tid = threadIdx.x;
-  if (tid == 0) bad = 0;
-  if (Rm != H) for (int e = tid; e < L * L; e += blockDim.x) Rm[e] = H[e];
-  __syncthreads();
-  if (L <= kWarpL) {
-    if (tid < 32) cholesky_team<R>(WarpTeam{tid, 32}, Rm, L, &bad);
-  } else {
-    cholesky_team<R>(CtaTeam{tid, (int)blockDim.x}, Rm, L, &bad);
-  }
-  __syncthreads();
-  // zero the strictly lower part
-  for (int e = tid; e < L * L; e += blockDim.x) {
-    const int i = e % L, j = e / L;
-    if (i > j) Rm[e] = czero<M>();
-  }
-  __syncthreads();
-  const bool ok = !bad;
-  __syncthreads();
-  return ok;
-}
-
-// Inverse of an upper triangular matrix with a real positive diagonal (the
-// Cholesky factors): R X = I solved bottom-up, right-looking -- row i of X is
-// final after scaling by 1 / R_ii, then the rows above shed their row-i term,
-// all elements in parallel.
-template <typename R>
-__device__ void sm_tri_inv(typename SmallMat<R>::M* Ri, const typename SmallMat<R>::M* Rm, int L) {
-  using M = typename SmallMat<R>::M;
   __shared__ R dinv[kMaxL];
-  for (int i = threadIdx.x; i < L; i += blockDim.x) dinv[i] = r_recip(Rm[i + i * L].x);
-  for (int e = threadIdx.x; e < L * L; e += blockDim.x) Ri[e] = (e % L) == (e / L) ? m_one<R>() : czero<M>();
+  if (threadIdx.x == 0) bad = 0;
+  const Cells c((int)threadIdx.x, (int)blockDim.x, L);
+  if (c.i < L)
+    for (int j = c.j0; j < c.i; j += c.step) H[c.i + j * L] = czero<M>();
   __syncthreads();
-  auto run = [&](auto tm) {
-    for (int i = L - 1; i >= 0; --i) {
-      for (int j = i + tm.rank; j < L; j += tm.size) {
-        const M v = Ri[i + j * L];
-        Ri[i + j * L] = cmake(v.x * dinv[i], v.y * dinv[i]);
-      }
-      tm.sync();
-      // rows r < i, columns j >= i: X_rj -= R_ri X_ij
-      const int nc = L - i;
-      for (int t = tm.rank; t < i * nc; t += tm.size) {
-        const int r = t % i, j = i + t / i;
-        Ri[r + j * L] = csub(Ri[r + j * L], cmul(Rm[r + i * L], Ri[i + j * L]));
-      }
-      tm.sync();
-    }
-  };
   if (L <= kWarpL) {
-    if (threadIdx.x < 32) run(WarpTeam{(int)threadIdx.x, 32});
+    if (threadIdx.x < 32) ldl_team<R, true>(WarpTeam{(int)threadIdx.x, 32}, H, L, dinv, &bad);
   } else {
-    run(CtaTeam{(int)threadIdx.x, (int)blockDim.x});
+    ldl_team<R, !std::is_same<R, double>::value>(CtaTeam{(int)threadIdx.x, (int)blockDim.x}, H, L, dinv, &bad);
   }
   __syncthreads();
+  if (bad) return false;  // shared: the same for every thread
+  for (int i = threadIdx.x; i < L; i += blockDim.x) dinv[i] = r_recip(r_sqrt(H[i + i * L].x));
+  __syncthreads();
+  if (c.i < L) {
+    const R q = dinv[c.i];
+    for (int j = c.j0; j < L; j += c.step) {
+      const M v = H[c.i + j * L];
+      const M w = cmake(v.x * q, v.y * q);
+      if (j >= c.i) {  // R_ij = U_ij / sqrt(d_i); and zero below the diagonal of R and Ri
+        Rm[c.i + j * L] = j == c.i ? cmake(r_sqrt(v.x), r_const<R>(0.0f)) : w;
+        if (j == c.i) Ri[c.i + j * L] = cmake(q, r_const<R>(0.0f));
+        else { Rm[j + c.i * L] = czero<M>(); Ri[j + c.i * L] = czero<M>(); }
+      } else {
+        Ri[j + c.i * L] = cmake(w.x, -w.y);  // R^-1_ji = conj(W_ij) / sqrt(d_i)
+      }
+    }
+  }
+  __syncthreads();
+  return true;
 }
 
 // Frobenius norm in FP64 (any scale): per-thread sums of |m|^2, a warp

@@ -70,7 +70,7 @@ struct SolverWork {
   DevBuf X64, R64, Y64;
   DevBuf xdf, ydf, diagdf;      // double-float residual MVP (mixed solves)
   DevBuf jpre64, diag32, jpre32;
-  DevBuf gpart;                 // per-CTA Gram partials [G][L*L], or [G][2 L*L] for gram2
+  DevBuf gpart;                 // per-CTA Gram partials [G][L*L], or [G][2 L*L] for a pair of Grams
   DevBuf partials, partials2;   // reduced Gram matrices (c128) [L*L]
   DevBuf vpart;                 // dot / norm partials
   DevBuf colf;                  // FP64 [2][L]: column scaling of the inner right-hand side and its inverse
@@ -117,8 +117,8 @@ __device__ __forceinline__ double2* slot(double2* st, int s, int L) { return st 
 // one-CTA steps
 // ---------------------------------------------------------------------------
 struct SmallSmem {
-  // dynamic smem carve-up: 6 matrices + reduction scratch
-  static size_t bytes(int L) { return 6 * (size_t)L * L * sizeof(double2) + (2 + kMaxL) * sizeof(int); }
+  // dynamic smem carve-up: 8 matrices + pivot rows and columns
+  static size_t bytes(int L) { return 8 * (size_t)L * L * sizeof(double2) + 2 * kMaxL * sizeof(int); }
 };
 
 #define SMALL_PROLOGUE                                                                              \
@@ -130,8 +130,10 @@ struct SmallSmem {
   [[maybe_unused]] M* m3 = m2 + L * L;                                                              \
   [[maybe_unused]] M* m4 = m3 + L * L;                                                              \
   [[maybe_unused]] M* m5 = m4 + L * L;                                                              \
-  [[maybe_unused]] int* piv = reinterpret_cast<int*>(m5 + L * L);                                   \
-  [[maybe_unused]] int* colperm = piv + 2;                                                          \
+  [[maybe_unused]] M* m6 = m5 + L * L;                                                              \
+  [[maybe_unused]] M* m7 = m6 + L * L;                                                              \
+  [[maybe_unused]] int* piv = reinterpret_cast<int*>(m7 + L * L);                                   \
+  [[maybe_unused]] int* colperm = piv + kMaxL;                                                         \
   const int LL = L * L;
 
 __device__ void fail(SolverCtl* ctl) {
@@ -197,8 +199,7 @@ __device__ bool chol_and_inverse(typename SmallMat<R>::M* m0, typename SmallMat<
       m0[e].y = dfl(m0[e].y.hi * sh, m0[e].y.lo * sh);
     }
     __syncthreads();
-    if (!sm_cholesky<R>(m1, m0, L)) return false;
-    sm_tri_inv<R>(m2, m1, L);
+    if (!sm_chol_inv<R>(m1, m2, m0, L)) return false;
     const float sr = ldexpf(1.0f, e2), si = ldexpf(1.0f, -e2);  // R = R' 2^e2, R^-1 = R'^-1 2^-e2
     for (int e = threadIdx.x; e < L * L; e += blockDim.x) {
       m1[e].x = dfl(m1[e].x.hi * sr, m1[e].x.lo * sr);
@@ -209,20 +210,18 @@ __device__ bool chol_and_inverse(typename SmallMat<R>::M* m0, typename SmallMat<
     __syncthreads();
     return true;
   } else {
-    if (!sm_cholesky<R>(m1, m0, L)) return false;
-    sm_tri_inv<R>(m2, m1, L);
-    return true;
+    return sm_chol_inv<R>(m1, m2, m0, L);
   }
 }
 
-// The L x L steps of a COCG-RQ iteration on shared-memory matrices (the six
+// The L x L steps of a COCG-RQ iteration on shared-memory matrices (the eight
 // L x L work matrices of SMALL_PROLOGUE); each one-CTA kernel fills the inputs
 // (from reduced Gram partials) and calls one of them.
 template <typename R> struct SmallWork {
-  typename SmallMat<R>::M *m0, *m1, *m2, *m3, *m4, *m5;
+  typename SmallMat<R>::M *m0, *m1, *m2, *m3, *m4, *m5, *m6, *m7;
   int *piv, *colperm;
 };
-#define SMALL_WORK SmallWork<R>{m0, m1, m2, m3, m4, m5, piv, colperm}
+#define SMALL_WORK SmallWork<R>{m0, m1, m2, m3, m4, m5, m6, m7, piv, colperm}
 
 // QR step 1: R1 = chol(H), R1inv, with H = W^H W in w.m0.  false: breakdown.
 template <typename R>
@@ -235,22 +234,20 @@ __device__ bool core_chol1(const SmallWork<R>& w, int L, double2* st, SolverCtl*
 }
 
 // COCG-RQ, the second CholQR2 step fused with beta, with H2 = W1^H W1 in
-// w.m0; load_gt(dst) puts W1^T W1 into a shared matrix.
+// w.m0, W1^T W1 in w.m6, R1 in w.m3, xi in w.m5 and Q^T Q in w.m7 (all loaded
+// at once: one trip to memory instead of five).
 //   R2 = chol(H2), R2inv, tau = R2 R1, xi = tau xi, err, stopping test;
 //   Q' = W1 R2^-1, so Q'^T Q' = R2^-T (W1^T W1) R2^-1 without a pass over Q'
 //   (R2 is near the identity: the second CholQR2 factor);
 //   beta = (Q^T Q)^-1 (tau^T Q'^T Q') ; Q^T Q <- Q'^T Q'.
 // Returns false on breakdown or when the stopping test passed (done).
-template <typename R, class LoadGT>
-__device__ bool core_chol2_beta(const SmallWork<R>& w, int L, double2* st, SolverCtl* ctl, double* hist, int full,
-                                LoadGT load_gt) {
+template <typename R>
+__device__ bool core_chol2_beta(const SmallWork<R>& w, int L, double2* st, SolverCtl* ctl, double* hist, int full) {
   const int LL = L * L;
   if (!chol_and_inverse<R>(w.m0, w.m1, w.m2, L)) { fail(ctl); return false; }
   sm_store(slot(st, kR2Inv, L), w.m2, LL);
-  sm_load(w.m3, slot(st, kR1, L), LL);
   sm_matmul(w.m4, w.m1, w.m3, L, false);  // tau = R2 R1
   sm_store(slot(st, kTau, L), w.m4, LL);
-  sm_load(w.m5, slot(st, kXi, L), LL);
   sm_matmul(w.m0, w.m4, w.m5, L, false);  // xi = tau xi
   sm_store(slot(st, kXi, L), w.m0, LL);
   const double nrm = sm_fro<R>(w.m0, LL);
@@ -269,75 +266,55 @@ __device__ bool core_chol2_beta(const SmallWork<R>& w, int L, double2* st, Solve
   }
   __syncthreads();
   if (stop) return false;
-  load_gt(w.m0);                               // W1^T W1
-  sm_matmul(w.m3, w.m0, w.m2, L, false);       // (W1^T W1) R2^-1
+  sm_matmul(w.m3, w.m6, w.m2, L, false);       // (W1^T W1) R2^-1
   sm_matmul(w.m5, w.m2, w.m3, L, true);        // Q'^T Q'
   sm_matmul(w.m0, w.m4, w.m5, L, true);        // tau^T Q'^T Q'
-  sm_load(w.m1, slot(st, kQtQ, L), LL);
-  if (!sm_lu_solve<R>(w.m1, w.m0, L, L, full != 0, w.colperm, w.piv)) { fail(ctl); return false; }
+  if (!sm_lu_solve<R>(w.m7, w.m0, L, L, full != 0, w.colperm, w.piv)) { fail(ctl); return false; }
   sm_store(slot(st, kBeta, L), w.m0, LL);
   sm_store(slot(st, kQtQ, L), w.m5, LL);
   return true;
 }
 
-// COCG-RQ alpha with S^T AS in w.m0 and Q^T Q in w.m1 (have_qq; else the kept
-// slot): alpha = (S^T AS)^-1 (Q^T Q) ; A_xi = alpha xi ; -alpha.
+// COCG-RQ alpha with S^T AS in w.m0, Q^T Q in w.m1 and xi in w.m2:
+// alpha = (S^T AS)^-1 (Q^T Q) ; A_xi = alpha xi ; -alpha.
 template <typename R>
-__device__ bool core_alpha(const SmallWork<R>& w, int L, double2* st, SolverCtl* ctl, bool have_qq, int full) {
+__device__ bool core_alpha(const SmallWork<R>& w, int L, double2* st, SolverCtl* ctl, int full) {
   const int LL = L * L;
-  if (have_qq) sm_store(slot(st, kQtQ, L), w.m1, LL);
-  else sm_load(w.m1, slot(st, kQtQ, L), LL);
   if (!sm_lu_solve<R>(w.m0, w.m1, L, L, full != 0, w.colperm, w.piv)) { fail(ctl); return false; }
   sm_store(slot(st, kAlpha, L), w.m1, LL);
   sm_store(slot(st, kNAlpha, L), w.m1, LL, true);
-  sm_load(w.m2, slot(st, kXi, L), LL);
   sm_matmul(w.m3, w.m1, w.m2, L, false);
   sm_store(slot(st, kAXi, L), w.m3, LL);
   return true;
 }
 
 // QR step 1: H = W^H W ; R1 = chol(H) ; R1inv
-template <typename R>
+template <typename R, typename P>
 __global__ void __launch_bounds__(kSmallThreads)
-k_small_chol1(const double2* __restrict__ part, int nparts, int L, double2* st, SolverCtl* ctl) {
+k_small_chol1(GramRef part, int L, double2* st, SolverCtl* ctl) {
   if (ctl_skip(ctl)) return;
   SMALL_PROLOGUE
-  sm_reduce<R>(m0, part, nparts, LL);
+  sm_gram<R, P>(m0, part, 0, LL);
+  __syncthreads();
   core_chol1<R>(SMALL_WORK, L, st, ctl);
 }
 
 // QR step 2: H2 = W1^H W1 ; R2 = chol ; R2inv ; tau = R2 R1.
 // mode 0: xi = tau (initial QR of the right-hand side)
-// mode 1: xi = tau xi ; err = ||xi|| / bnorm ; stopping test
 // mode 2: like mode 0 but R = tau returned in kXi only (qr_reduced)
-template <typename R>
+template <typename R, typename P>
 __global__ void __launch_bounds__(kSmallThreads)
-k_small_chol2(const double2* __restrict__ part, int nparts, int L, double2* st, SolverCtl* ctl, double tol,
-              double* hist, int k, int mode) {
+k_small_chol2(GramRef part, int L, double2* st, SolverCtl* ctl, int mode) {
   if (ctl_skip(ctl)) return;
   SMALL_PROLOGUE
-  sm_reduce<R>(m0, part, nparts, LL);
+  sm_gram<R, P>(m0, part, 0, LL);
+  sm_load(m3, slot(st, kR1, L), LL);
+  __syncthreads();
   if (!chol_and_inverse<R>(m0, m1, m2, L)) { fail(ctl); return; }
   sm_store(slot(st, kR2Inv, L), m2, LL);
-  sm_load(m3, slot(st, kR1, L), LL);
   sm_matmul(m4, m1, m3, L, false);  // tau = R2 R1
   sm_store(slot(st, kTau, L), m4, LL);
-  if (mode != 1) {
-    sm_store(slot(st, kXi, L), m4, LL);
-    return;
-  }
-  sm_load(m5, slot(st, kXi, L), LL);
-  sm_matmul(m0, m4, m5, L, false);  // xi = tau xi
-  sm_store(slot(st, kXi, L), m0, LL);
-  const double nrm = sm_fro<R>(m0, LL);
-  if (threadIdx.x == 0) {
-    const double err = nrm / ctl->bnorm;
-    ctl->err = err;
-    if (hist) hist[k] = err;
-    ctl->iter = k + 1;
-    if (!isfinite(err)) { ctl->status = BDDA_ERR_BREAKDOWN; ctl->done = 1; }
-    else if (err < tol) ctl->done = 1;
-  }
+  sm_store(slot(st, kXi, L), m4, LL);
 }
 
 // COCG-RQ, the second CholQR2 step fused with beta.  part holds the
@@ -346,54 +323,53 @@ k_small_chol2(const double2* __restrict__ part, int nparts, int L, double2* st, 
 //   Q' = W1 R2^-1, so Q'^T Q' = R2^-T (W1^T W1) R2^-1 without a pass over Q'
 //   (R2 is near the identity: the second CholQR2 factor);
 //   beta = (Q^T Q)^-1 (tau^T Q'^T Q') ; Q^T Q <- Q'^T Q'.
-template <typename R>
+template <typename R, typename P>
 __global__ void __launch_bounds__(kSmallThreads)
-k_small_chol2_beta(const double2* __restrict__ part, int L, double2* st, SolverCtl* ctl, double* hist, int full) {
+k_small_chol2_beta(GramRef part, int L, double2* st, SolverCtl* ctl, double* hist, int full) {
   if (ctl_skip(ctl)) return;
   SMALL_PROLOGUE
-  sm_reduce<R>(m0, part, 1, LL);
-  core_chol2_beta<R>(SMALL_WORK, L, st, ctl, hist, full, [&](M* d) { sm_reduce<R>(d, part + LL, 1, LL); });
+  sm_load(m3, slot(st, kR1, L), LL);
+  sm_load(m5, slot(st, kXi, L), LL);
+  sm_load(m7, slot(st, kQtQ, L), LL);
+  sm_gram<R, P>(m0, part, 0, LL);
+  sm_gram<R, P>(m6, part, LL, LL);
+  __syncthreads();
+  core_chol2_beta<R>(SMALL_WORK, L, st, ctl, hist, full);
 }
 
 // COCG-RQ alpha: alpha = (S^T AS)^-1 (Q^T Q) ; A_xi = alpha xi ; -alpha
-template <typename R>
+// (pQQ, first iteration: Q^T Q, else the kept slot)
+template <typename R, typename P>
 __global__ void __launch_bounds__(kSmallThreads)
-k_small_cocg_alpha(const double2* __restrict__ pSAS, const double2* __restrict__ pQQ, int nparts, int L, double2* st,
-                   SolverCtl* ctl, int full) {
+k_small_cocg_alpha(GramRef pSAS, GramRef pQQ, int L, double2* st, SolverCtl* ctl, int full) {
   if (ctl_skip(ctl)) return;
   SMALL_PROLOGUE
-  sm_reduce<R>(m0, pSAS, nparts, LL);
-  if (pQQ) sm_reduce<R>(m1, pQQ, nparts, LL);
-  core_alpha<R>(SMALL_WORK, L, st, ctl, pQQ != nullptr, full);
-}
-
-// COCG-RQ beta: beta = (Q^T Q)^-1 (tau^T Q'^T Q') ; Q^T Q <- Q'^T Q'
-template <typename R>
-__global__ void __launch_bounds__(kSmallThreads)
-k_small_cocg_beta(const double2* __restrict__ pQQn, int nparts, int L, double2* st, SolverCtl* ctl, int full) {
-  if (ctl_skip(ctl)) return;
-  SMALL_PROLOGUE
-  sm_reduce<R>(m0, pQQn, nparts, LL);        // Q'^T Q'
-  sm_load(m1, slot(st, kTau, L), LL);
-  sm_matmul(m2, m1, m0, L, true);            // tau^T Q'^T Q'
-  sm_load(m3, slot(st, kQtQ, L), LL);
-  if (!sm_lu_solve<R>(m3, m2, L, L, full != 0, colperm, piv)) { fail(ctl); return; }
-  sm_store(slot(st, kBeta, L), m2, LL);
-  sm_store(slot(st, kQtQ, L), m0, LL);
+  if (pQQ.p) {
+    sm_gram<R, P>(m1, pQQ, 0, LL);
+    __syncthreads();
+    sm_store(slot(st, kQtQ, L), m1, LL);
+  } else {
+    sm_load(m1, slot(st, kQtQ, L), LL);
+  }
+  sm_load(m2, slot(st, kXi, L), LL);
+  sm_gram<R, P>(m0, pSAS, 0, LL);
+  __syncthreads();
+  core_alpha<R>(SMALL_WORK, L, st, ctl, full);
 }
 
 // BiCG*: X = M^-1 RHS with M = reduce(pM) (stored in kM), RHS = scale * reduce(pR).
 // out slots: x -> so, -x -> sno (optional)
-template <typename R>
+template <typename R, typename P>
 __global__ void __launch_bounds__(kSmallThreads)
-k_small_solve(const double2* __restrict__ pM, const double2* __restrict__ pR, int nparts, int L, double2* st,
-              SolverCtl* ctl, int mslot_in, int mslot_store, double rhs_scale, const double2* scal_div, int so, int sno) {
+k_small_solve(GramRef pM, GramRef pR, int L, double2* st, SolverCtl* ctl, int mslot_in, int mslot_store, double rhs_scale,
+              const double2* scal_div, int so, int sno) {
   if (ctl_skip(ctl)) return;
   SMALL_PROLOGUE
-  if (pM) sm_reduce<R>(m0, pM, nparts, LL);
+  if (pM.p) sm_gram<R, P>(m0, pM, 0, LL);
   else sm_load(m0, slot(st, mslot_in, L), LL);
+  sm_gram<R, P>(m1, pR, 0, LL);
+  __syncthreads();
   if (mslot_store >= 0) sm_store(slot(st, mslot_store, L), m0, LL);
-  sm_reduce<R>(m1, pR, nparts, LL);
   double2 sc = make_double2(rhs_scale, 0.0);
   if (scal_div) sc = cdiv(sc, *scal_div);
   const M scm = m_from_double2<M>(sc);
@@ -447,10 +423,10 @@ __global__ void __launch_bounds__(256) k_small_err(const double* __restrict__ vp
 }
 
 // st[s] = reduce(partials)
-__global__ void __launch_bounds__(kSmallThreads)
-k_small_store_reduce(const double2* __restrict__ part, int nparts, int L, double2* st, SolverCtl* ctl, int s) {
+template <typename P>
+__global__ void __launch_bounds__(kSmallThreads) k_small_store_reduce(GramRef part, int L, double2* st, SolverCtl* ctl, int s) {
   if (ctl_skip(ctl)) return;
-  sm_reduce<double>(slot(st, s, L), part, nparts, L * L);
+  sm_gram<double, P>(slot(st, s, L), part, 0, L * L);
 }
 
 // ---------------------------------------------------------------------------
@@ -484,25 +460,23 @@ struct Krylov {
     ++mvps;
     return op_block_mvp<T>(op, op->dip, x, n, y, n, L, diag, jpre, st, &ctl()->done);
   }
-  // out = op(A)^T B (L x L, FP64): per-CTA partials, then a multi-CTA ordered reduction
-  template <bool CONJ> void gram(const C* A, const C* B, double2* out) {
+  using GP = typename GramPart<T>::type;
+  // Gram op(A)^T B (L x L) into place `which` (0 or 1; BOTH takes both: A^H A, then A^T A): per-CTA partials, for L > 8
+  // followed by a multi-CTA ordered reduction to FP64 (up to L = 8 the one-CTA kernel that reads it sums the partials)
+  template <bool CONJ, bool BOTH = false> GramRef gram(const C* A, const C* B, int which = 0) {
+    const int LL = L * L, LLo = BOTH ? 2 * LL : LL;
+    GP* part = w->gpart.template as<GP>() + (size_t)which * LL * G();
     op->timer.begin(kGram, st);
-    using P = typename GramPart<T>::type;
-    k_gram<T, CONJ><<<G(), kGramThreads, 0, st>>>(A, n, B, n, n, L, w->gpart.template as<P>(), ctl());
-    k_gram_reduce<P><<<(L * L + kRedEntries - 1) / kRedEntries, kRedEntries * kRedGroups, 0, st>>>(
-        w->gpart.template as<P>(), G(), L * L, out, ctl());
+    k_gram<T, CONJ, BOTH><<<G(), kGramThreads, 0, st>>>(A, n, B, n, n, L, part, ctl());
+    GramRef r{part, G(), LLo};
+    if (L > kWarpL) {
+      double2* out = (which ? w->partials2 : w->partials).template as<double2>();
+      k_gram_reduce<GP><<<(LLo + kRedEntries - 1) / kRedEntries, kRedEntries * kRedGroups, 0, st>>>(part, G(), LLo, out, ctl());
+      op->timer.count(kGram);
+      r = GramRef{out, 0, LLo};
+    }
     op->timer.end(kGram, st);
-    op->timer.count(kGram);
-  }
-  // out[0 .. LL) = A^H A, out[LL .. 2 LL) = A^T A
-  void gram2(const C* A, double2* out) {
-    op->timer.begin(kGram, st);
-    using P = typename GramPart<T>::type;
-    k_gram<T, true, true><<<G(), kGramThreads, 0, st>>>(A, n, A, n, n, L, w->gpart.template as<P>(), ctl());
-    k_gram_reduce<P><<<(2 * L * L + kRedEntries - 1) / kRedEntries, kRedEntries * kRedGroups, 0, st>>>(
-        w->gpart.template as<P>(), G(), 2 * L * L, out, ctl());
-    op->timer.end(kGram, st);
-    op->timer.count(kGram);
+    return r;
   }
   // Out1 = A Ma ; Out2 = Out1 + B Mb
   void rowmm2(const C* A, const double2* Ma, const C* B, const double2* Mb, C* Out1, C* Out2) {
@@ -558,31 +532,23 @@ struct Krylov {
 
   // [Q, R] = qr(A) by CholQR2 ; R -> kXi (mode 0/2).  W is scratch (may equal Q).
   void cholqr2(const C* A, C* W, C* Q, int mode) {
-    double2* p = w->partials.template as<double2>();
-    gram<true>(A, A, p);
-    small_launch(k_small_chol1<SR>, (const double2*)p, 1, L, small(), ctl());
+    small_launch(k_small_chol1<SR, GP>, gram<true>(A, A), L, small(), ctl());
     rowmm(A, sl(kR1Inv), nullptr, nullptr, nullptr, W);
-    gram<true>(W, W, p);
-    small_launch(k_small_chol2<SR>, (const double2*)p, 1, L, small(), ctl(), 0.0, (double*)nullptr, 0, mode);
+    small_launch(k_small_chol2<SR, GP>, gram<true>(W, W), L, small(), ctl(), mode);
     rowmm(W, sl(kR2Inv), nullptr, nullptr, nullptr, Q);
   }
 
   // One block COCG-RQ iteration; first adds the Gram Q^T Q of the starting block.
   int cocg_iteration(bool first, C* Q, C* Qn, C* S, C* AS, C* W, C* X, bool full) {
-    double2* p = w->partials.template as<double2>();
-    double2* p2 = w->partials2.template as<double2>();
     BDDA_TRY(mvp(S, AS));
-    gram<false>(S, AS, p);
-    if (first) gram<false>(Q, Q, p2);
-    small_launch(k_small_cocg_alpha<SR>, (const double2*)p, (const double2*)(first ? p2 : nullptr), 1, L, small(), ctl(),
-                 (int)full);
+    const GramRef sas = gram<false>(S, AS), qq = first ? gram<false>(Q, Q, 1) : GramRef{nullptr, 0, 0};
+    small_launch(k_small_cocg_alpha<SR, GP>, sas, qq, L, small(), ctl(), (int)full);
     rowmm(S, sl(kAXi), nullptr, nullptr, X, X);           // X += S alpha xi
     rowmm(AS, sl(kNAlpha), nullptr, nullptr, Q, W);       // W = Q - AS alpha
-    gram<true>(W, W, p);
-    small_launch(k_small_chol1<SR>, (const double2*)p, 1, L, small(), ctl());
+    small_launch(k_small_chol1<SR, GP>, gram<true>(W, W), L, small(), ctl());
     rowmm(W, sl(kR1Inv), nullptr, nullptr, nullptr, W);   // W1
-    gram2(W, p);                                          // W1^H W1, W1^T W1
-    small_launch(k_small_chol2_beta<SR>, (const double2*)p, L, small(), ctl(), w->hist.as<double>(), (int)full);
+    const GramRef w1 = gram<true, true>(W, W);            // W1^H W1, W1^T W1
+    small_launch(k_small_chol2_beta<SR, GP>, w1, L, small(), ctl(), w->hist.as<double>(), (int)full);
     rowmm2(W, sl(kR2Inv), S, sl(kBeta), Qn, S);           // Q' = W1 R2^-1 ; S = Q' + S beta
     return BDDA_OK;
   }
@@ -722,8 +688,6 @@ struct Krylov {
   // Block BiCGSTAB (bl_bicgstab_mvp_fft.cpp:21-98 / bl_bicgstab_jacobi_mvp_fft.cpp:21-96)
   int bicgstab(const C* Bp, C* X, double tol, int itermax, int* iters, double* err, int* status) {
     C* R = blk(0); C* P = blk(1); C* R0 = blk(2); C* V = blk(3); C* Tm = blk(4); C* Z = blk(5); C* Pt = blk(6);
-    double2* p = w->partials.template as<double2>();
-    double2* p2 = w->partials2.template as<double2>();
     double2* vp = w->vpart.as<double2>();
     double2* scal = sl(kNumSlots);  // 2 scalars after the matrix slots
     BDDA_CUDA(cudaMemsetAsync(X, 0, sizeof(C) * (size_t)n * L, st));
@@ -734,10 +698,9 @@ struct Krylov {
     const int gv = vec_grid((size_t)n * L);
     BDDA_TRY(iterate(1, X, Bp, nullptr, false, itermax, [&](bool) -> int {
       BDDA_TRY(mvp(P, V));                                   // V = A P
-      gram<true>(R0, V, p);
-      gram<true>(R0, R, p2);
-      small_launch(k_small_solve<double>, (const double2*)p, (const double2*)p2, 1, L, small(), ctl(), 0, (int)kM, 1.0,
-                   (const double2*)nullptr, (int)kAlpha, (int)kNAlpha);
+      const GramRef rv = gram<true>(R0, V), rr = gram<true>(R0, R, 1);
+      small_launch(k_small_solve<double, GP>, rv, rr, L, small(), ctl(), 0, (int)kM, 1.0, (const double2*)nullptr, (int)kAlpha,
+                   (int)kNAlpha);
       rowmm(V, sl(kNAlpha), nullptr, nullptr, R, Tm);        // T = R - V alpha
       BDDA_TRY(mvp(Tm, Z));                                  // Z = A T
       dotc(Z, Tm, vp);
@@ -751,8 +714,7 @@ struct Krylov {
       op->timer.begin(kSmall, st);
       k_small_err<<<1, 256, 0, st>>>(w->vpart.as<double>(), gv, L, ctl(), w->hist.as<double>());
       op->timer.end(kSmall, st);
-      gram<true>(R0, Z, p);
-      small_launch(k_small_solve<double>, (const double2*)nullptr, (const double2*)p, 1, L, small(), ctl(), (int)kM, -1, -1.0,
+      small_launch(k_small_solve<double, GP>, GramRef{nullptr, 0, 0}, gram<true>(R0, Z), L, small(), ctl(), (int)kM, -1, -1.0,
                    (const double2*)nullptr, (int)kBeta, -1);  // beta = M^-1 (-R0^H Z)
       axpby(nullptr, P, scal + 1, V, Pt);                    // Pt = P - zeta V
       rowmm(Pt, sl(kBeta), nullptr, nullptr, R, P);          // P = R + Pt beta
@@ -767,8 +729,6 @@ struct Krylov {
   // Block BiCGGR (bl_bicggr_mvp_fft.cpp:18-116 / bl_bicggr_jacobi_mvp_fft.cpp:18-117)
   int bicggr(const C* Bp, C* X, double tol, int itermax, int* iters, double* err, int* status) {
     C* R = blk(0); C* P = blk(1); C* R0 = blk(2); C* V = blk(3); C* Wm = blk(4); C* U = blk(5); C* Y = blk(6); C* Rn = blk(7);
-    double2* p = w->partials.template as<double2>();
-    double2* p2 = w->partials2.template as<double2>();
     double2* vp = w->vpart.as<double2>();
     double2* scal = sl(kNumSlots);
     BDDA_CUDA(cudaMemsetAsync(X, 0, sizeof(C) * (size_t)n * L, st));
@@ -780,12 +740,10 @@ struct Krylov {
     BDDA_CUDA(cudaMemcpyAsync(Wm, V, sizeof(C) * (size_t)n * L, cudaMemcpyDeviceToDevice, st));
     const int gv = vec_grid((size_t)n * L);
     BDDA_TRY(iterate(2, X, Bp, &R, false, itermax, [&](bool) -> int {
-      gram<true>(R0, V, p);
-      gram<true>(R0, R, p2);
-      small_launch(k_small_solve<double>, (const double2*)p, (const double2*)p2, 1, L, small(), ctl(), 0, -1, 1.0,
-                   (const double2*)nullptr, (int)kAlpha, -1);
+      const GramRef rv = gram<true>(R0, V), rr = gram<true>(R0, R, 1);
+      small_launch(k_small_solve<double, GP>, rv, rr, L, small(), ctl(), 0, -1, 1.0, (const double2*)nullptr, (int)kAlpha, -1);
       // keep R0^H R (old R) for gamma
-      small_launch(k_small_store_reduce, (const double2*)p2, 1, L, small(), ctl(), (int)kM2);
+      small_launch(k_small_store_reduce<GP>, rr, L, small(), ctl(), (int)kM2);
       dotc(Wm, R, vp);
       dotc(Wm, Wm, vp + gv);
       op->timer.begin(kSmall, st);
@@ -801,8 +759,7 @@ struct Krylov {
       k_small_err<<<1, 256, 0, st>>>(w->vpart.as<double>(), gv, L, ctl(), w->hist.as<double>());
       op->timer.end(kSmall, st);
       BDDA_TRY(mvp(Rn, Wm));                                 // W = A Rnew
-      gram<true>(R0, Rn, p);
-      small_launch(k_small_solve<double>, (const double2*)nullptr, (const double2*)p, 1, L, small(), ctl(), (int)kM2, -1, 1.0,
+      small_launch(k_small_solve<double, GP>, GramRef{nullptr, 0, 0}, gram<true>(R0, Rn), L, small(), ctl(), (int)kM2, -1, 1.0,
                    (const double2*)scal, (int)kBeta, -1);    // gamma = (R0^H R)^-1 (R0^H Rnew / zeta)
       std::swap(R, Rn);
       rowmm(U, sl(kBeta), nullptr, nullptr, R, P);           // P = R + U gamma
@@ -852,7 +809,7 @@ static int ensure_work(Op* op, int n, int L, int itermax, bool need64, bool need
   BDDA_CUDA(w->diag32.ensure(sizeof(float2) * (size_t)n, op->stream));
   BDDA_CUDA(w->jpre32.ensure(sizeof(float2) * (size_t)n, op->stream));
   const size_t LL = (size_t)L * L;
-  BDDA_CUDA(w->gpart.ensure(sizeof(double2) * 2 * LL * gram_grid(n), op->stream));  // two Grams per CTA (gram2)
+  BDDA_CUDA(w->gpart.ensure(sizeof(double2) * 2 * LL * gram_grid(n), op->stream));  // two Grams per CTA
   BDDA_CUDA(w->partials.ensure(sizeof(double2) * 2 * LL, op->stream));
   BDDA_CUDA(w->partials2.ensure(sizeof(double2) * 2 * LL, op->stream));
   BDDA_CUDA(w->vpart.ensure(sizeof(double2) * 2 * (size_t)std::max(vec_grid((size_t)n * L) * L, 2 * 608), op->stream));
@@ -870,20 +827,18 @@ static int ensure_work(Op* op, int n, int L, int itermax, bool need64, bool need
       if (e != cudaSuccess) attr_err = e;
     };
     const int mx = (int)SmallSmem::bytes(kMaxL);
-    set((const void*)k_small_chol1<double>, mx);
-    set((const void*)k_small_chol2<double>, mx);
-    set((const void*)k_small_cocg_alpha<double>, mx);
-    set((const void*)k_small_cocg_beta<double>, mx);
-    set((const void*)k_small_solve<double>, mx);
-    set((const void*)k_small_chol1<dfl>, mx);
-    set((const void*)k_small_chol2<dfl>, mx);
-    set((const void*)k_small_cocg_alpha<dfl>, mx);
-    set((const void*)k_small_cocg_beta<dfl>, mx);
-    set((const void*)k_small_chol2_beta<double>, mx);
-    set((const void*)k_small_chol2_beta<dfl>, mx);
+    set((const void*)k_small_chol1<double, double2>, mx);
+    set((const void*)k_small_chol2<double, double2>, mx);
+    set((const void*)k_small_cocg_alpha<double, double2>, mx);
+    set((const void*)k_small_solve<double, double2>, mx);
+    set((const void*)k_small_solve<double, dfc>, mx);
+    set((const void*)k_small_chol1<dfl, dfc>, mx);
+    set((const void*)k_small_chol2<dfl, dfc>, mx);
+    set((const void*)k_small_cocg_alpha<dfl, dfc>, mx);
+    set((const void*)k_small_chol2_beta<double, double2>, mx);
+    set((const void*)k_small_chol2_beta<dfl, dfc>, mx);
     set((const void*)k_rowmm2<double>, rowmm_smem<double>(kMaxL, true));
     set((const void*)k_rowmm2<float>, rowmm_smem<float>(kMaxL, true));
-    set((const void*)k_small_store_reduce, mx);
     set((const void*)k_rowmm<double>, rowmm_smem<double>(kMaxL, true));
     set((const void*)k_rowmm<float>, rowmm_smem<float>(kMaxL, true));
   });
