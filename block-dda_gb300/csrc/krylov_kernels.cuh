@@ -7,6 +7,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "pdl.cuh"
 
 namespace bdda {
 
@@ -61,6 +62,7 @@ k_gram(const typename cplx<T>::type* __restrict__ A, int lda,
        int n, int L, typename GramPart<T>::type* __restrict__ partials, const SolverCtl* ctl) {
   using C = typename cplx<T>::type;
   using P = typename GramPart<T>::type;
+  pdl_begin();
   if (ctl_skip(ctl)) return;
   __shared__ C sa[kMaxL][kGramRows + 1];
   __shared__ C sb[kMaxL][kGramRows + 1];
@@ -147,6 +149,7 @@ constexpr int kRedEntries = 16, kRedGroups = 16;
 template <typename P>
 __global__ void __launch_bounds__(kRedEntries * kRedGroups)
 k_gram_reduce(const P* __restrict__ part, int nparts, int LL, double2* __restrict__ out, const SolverCtl* ctl) {
+  pdl_begin();
   if (ctl_skip(ctl)) return;
   __shared__ P red[kRedGroups][kRedEntries];
   const int el = threadIdx.x % kRedEntries, g = threadIdx.x / kRedEntries;
@@ -178,6 +181,7 @@ k_gram_reduce(const P* __restrict__ part, int nparts, int LL, double2* __restric
 template <typename T>
 __global__ void __launch_bounds__(256)
 k_colnorm2(const typename cplx<T>::type* __restrict__ A, int lda, int n, int L, double* __restrict__ partials) {
+  pdl_begin();
   using C = typename cplx<T>::type;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const long long rows_per = ((long long)n + gridDim.x - 1) / gridDim.x;
@@ -210,6 +214,7 @@ k_rowmm(int n, int L, const typename cplx<T>::type* A, int lda, const double2* _
   // before it writes, each Cadd element is read by the thread that then
   // writes it, and CTAs own disjoint rows.
   using C = typename cplx<T>::type;
+  pdl_begin();
   if (ctl_skip(ctl)) return;
   // dynamic smem: ta[L][kRowRows], tb[L][kRowRows], ma[L*L], mb[L*L]
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -251,6 +256,7 @@ k_rowmm2(int n, int L, const typename cplx<T>::type* A, const double2* __restric
          const typename cplx<T>::type* B, const double2* __restrict__ Mb,
          typename cplx<T>::type* Out1, typename cplx<T>::type* Out2, const SolverCtl* ctl) {
   using C = typename cplx<T>::type;
+  pdl_begin();
   if (ctl_skip(ctl)) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* ta = reinterpret_cast<C*>(smem_raw);
@@ -295,6 +301,7 @@ __global__ void k_axpby(int n, int L, const double2* __restrict__ a, const typen
                         const double2* __restrict__ b, const typename cplx<T>::type* B, int ldb,
                         typename cplx<T>::type* Out, int ldo, const SolverCtl* ctl) {
   using C = typename cplx<T>::type;
+  pdl_begin();
   if (ctl_skip(ctl)) return;
   const C ca = a ? cmake((T)a->x, (T)a->y) : cmake((T)1, (T)0);
   const C cb = b ? cmake((T)b->x, (T)b->y) : cmake((T)1, (T)0);
@@ -313,6 +320,7 @@ __global__ void __launch_bounds__(256)
 k_dotc(int n, int L, const typename cplx<T>::type* __restrict__ A, int lda,
        const typename cplx<T>::type* __restrict__ B, int ldb, double2* __restrict__ partials, const SolverCtl* ctl) {
   using C = typename cplx<T>::type;
+  pdl_begin();
   if (ctl_skip(ctl)) return;
   __shared__ double2 red[8];
   const size_t total = (size_t)n * L;

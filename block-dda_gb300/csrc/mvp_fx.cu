@@ -31,6 +31,7 @@
 
 #include "fx_fft.cuh"
 #include "mvp.hpp"
+#include "pdl.cuh"
 #include "tile_passes.cuh"
 
 namespace bdda {
@@ -169,6 +170,7 @@ __global__ void __launch_bounds__(kFxThreads, MB)
 k_fx_a(const typename Io::E* __restrict__ x, int ldx, int nfield, int fpg, int fc, const int* __restrict__ occ,
        const int* __restrict__ tiles, int nx, int ny, int nz, int nzp, int nzt, fx::Plan p, const Fac* __restrict__ tw,
        Val* __restrict__ t1, int* __restrict__ ea, const int* done) {
+  pdl_begin();
   if (skip(done)) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Val* lines = reinterpret_cast<Val*>(smem_raw);                 // [kTZ][LW]
@@ -220,6 +222,7 @@ __global__ void __launch_bounds__(kFxThreads, MB)
 k_fx_y(const Val* __restrict__ src, Val* __restrict__ dst, const unsigned char* __restrict__ tmask, int fc, int Px, int ny,
        int nz, int nzp, int nzt, fx::Plan p, const Fac* __restrict__ tw, const int* __restrict__ ein, int* __restrict__ eout,
        const int* done) {
+  pdl_begin();
   if (skip(done)) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Val* lines = reinterpret_cast<Val*>(smem_raw);          // [kTZ][LW]
@@ -264,6 +267,7 @@ k_fx_e(const Val* __restrict__ t1, const int* __restrict__ ein, int nfield, int 
        const int* __restrict__ tiles, int nx, int ny, int nz, int nzp, int nzt, fx::Plan p, const Fac* __restrict__ tw,
        const typename Io::E* __restrict__ x, int ldx, const typename Io::E* __restrict__ diag,
        const typename Io::E* __restrict__ jpre, typename Io::E* __restrict__ y, int ldy, const int* done) {
+  pdl_begin();
   if (skip(done)) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Val* lines = reinterpret_cast<Val*>(smem_raw);           // [kTZ][LW]
@@ -338,6 +342,7 @@ k_fx_c(Val* __restrict__ t2, int L, int Px, int Py, int nz, int nzp, fx::Plan p,
        const Fac* __restrict__ ghat, const int* __restrict__ gexp, const int* __restrict__ ein, int* __restrict__ eout,
        const int* done) {
   constexpr int fc = SIX ? 6 : 3, nc = SIX ? 9 : 6;
+  pdl_begin();
   if (skip(done)) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -608,12 +613,12 @@ cudaError_t launch(const MvpGeom& g, const FxTables& t, const void* xv, int ldx,
   const int asm_ = fx_smem(px, kTZ * g.nx), bsm = fx_smem(py, kTZ * g.ny), dsm = fx_smem(py, g.Py),
             esm = fx_smem(px, kTZ * (g.nx + g.Px));
   auto* ka = fits(kXMany, asm_) ? k_fx_a<Io, kXMany> : k_fx_a<Io, kXFew>;
-  ka<<<xgrid, kFxThreads, asm_, st>>>(x, ldx, nfield, fpg, g.f, g.occ, g.tiles, g.nx, g.ny, g.nz,
+  launch_pdl(ka, xgrid, kFxThreads, asm_, st, x, ldx, nfield, fpg, g.f, g.occ, g.tiles, g.nx, g.ny, g.nz,
                                                                  g.nzp, g.nzt, px, t.tw[0], t1, w.ea, done);
   end(kPassA64);
   begin(kPassB64);
   auto* kb = fits(kXMany, bsm) ? k_fx_y<false, kXMany> : k_fx_y<false, kXFew>;
-  kb<<<ygrid, kFxThreads, bsm, st>>>(t1, t2, g.tmask, g.f, g.Px, g.ny, g.nz, g.nzp, g.nzt, py,
+  launch_pdl(kb, ygrid, kFxThreads, bsm, st, t1, t2, g.tmask, g.f, g.Px, g.ny, g.nz, g.nzp, g.nzt, py,
                                                                     t.tw[1], w.ea, w.eb, done);
   end(kPassB64);
   begin(kPassC64);
@@ -623,17 +628,17 @@ cudaError_t launch(const MvpGeom& g, const FxTables& t, const void* xv, int ldx,
     const long long ntask = (long long)g.Px * g.Py * L;
     const unsigned grid = (unsigned)((ntask + wpc - 1) / wpc);
     auto* kc = g.f == 6 ? k_fx_c<true, kCSix> : fits(kCMany, wpc * per_warp) ? k_fx_c<false, kCMany> : k_fx_c<false, kCFew>;
-    kc<<<grid, wpc * 32, wpc * per_warp, st>>>(t2, L, g.Px, g.Py, g.nz, g.nzp, pz, t.tw[2], t.ghat, t.gexp, w.eb, w.ec, done);
+    launch_pdl(kc, grid, wpc * 32, wpc * per_warp, st, t2, L, g.Px, g.Py, g.nz, g.nzp, pz, t.tw[2], t.ghat, t.gexp, w.eb, w.ec, done);
   }
   end(kPassC64);
   begin(kPassD64);
   auto* kd = fits(kXMany, dsm) ? k_fx_y<true, kXMany> : k_fx_y<true, kXFew>;
-  kd<<<ygrid, kFxThreads, dsm, st>>>(t2, t1, g.tmask, g.f, g.Px, g.ny, g.nz, g.nzp, g.nzt, py, t.tw[1],
+  launch_pdl(kd, ygrid, kFxThreads, dsm, st, t2, t1, g.tmask, g.f, g.Px, g.ny, g.nz, g.nzp, g.nzt, py, t.tw[1],
                                                              w.ec, w.eb, done);
   end(kPassD64);
   begin(kPassE64);
   auto* ke = fits(kXMany, esm) ? k_fx_e<Io, kXMany> : k_fx_e<Io, kXFew>;
-  ke<<<xgrid, kFxThreads, esm, st>>>(t1, w.eb, nfield, fpg, g.f, g.occ, g.tiles, g.nx, g.ny,
+  launch_pdl(ke, xgrid, kFxThreads, esm, st, t1, w.eb, nfield, fpg, g.f, g.occ, g.tiles, g.nx, g.ny,
                                                                           g.nz, g.nzp, g.nzt, px, t.tw[0], x, ldx, diag, jpre,
                                                                           y, ldy, done);
   end(kPassE64);

@@ -292,6 +292,7 @@ __device__ bool core_alpha(const SmallWork<R>& w, int L, double2* st, SolverCtl*
 template <typename R, typename P>
 __global__ void __launch_bounds__(kSmallThreads)
 k_small_chol1(GramRef part, int L, double2* st, SolverCtl* ctl) {
+  pdl_begin();
   if (ctl_skip(ctl)) return;
   SMALL_PROLOGUE
   sm_gram<R, P>(m0, part, 0, LL);
@@ -305,6 +306,7 @@ k_small_chol1(GramRef part, int L, double2* st, SolverCtl* ctl) {
 template <typename R, typename P>
 __global__ void __launch_bounds__(kSmallThreads)
 k_small_chol2(GramRef part, int L, double2* st, SolverCtl* ctl, int mode) {
+  pdl_begin();
   if (ctl_skip(ctl)) return;
   SMALL_PROLOGUE
   sm_gram<R, P>(m0, part, 0, LL);
@@ -326,6 +328,7 @@ k_small_chol2(GramRef part, int L, double2* st, SolverCtl* ctl, int mode) {
 template <typename R, typename P>
 __global__ void __launch_bounds__(kSmallThreads)
 k_small_chol2_beta(GramRef part, int L, double2* st, SolverCtl* ctl, double* hist, int full) {
+  pdl_begin();
   if (ctl_skip(ctl)) return;
   SMALL_PROLOGUE
   sm_load(m3, slot(st, kR1, L), LL);
@@ -342,6 +345,7 @@ k_small_chol2_beta(GramRef part, int L, double2* st, SolverCtl* ctl, double* his
 template <typename R, typename P>
 __global__ void __launch_bounds__(kSmallThreads)
 k_small_cocg_alpha(GramRef pSAS, GramRef pQQ, int L, double2* st, SolverCtl* ctl, int full) {
+  pdl_begin();
   if (ctl_skip(ctl)) return;
   SMALL_PROLOGUE
   if (pQQ.p) {
@@ -363,6 +367,7 @@ template <typename R, typename P>
 __global__ void __launch_bounds__(kSmallThreads)
 k_small_solve(GramRef pM, GramRef pR, int L, double2* st, SolverCtl* ctl, int mslot_in, int mslot_store, double rhs_scale,
               const double2* scal_div, int so, int sno) {
+  pdl_begin();
   if (ctl_skip(ctl)) return;
   SMALL_PROLOGUE
   if (pM.p) sm_gram<R, P>(m0, pM, 0, LL);
@@ -383,6 +388,7 @@ k_small_solve(GramRef pM, GramRef pR, int L, double2* st, SolverCtl* ctl, int ms
 // zeta = sum(p1) / sum(p2) ; kZetaI = zeta I ; kNZetaI = -zeta I ; scal[0] = zeta, scal[1] = -zeta
 __global__ void k_small_zeta(const double2* __restrict__ p1, const double2* __restrict__ p2, int nparts, int L, double2* st,
                              double2* scal, SolverCtl* ctl) {
+  pdl_begin();
   if (ctl_skip(ctl)) return;
   __shared__ double2 z;
   if (threadIdx.x == 0) {
@@ -409,6 +415,7 @@ __global__ void k_small_zeta(const double2* __restrict__ p1, const double2* __re
 // The iteration index and tolerance come from the control block (captured cycles).
 __global__ void __launch_bounds__(256) k_small_err(const double* __restrict__ vpart, int nparts, int L, SolverCtl* ctl,
                                                    double* hist) {
+  pdl_begin();
   if (ctl_skip(ctl)) return;
   const double s = block_sum_256(vpart, nparts * L);
   if (threadIdx.x == 0) {
@@ -425,6 +432,7 @@ __global__ void __launch_bounds__(256) k_small_err(const double* __restrict__ vp
 // st[s] = reduce(partials)
 template <typename P>
 __global__ void __launch_bounds__(kSmallThreads) k_small_store_reduce(GramRef part, int L, double2* st, SolverCtl* ctl, int s) {
+  pdl_begin();
   if (ctl_skip(ctl)) return;
   sm_gram<double, P>(slot(st, s, L), part, 0, L * L);
 }
@@ -467,11 +475,11 @@ struct Krylov {
     const int LL = L * L, LLo = BOTH ? 2 * LL : LL;
     GP* part = w->gpart.template as<GP>() + (size_t)which * LL * G();
     op->timer.begin(kGram, st);
-    k_gram<T, CONJ, BOTH><<<G(), kGramThreads, 0, st>>>(A, n, B, n, n, L, part, ctl());
+    launch_pdl(k_gram<T, CONJ, BOTH>, G(), kGramThreads, 0, st, A, n, B, n, n, L, part, ctl());
     GramRef r{part, G(), LLo};
     if (L > kWarpL) {
       double2* out = (which ? w->partials2 : w->partials).template as<double2>();
-      k_gram_reduce<GP><<<(LLo + kRedEntries - 1) / kRedEntries, kRedEntries * kRedGroups, 0, st>>>(part, G(), LLo, out, ctl());
+      launch_pdl(k_gram_reduce<GP>, (LLo + kRedEntries - 1) / kRedEntries, kRedEntries * kRedGroups, 0, st, part, G(), LLo, out, ctl());
       op->timer.count(kGram);
       r = GramRef{out, 0, LLo};
     }
@@ -481,34 +489,34 @@ struct Krylov {
   // Out1 = A Ma ; Out2 = Out1 + B Mb
   void rowmm2(const C* A, const double2* Ma, const C* B, const double2* Mb, C* Out1, C* Out2) {
     op->timer.begin(kUpdate, st);
-    k_rowmm2<T><<<(n + kRowRows - 1) / kRowRows, kRowThreads, rowmm_smem<T>(L, true), st>>>(n, L, A, Ma, B, Mb, Out1,
+    launch_pdl(k_rowmm2<T>, (n + kRowRows - 1) / kRowRows, kRowThreads, rowmm_smem<T>(L, true), st, n, L, A, Ma, B, Mb, Out1,
                                                                                          Out2, ctl());
     op->timer.end(kUpdate, st);
   }
   void rowmm(const C* A, const double2* Ma, const C* B, const double2* Mb, const C* Cadd, C* Out) {
     op->timer.begin(kUpdate, st);
-    k_rowmm<T><<<(n + kRowRows - 1) / kRowRows, kRowThreads, rowmm_smem<T>(L, B != nullptr), st>>>(
+    launch_pdl(k_rowmm<T>, (n + kRowRows - 1) / kRowRows, kRowThreads, rowmm_smem<T>(L, B != nullptr), st,
         n, L, A, n, Ma, B, n, Mb, Cadd, n, Out, n, ctl());
     op->timer.end(kUpdate, st);
   }
   void axpby(const double2* a, const C* A, const double2* b, const C* B, C* Out) {
     op->timer.begin(kUpdate, st);
-    k_axpby<T><<<vec_grid((size_t)n * L), 256, 0, st>>>(n, L, a, A, n, b, B, n, Out, n, ctl());
+    launch_pdl(k_axpby<T>, vec_grid((size_t)n * L), 256, 0, st, n, L, a, A, n, b, B, n, Out, n, ctl());
     op->timer.end(kUpdate, st);
   }
   void dotc(const C* A, const C* B, double2* part) {
     op->timer.begin(kGram, st);
-    k_dotc<T><<<vec_grid((size_t)n * L), 256, 0, st>>>(n, L, A, n, B, n, part, ctl());
+    launch_pdl(k_dotc<T>, vec_grid((size_t)n * L), 256, 0, st, n, L, A, n, B, n, part, ctl());
     op->timer.end(kGram, st);
   }
   void colnorm(const C* A, double* part) {
     op->timer.begin(kGram, st);
-    k_colnorm2<T><<<vec_grid((size_t)n * L), 256, 0, st>>>(A, n, n, L, part);
+    launch_pdl(k_colnorm2<T>, vec_grid((size_t)n * L), 256, 0, st, A, n, n, L, part);
     op->timer.end(kGram, st);
   }
   template <typename K, typename... Args> void small_launch(K kern, Args... args) {
     op->timer.begin(kSmall, st);
-    kern<<<1, kSmallThreads, SmallSmem::bytes(L), st>>>(args...);
+    launch_pdl(kern, 1, kSmallThreads, SmallSmem::bytes(L), st, args...);
     op->timer.end(kSmall, st);
   }
 
@@ -706,13 +714,13 @@ struct Krylov {
       dotc(Z, Tm, vp);
       dotc(Z, Z, vp + gv);
       op->timer.begin(kSmall, st);
-      k_small_zeta<<<1, 256, 0, st>>>(vp, vp + gv, gv, L, small(), scal, ctl());
+      launch_pdl(k_small_zeta, 1, 256, 0, st, vp, vp + gv, gv, L, small(), scal, ctl());
       op->timer.end(kSmall, st);
       rowmm(P, sl(kAlpha), Tm, sl(kZetaI), X, X);            // X = X + P alpha + zeta T
       axpby(nullptr, Tm, scal + 1, Z, R);                    // R = T - zeta Z
       colnorm(R, w->vpart.as<double>());
       op->timer.begin(kSmall, st);
-      k_small_err<<<1, 256, 0, st>>>(w->vpart.as<double>(), gv, L, ctl(), w->hist.as<double>());
+      launch_pdl(k_small_err, 1, 256, 0, st, w->vpart.as<double>(), gv, L, ctl(), w->hist.as<double>());
       op->timer.end(kSmall, st);
       small_launch(k_small_solve<double, GP>, GramRef{nullptr, 0, 0}, gram<true>(R0, Z), L, small(), ctl(), (int)kM, -1, -1.0,
                    (const double2*)nullptr, (int)kBeta, -1);  // beta = M^-1 (-R0^H Z)
@@ -747,7 +755,7 @@ struct Krylov {
       dotc(Wm, R, vp);
       dotc(Wm, Wm, vp + gv);
       op->timer.begin(kSmall, st);
-      k_small_zeta<<<1, 256, 0, st>>>(vp, vp + gv, gv, L, small(), scal, ctl());
+      launch_pdl(k_small_zeta, 1, 256, 0, st, vp, vp + gv, gv, L, small(), scal, ctl());
       op->timer.end(kSmall, st);
       axpby(nullptr, P, scal + 1, V, Rn);                    // S = P - zeta V   (Rn as scratch)
       rowmm(Rn, sl(kAlpha), nullptr, nullptr, nullptr, U);   // U = S alpha
@@ -756,7 +764,7 @@ struct Krylov {
       rowmm(Wm, sl(kNZetaI), Y, sl(kNIdent), R, Rn);         // Rn = R - zeta W - Y
       colnorm(Rn, w->vpart.as<double>());
       op->timer.begin(kSmall, st);
-      k_small_err<<<1, 256, 0, st>>>(w->vpart.as<double>(), gv, L, ctl(), w->hist.as<double>());
+      launch_pdl(k_small_err, 1, 256, 0, st, w->vpart.as<double>(), gv, L, ctl(), w->hist.as<double>());
       op->timer.end(kSmall, st);
       BDDA_TRY(mvp(Rn, Wm));                                 // W = A Rnew
       small_launch(k_small_solve<double, GP>, GramRef{nullptr, 0, 0}, gram<true>(R0, Rn), L, small(), ctl(), (int)kM2, -1, 1.0,

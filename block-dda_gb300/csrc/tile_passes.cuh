@@ -16,6 +16,7 @@
 
 #include "fft_core.cuh"
 #include "mvp.hpp"
+#include "pdl.cuh"
 #include "static_fft.cuh"
 
 namespace bdda {
@@ -258,6 +259,7 @@ __global__ void __launch_bounds__(kTileThreads)
 k_pass_a2i(const float2* __restrict__ x, int ldx, int nfield, int fpg, int fc, const int* __restrict__ occ,
            const int* __restrict__ tiles, int nx, int ny, int nz, int nzp, int nzt, const float2* __restrict__ twx,
            float2* __restrict__ t1, const int* done) {
+  pdl_begin();
   if (skip(done)) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   constexpr int Px = P::N;
@@ -324,6 +326,7 @@ k_pass_e2i(const float2* __restrict__ t1, int nfield, int fpg, int fc, const int
            const int* __restrict__ tiles, int nx, int ny, int nz, int nzp, int nzt, const float2* __restrict__ twx,
            const float2* __restrict__ x, int ldx, const float2* __restrict__ diag, const float2* __restrict__ jpre,
            float2* __restrict__ y, int ldy, const int* done) {
+  pdl_begin();
   if (skip(done)) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   constexpr int Px = P::N;

@@ -36,11 +36,11 @@ cudaError_t launch_x(int pass, const TileArgs& a) {
   cudaError_t e = cudaSuccess;
   if (pass == kTileA) {
     if ((e = set_smem(tile::k_pass_a2i<P>, smem_ae, oa, ca)) != cudaSuccess) return e;
-    tile::k_pass_a2i<P><<<grid, kTileThreads, smem_x2(g.nx), a.st>>>(
+    launch_pdl(tile::k_pass_a2i<P>, grid, kTileThreads, smem_x2(g.nx), a.st,
         a.x, a.ldx, a.nfield, fpg, g.f, g.occ, g.tiles, g.nx, g.ny, g.nz, g.nzp, g.nzt, a.twx, a.t1, a.done);
   } else {
     if ((e = set_smem(tile::k_pass_e2i<P>, smem_ae, oe, ce)) != cudaSuccess) return e;
-    tile::k_pass_e2i<P><<<grid, kTileThreads, smem_x2(g.nx), a.st>>>(
+    launch_pdl(tile::k_pass_e2i<P>, grid, kTileThreads, smem_x2(g.nx), a.st,
         a.t1, a.nfield, fpg, g.f, g.occ, g.tiles, g.nx, g.ny, g.nz, g.nzp, g.nzt, a.twx, a.x, a.ldx, a.diag, a.jpre, a.y,
         a.ldy, a.done);
   }

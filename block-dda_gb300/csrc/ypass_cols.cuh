@@ -26,6 +26,7 @@
 #include <mutex>
 
 #include "mvp.hpp"
+#include "pdl.cuh"
 #include "pfft.cuh"
 #include "static_fft.cuh"
 #include "tile_passes.cuh"
@@ -157,6 +158,7 @@ template <bool INV, class P, int NBUF>
 __global__ void __launch_bounds__(threads<P>(), min_blocks<P>())
 k_pass_y(const float2* __restrict__ src, float2* __restrict__ dst, const unsigned char* __restrict__ tmask, int ny, int nz,
          int nzp, int nzt, int ntask, const float4* __restrict__ tw, const int* done) {
+  pdl_begin();
   if (done && *(volatile const int*)done) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   constexpr int Py = P::N, T = threads<P>(), step = T / kPairs;
@@ -249,7 +251,7 @@ cudaError_t launch_buf(const TileArgs& a, int waves, int ntask) {
       resident = nb;
   });
   if (cfg != cudaSuccess) return cfg;
-  k_pass_y<INV, P, NBUF><<<std::min(ntask, waves * resident * a.sms), threads<P>(), smem, a.st>>>(
+  launch_pdl(k_pass_y<INV, P, NBUF>, std::min(ntask, waves * resident * a.sms), threads<P>(), smem, a.st,
       INV ? a.t2 : a.t1, INV ? a.t1 : a.t2, g.tmask, g.ny, g.nz, g.nzp, g.nzt, ntask, a.twyp, a.done);
   return cudaGetLastError();
 }

@@ -14,6 +14,7 @@
 #include <mutex>
 
 #include "mvp.hpp"
+#include "pdl.cuh"
 #include "pfft.cuh"
 #include "static_fft.cuh"
 
@@ -57,6 +58,7 @@ template <class P>
 __global__ void __launch_bounds__(kZWarps * 32)
 k_pass_c_packed(float2* __restrict__ t2, int L, int Px, int Py, int nz, int nzp, const float4* __restrict__ twz,
                 const float2* __restrict__ ghat, const int* done) {
+  pdl_begin();
   if (done && *(volatile const int*)done) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   constexpr int Pz = P::N, LW = P::LW;
@@ -127,7 +129,7 @@ cudaError_t launch(const MvpGeom& g, float2* t2, int L, const float4* twz, const
   const int wpc = z_warps_per_cta(per_warp);
   const long long ntask = (long long)g.Px * g.Py * ((L + 1) / 2);
   const unsigned grid = (unsigned)((ntask + wpc - 1) / wpc);
-  k_pass_c_packed<P><<<grid, wpc * 32, wpc * per_warp, st>>>(t2, L, g.Px, g.Py, g.nz, g.nzp, twz, ghat, done);
+  launch_pdl(k_pass_c_packed<P>, grid, wpc * 32, wpc * per_warp, st, t2, L, g.Px, g.Py, g.nz, g.nzp, twz, ghat, done);
   return cudaGetLastError();
 }
 

@@ -34,6 +34,7 @@
 
 #include "async_copy.cuh"
 #include "mvp.hpp"
+#include "pdl.cuh"
 #include "static_fft.cuh"
 #include "zproduct.cuh"
 
@@ -68,6 +69,7 @@ template <class P>
 __global__ void __launch_bounds__(kZWarps * 32)
 k_pass_c_pipe(float2* __restrict__ t2, int L, int nlines, int nz, int nzp, const float2* __restrict__ twz,
               const float2* __restrict__ ghat, const int* done, int* status, int stall) {
+  pdl_begin();
   if (done && *(volatile const int*)done) return;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   constexpr int Pz = P::N, LW = P::LW;
@@ -216,7 +218,7 @@ bool launch(const MvpGeom& g, float2* t2, int L, const float2* twz, const float2
   }
   const long long nlines = (long long)g.Px * g.Py;
   const long long grid = std::min<long long>(nlines, (long long)per_sm * nsm);
-  k_pass_c_pipe<P><<<(unsigned)grid, nw * 32, bytes, st>>>(t2, L, (int)nlines, g.nz, g.nzp, twz, ghat, done, g.kstat,
+  launch_pdl(k_pass_c_pipe<P>, (unsigned)grid, nw * 32, bytes, st, t2, L, (int)nlines, g.nz, g.nzp, twz, ghat, done, g.kstat,
                                                              g.zstall);
   *err = cudaGetLastError();
   return true;

@@ -15,6 +15,7 @@
 #include <mutex>
 
 #include "mvp.hpp"
+#include "pdl.cuh"
 #include "static_fft.cuh"
 #include "zproduct.cuh"
 
@@ -26,6 +27,7 @@ __global__ void __launch_bounds__(kZWarps * 32)
 k_pass_c_static(C* __restrict__ t2, int L, int Px, int Py, int nz, int nzp, const C* __restrict__ twz,
                 const C* __restrict__ ghat, const int* done) {
   constexpr int fc = SIX ? 6 : 3;
+  pdl_begin();
   if (done && *(volatile const int*)done) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   constexpr int Pz = P::N, LW = P::LW;
@@ -72,7 +74,7 @@ cudaError_t launch_f(const MvpGeom& g, C* t2, int L, const C* twz, const C* ghat
   const int wpc = z_warps_per_cta(per_warp);
   const long long ntask = (long long)g.Px * g.Py * L;
   const unsigned grid = (unsigned)((ntask + wpc - 1) / wpc);
-  k_pass_c_static<P, SIX, C><<<grid, wpc * 32, wpc * per_warp, st>>>(t2, L, g.Px, g.Py, g.nz, g.nzp, twz, ghat, done);
+  launch_pdl(k_pass_c_static<P, SIX, C>, grid, wpc * 32, wpc * per_warp, st, t2, L, g.Px, g.Py, g.nz, g.nzp, twz, ghat, done);
   return cudaGetLastError();
 }
 
