@@ -94,7 +94,7 @@ template <typename T> struct MvpPrec {
   const C* ghat;  // [Px][Py][6 or 9][Pz] (digit-reversed frequencies), divided by Px*Py*Pz
   const float4* twzp = nullptr;  // complex FP32: z twiddle pairs {wx, wx, wy, wy} (packed z pass)
   // staged tables (stage_twiddles) of the compile-time-plan kernels: x, y pairs, z, z pairs (packed z pass)
-  const C* twxs = nullptr;
+  const float4* twxps = nullptr;
   const float4* twyps = nullptr;
   const C* twzs = nullptr;
   const float4* twzps = nullptr;
@@ -234,8 +234,8 @@ struct TileArgs {
   const float2* jpre;
   float2* t1;
   float2* t2;
-  const float2* twx;   // staged x twiddles
-  const float4* twyp;  // staged y twiddle pairs {wx, wx, wy, wy}
+  const float4* twxp;  // staged twiddle pairs {wx, wx, wy, wy} of x and y
+  const float4* twyp;
   int sms;              // multiprocessors of the device
   cudaStream_t st;
   const int* done;

@@ -82,9 +82,9 @@ Op::~Op() {
   solver.reset();
   for (auto* o : {&dip, &cub}) { o->occ.release(); o->tiles.release(); o->tmask.release(); }
   for (int i = 0; i < 3; ++i) {
-    tw32[i].release(); twfx[i].release(); tw32p[i].release(); tws32[i].release(); tws32p[i].release();
+    tw32[i].release(); twfx[i].release(); tw32p[i].release(); tws32p[i].release();
   }
-  fxpos.release();
+  tws32z.release(); fxpos.release();
   ghat32.release(); ghatfx.release(); gexpfx.release();
   kstat.release();
   for (int i = 0; i < 2; ++i) { t1[i].release(); t2[i].release(); }
@@ -425,11 +425,11 @@ int bdda_op_create(bdda_op** out, const int n[3], int f, double lf, double k_re,
       tsf[t] = make_float2((float)ts[t].x, (float)ts[t].y);
       tsp[t] = make_float4(tsf[t].x, tsf[t].x, tsf[t].y, tsf[t].y);
     }
-    BDDA_CUDA(op->tws32[i].ensure(nts * sizeof(float2), op->stream));
-    BDDA_CUDA(cudaMemcpyAsync(op->tws32[i].p, tsf.data(), nts * sizeof(float2), cudaMemcpyHostToDevice, op->stream));
-    if (i > 0) {
-      BDDA_CUDA(op->tws32p[i].ensure(nts * sizeof(float4), op->stream));
-      BDDA_CUDA(cudaMemcpyAsync(op->tws32p[i].p, tsp.data(), nts * sizeof(float4), cudaMemcpyHostToDevice, op->stream));
+    BDDA_CUDA(op->tws32p[i].ensure(nts * sizeof(float4), op->stream));
+    BDDA_CUDA(cudaMemcpyAsync(op->tws32p[i].p, tsp.data(), nts * sizeof(float4), cudaMemcpyHostToDevice, op->stream));
+    if (i == 2) {
+      BDDA_CUDA(op->tws32z.ensure(nts * sizeof(float2), op->stream));
+      BDDA_CUDA(cudaMemcpyAsync(op->tws32z.p, tsf.data(), nts * sizeof(float2), cudaMemcpyHostToDevice, op->stream));
     }
     BDDA_CUDA(wait_stream(op->stream));  // tw / tf / ts die at the end of this iteration
   }

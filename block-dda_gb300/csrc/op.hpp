@@ -92,9 +92,9 @@ struct Op {
   DevBuf fxpos;     // int [3][kMaxLine]: the complex FP32 order's positions in the fixed-point order
   DevBuf tw32p[3];  // complex FP32 twiddle pairs {wx, wx, wy, wy} of the packed z pass ([2] only)
   // staged twiddles (stage_twiddles) of the compile-time-plan kernels: complex
-  // FP32 per axis, as pairs {wx, wx, wy, wy} for the y passes and the packed z pass.  Every DevBuf of the operator is
+  // FP32 along z, and per axis as pairs {wx, wx, wy, wy}.  Every DevBuf of the operator is
   // released in ~Op, before its stream is destroyed.
-  DevBuf tws32[3], tws32p[3];
+  DevBuf tws32z, tws32p[3];
   DevBuf ghat32, ghatfx, gexpfx;  // Green spectra: complex FP32; Q62 with its exponents
   DevBuf kstat;     // int: status word of the pipelined z pass (take_kernel_status)
   Occupancy dip;    // dipole occupancy (set_dipoles)
@@ -122,10 +122,10 @@ struct Op {
   unsigned long long buffer_sig() const {
     unsigned long long h = 0;
     for (int i = 0; i < 3; ++i)
-      for (const DevBuf* b : {&tw32[i], &twfx[i], &tw32p[i], &tws32[i], &tws32p[i]}) h = sig_add(h, *b);
+      for (const DevBuf* b : {&tw32[i], &twfx[i], &tw32p[i], &tws32p[i]}) h = sig_add(h, *b);
     for (int i = 0; i < 2; ++i)
       for (const DevBuf* b : {&t1[i], &t2[i]}) h = sig_add(h, *b);
-    for (const DevBuf* b : {&texp, &ghat32, &ghatfx, &gexpfx, &kstat, &dip.occ, &dip.tiles, &dip.tmask})
+    for (const DevBuf* b : {&texp, &ghat32, &ghatfx, &gexpfx, &tws32z, &kstat, &dip.occ, &dip.tiles, &dip.tmask})
       h = sig_add(h, *b);
     return h;
   }
@@ -151,7 +151,7 @@ struct Op {
   }
   MvpPrec<float> tables32() const {
     return {tw32[0].as<float2>(), tw32[1].as<float2>(), tw32[2].as<float2>(), ghat32.as<float2>(), tw32p[2].as<float4>(),
-            tws32[0].as<float2>(), tws32p[1].as<float4>(), tws32[2].as<float2>(), tws32p[2].as<float4>()};
+            tws32p[0].as<float4>(), tws32p[1].as<float4>(), tws32z.as<float2>(), tws32p[2].as<float4>()};
   }
   FxTables tables_fx() const {
     return {{fxplan[0], fxplan[1], fxplan[2]},

@@ -3,8 +3,7 @@
 // the plan tables) so that the build compiles them in parallel.
 #pragma once
 
-#include "tile_static.cuh"
-#include "ypass_cols.cuh"
+#include "xpass_cols.cuh"
 #include "zpass_packed.cuh"
 #include "zpass_pipe.cuh"
 #include "zpass_static.cuh"
@@ -49,7 +48,7 @@ bool dispatch_tile(int pass, const TileArgs& a, cudaError_t* err) {
 #define BDDA_TPLAN(I, N, S, LW, ...)                                                     \
   case N:                                                                                \
     if constexpr ((I) % kParts == PART) {                                                \
-      *err = tstatic::launch_x<sfft::Plan<N, S, LW, __VA_ARGS__>>(pass, a);              \
+      *err = xcol::launch<sfft::Plan<N, S, LW, __VA_ARGS__>>(pass, a);                   \
       return true;                                                                       \
     }                                                                                    \
     return false;
