@@ -38,6 +38,7 @@ def _sources():
 
 def _inputs():
     return _sources() + glob.glob(os.path.join(CSRC, "*.cuh")) + glob.glob(os.path.join(CSRC, "*.hpp")) + \
+        glob.glob(os.path.join(CSRC, "*.inc")) + \
         [os.path.join(REPO, "include", "bdda.h"), os.path.abspath(__file__)]
 
 

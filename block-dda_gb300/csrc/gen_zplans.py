@@ -9,8 +9,9 @@
               line triple instead of four or more
   zwplans.inc three-line plans of the 16-byte z passes (FP64 / double-float:
               register radices <= 16, no fused step)
-  tplans.inc  single-line plans of the strided x / y passes (one warp per
-              line, eight lines per CTA filled and drained as a tile)
+  tplans.inc  plans of the strided x / y passes: the radix sequences of the
+              column-pair kernels (column_radices); S and LW are the layout
+              for one warp per line, which those kernels do not use
 
 For every 5-smooth line length 2 <= N <= 512 it picks, among the radix
 sequences with the fewest or one more than the fewest stages (register
@@ -26,10 +27,9 @@ Bank model: 32 banks of 4 bytes; 8-byte accesses are served per half-warp and
 a group takes as many wavefronts as the largest number of distinct words in one
 bank (this reproduces the shared-memory wavefront counts ncu reports).
 
-  yplans.inc  the column-pair y passes (two lines interleaved element by
-              element per warp): the radix sequences of tplans.inc, the
-              padded layout chosen for the interleaved pairs and the 16-byte
-              tile fill / drain of eight column pairs
+  yplans.inc  the y passes: the radix sequences of tplans.inc; S and LW are
+              the layout for two lines interleaved element by element, which
+              the column-pair kernels do not use
 
 Usage: python gen_zplans.py [z] [zw] [t] [il]   (writes the tables beside it;
        il reads the radix sequences from tplans.inc)
@@ -239,7 +239,7 @@ def stage_cost_il(n, rad, S, LW):
 
 
 def cost_y_il(n, rad, S, LW):
-    """One line pair of a column-pair y pass (k_pass_y2i): its transform plus
+    """One interleaved line pair of a tile: its transform plus
     its share of the tile fill and drain, where the eight lanes of a
     quarter-warp move one row of the task's eight column pairs (pair p of row
     r at 16-byte chunk p LW + addr(r)), over the n rows of the padded line."""
@@ -282,6 +282,64 @@ def choose(n, cost, first=RADICES, max_pad=None):
                 if best is None or key < best[0]:
                     best = (key, rad, S, LW)
     return best[1], best[2], best[3]
+
+
+COL_PAIRS = 8           # column pairs of a tile of the x / y passes (kPairs)
+COL_SMEM = 228 * 1024   # shared memory of an SM
+COL_MAX_N = 360         # lines column_radices chooses for
+
+
+def column_cost(n, rad):
+    """Threads-per-CTA rule of ypass_cols.cuh: the rounds of a stage's
+    butterfly threads, weighted by its radix, at the best CTA size, over the
+    threads per SM, up to 896, that registers and tiles admit."""
+    regs = 768 if max(rad) > 10 else 1024
+    best = None
+    for t in range(64, 385, 32):
+        c = sum(-(-COL_PAIRS * (n // r) // t) * t * r for r in rad)
+        ctas = min(regs // t, COL_SMEM // (n * 16 * COL_PAIRS + 1024))
+        c = c / min(ctas * t, 896)
+        best = c if best is None else min(best, c)
+    return best
+
+
+def column_radices(n):
+    """Radix sequence of the column-pair x / y passes (ypass_cols.cuh), which
+    pay for exchanges between stages and have no bank conflicts to model: the
+    fewest stages (two for the short lines that one radix would do, so that a
+    tile has more than eight threads); of two-stage sequences the one with the
+    smallest largest radix (registers), of longer ones that of least
+    column_cost.  Ascending, so that the inverse pass, whose first stage reads
+    global memory, starts with the largest radix.  Both y passes / both x
+    passes, ps per point, against the sequences of cost_tile at the same CTA
+    sizes: 120 = 10 12 for 6 4 5 4.0 / 5.7 from 5.1 / 7.3; 90 = 9 10 for 6 3 5
+    4.7 / 6.2 from 5.1 / 7.0; 270 = 3 9 10 for 3 10 9 5.0 / 6.3 from 5.1 / 6.5;
+    288 = 4 8 9 for 9 2 16 4.9 / 6.2 from 5.9 / 7.1; 360 = 4 9 10 for 2 12 15
+    6.7 / 6.6 from 7.1 / 7.1.  Lines above COL_MAX_N, of which an SM holds four
+    tiles at most, keep cost_tile's: 400 = 4 10 10 for 5 5 16 measured 7.0 /
+    6.5 against 6.8 / 6.4, 512 = 2 16 16 for 8 4 16 8.8 / 8.4 against 7.8 / 7.3."""
+    best = None
+
+    def rec(rem, lo, cur):
+        nonlocal best
+        if rem == 1:
+            if len(cur) > 1 or n <= 5:
+                key = (len(cur), max(cur) if len(cur) < 3 else column_cost(n, cur), [-r for r in cur])
+                best = key if best is None else min(best, key)
+            return
+        for r in sorted(RADICES):
+            if r >= lo and rem % r == 0:
+                rec(rem // r, r, cur + [r])
+    rec(n, 2, [])
+    return tuple(-r for r in best[2])
+
+
+def t_entry(n):
+    """Plan of the x / y table."""
+    if n > COL_MAX_N:
+        return choose(n, cost_tile)
+    rad = column_radices(n)
+    return (rad,) + choose_layout(n, rad, cost_tile)
 
 
 FUSED_WIDE_MIN_N = 181  # kFusedWideMinN: shorter z lines keep the packed-pair kernel's plans
@@ -343,12 +401,9 @@ def main():
     here = os.path.dirname(os.path.abspath(__file__))
     which = sys.argv[1:] or ["z", "t"]
     if "il" in which:
-        # the column-pair y passes: the radix sequences of the single-line
-        # table (they fix the digit order the Green spectrum is packed in),
-        # the layout for interleaved line pairs and 16-byte rows of eight
-        # pairs.  (The x passes drain two rows of four pairs per quarter-warp;
-        # modelled the same way, tplans.inc's layouts are already as good
-        # there, so they keep that table.)
+        # the y passes: the radix sequences of the x / y table (they fix the
+        # digit order the Green spectrum is packed in), the layout for
+        # interleaved line pairs and 16-byte rows of eight pairs
         rad = read_radices(os.path.join(here, "tplans.inc"), "BDDA_TPLAN")
         write_il(os.path.join(here, "yplans.inc"), "BDDA_YPLAN",
                  "column-pair y passes (line pairs interleaved, eight pairs per task)", cost_y_il, rad)
@@ -360,8 +415,8 @@ def main():
         write(os.path.join(here, "zwplans.inc"), "BDDA_ZWPLAN",
               "16-byte (FP64 / double-float) z passes (three lines per warp)", cost_z)
     if "t" in which:
-        write(os.path.join(here, "tplans.inc"), "BDDA_TPLAN", "strided x / y passes (one line per warp)",
-              cost_tile)
+        write(os.path.join(here, "tplans.inc"), "BDDA_TPLAN", "strided x / y passes (one line per warp)", cost_tile,
+              entry=t_entry)
 
 
 if __name__ == "__main__":

@@ -38,36 +38,41 @@ constexpr int kCols = 16;           // z-columns per task
 constexpr int kPairs = kCols / 2;   // threads of one butterfly
 constexpr int kLoads = 8;           // elements a thread reads from global memory before it transforms them
 
-// Threads per CTA: the multiple of 32 whose rounds over a stage's 8 N / R
-// butterfly threads idle least, weighted by the stages' work.
-template <class P>
-constexpr int threads() {
-  int best = 64;
-  long cost = -1;
-  for (int t = 64; t <= 256; t += 32) {
-    long c = 0;
-    for (int s = 0; s < P::nst; ++s) {
-      const int items = kPairs * (P::N / P::rad[s]);
-      c += (long)((items + t - 1) / t) * t * (6 * P::rad[s] + 10);
-    }
-    if (cost < 0 || c <= cost) { best = t; cost = c; }
-  }
-  return best;
-}
 template <class P>
 constexpr int max_radix() {
   int m = 0;
   for (int s = 0; s < P::nst; ++s) m = P::rad[s] > m ? P::rad[s] : m;
   return m;
 }
-// CTAs per SM to compile for: 1024 threads (64 registers), 768 for radices above 10, whose pair butterflies take four
+// Threads per SM to compile for: 1024 (64 registers), 768 for radices above 10, whose pair butterflies take four
 // registers an element.  N=65536, L=32 at 768 / 512 threads instead: forward 2.11 -> 2.09, inverse 1.75 -> 1.62 ms;
 // Py=160 (10 x 16): forward 0.180 -> 0.174 ms.
 template <class P>
-constexpr int min_blocks() {
-  const int b = (max_radix<P>() > 10 ? 768 : 1024) / threads<P>();
-  return b < 1 ? 1 : b;
+constexpr int sm_threads() { return max_radix<P>() > 10 ? 768 : 1024; }
+// Shared memory of an SM, and what a CTA takes beside its tile.
+constexpr int kSmemSm = 228 * 1024, kSmemCta = 1024;
+// Threads per CTA: the multiple of 32 with the least idling over a stage's 8 N / R butterfly threads, weighted by the
+// stages' work, over the threads, up to 896, that the tiles fitting an SM make.  Without the second factor 288 = 9 2 16
+// took 64 threads, three CTAs of them for each six tiles' room (y 7.9, x 9.7 ps per point for both directions; with it 5.9
+// and 7.1), 360 = 2 12 15 likewise (9.0 / 13.9 -> 7.1 / 7.1).
+template <class P>
+constexpr int threads() {
+  int best = 64;
+  long cost = -1;
+  for (int t = 64; t <= 384; t += 32) {
+    long c = 0;
+    for (int s = 0; s < P::nst; ++s) {
+      const int items = kPairs * (P::N / P::rad[s]);
+      c += (long)((items + t - 1) / t) * t * P::rad[s];
+    }
+    const int room = kSmemSm / (P::N * kCols * 8 + kSmemCta), ctas = std::min(sm_threads<P>() / t, room);
+    c = c * 896 / std::min(ctas * t, 896);
+    if (cost < 0 || c <= cost) { best = t; cost = c; }
+  }
+  return best;
 }
+template <class P>
+constexpr int min_blocks() { return sm_threads<P>() / threads<P>(); }
 
 // Rows a task reads, at most.
 template <class P, bool INV>
