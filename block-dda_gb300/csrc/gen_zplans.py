@@ -342,17 +342,14 @@ def t_entry(n):
     return (rad,) + choose_layout(n, rad, cost_tile)
 
 
-FUSED_WIDE_MIN_N = 181  # kFusedWideMinN: shorter z lines keep the packed-pair kernel's plans
+FUSED_WIDE_MIN_N = 181  # kFusedWideMinN: shorter z lines run in zpass_cols.cuh
 
 
 def z_entry(n):
     """Plan of the complex FP32 z table.  Lines shorter than FUSED_WIDE_MIN_N
-    (the packed-pair z pass's range: three 8-warp CTAs of it fit up to a
-    pitch of ~200) keep the 16-byte table's plan (cost_z, radices <= 16, a
-    fused step only up to radix 5), on which the packed kernel was measured
-    faster than the two-stage fused plans (N=16384, Pz=150: packed 10 x 15
-    0.64 ms, pipelined 15 x 10 0.76 ms); longer lines take the two-stage fused
-    model (cost_zf, first-stage radices up to 32)."""
+    have the 16-byte table's plan (cost_z): the f = 6 pass runs it, and the
+    f = 3 pass (zpass_cols.cuh) takes its own two radices.  Longer lines take
+    the two-stage fused model (cost_zf, first-stage radices up to 32)."""
     if n < FUSED_WIDE_MIN_N:
         return choose(n, cost_z)
     return choose(n, cost_zf, FIRST_RADICES, Z_MAX_PAD)

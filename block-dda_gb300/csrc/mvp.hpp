@@ -16,24 +16,37 @@ constexpr int kTileThreads = kTZ * 32;
 // Warps per CTA of the fused z pass (one (x, y, rhs) task each), at most.
 constexpr int kZWarps = 8;
 // The fused z pass (f = 3) runs its last forward stage, the Green product and
-// its first inverse stage in one sweep (sfft::middle3 / pk::middle3) when the
-// z plan has two or more stages and a last radix Rl <= kFusedMaxRadix (fused_z); a
-// thread then takes the Rl adjacent frequencies b Rl .. b Rl + Rl - 1 of a
+// its first inverse stage in one sweep (sfft::middle3, zpass_cols.cuh) when
+// the z plan has two or more stages and, for lines of kFusedWideMinN points
+// and more (one warp per task), a last radix Rl <= kFusedMaxRadix (fused_z);
+// a thread then takes the Rl adjacent frequencies b Rl .. b Rl + Rl - 1 of a
 // butterfly b, so the complex FP32 Green spectrum of such operators is stored
 // last-radix-major (frequency b Rl + i at i (Pz / Rl) + b): the lanes' loads
 // of one component are then adjacent (coalesced).  With the complex FP32 z
 // table's first-stage radices up to 32, most lengths are two stages with a
 // fused last radix (250 = 25 x 10, 243 = 27 x 9, 270 = 27 x 10): the first
 // stage reads T2 and writes shared memory, the fused step reads and writes it
-// once, the last inverse stage reads it and writes T2.  Shorter lines (below
-// kFusedWideMinN points, the packed-pair kernel's range) keep plans of radices
-// <= 16 and fuse only up to radix 5, the packed kernel's limit
-// (zpacked::supported).
+// once, the last inverse stage reads it and writes T2.  Shorter lines have
+// plans of radices <= 16, whose few butterflies a CTA of several tasks shares
+// out (zpass_cols.cuh).
 constexpr int kFusedMaxRadix = 10;
-constexpr int kFusedMaxRadixShort = 5;
 constexpr int kFusedWideMinN = 181;
 BDDA_HD constexpr bool fused_z(int N, int nst, int rl) {
-  return nst >= 2 && (rl <= kFusedMaxRadixShort || (rl <= kFusedMaxRadix && N >= kFusedWideMinN));
+  return N < kFusedWideMinN ? nst == 2 || (nst > 2 && rl <= 5) : nst >= 2 && rl <= kFusedMaxRadix;
+}
+// Last radix of the column kernels' two-stage z plans (lines shorter than
+// kFusedWideMinN, zpass_cols.cuh): the largest up to 9 whose cofactor is a
+// radix too (the middle step holds three lines of it per right-hand side: 128
+// = 16 8 0.173 ms, 8 16 0.190; 150 = 15 10 0.215, 10 15 0.270), else 10, else
+// the largest (180 = 12 15 0.288, 15 12 0.330).
+BDDA_HD constexpr bool is_z_radix(int r) { return (r >= 2 && r <= 6) || (r >= 8 && r <= 10) || r == 12 || r == 15 || r == 16; }
+BDDA_HD constexpr int z_col_last_radix(int N) {
+  for (int r = 9; r >= 2; --r)
+    if (N % r == 0 && is_z_radix(r) && is_z_radix(N / r)) return r;
+  if (N % 10 == 0 && is_z_radix(N / 10)) return 10;
+  for (int r = 16; r > 10; --r)
+    if (N % r == 0 && is_z_radix(r) && is_z_radix(N / r)) return r;
+  return 0;
 }
 // (complex FP32 only: the double-float fused step needs 168 registers and ran
 // slower than the separate stages, 54.9 vs 41.6 ms per N=65536, L=32 pass.)
@@ -54,8 +67,8 @@ inline int z_warps_per_cta(int per_warp) {
 // by the autotuner (op.cu: candidates timed with CUDA events on the operator's
 // own buffers) or left at the defaults.
 struct MvpTune {
-  // pass C kernel: -1 the default rule (pipelined where the plan and shared memory allow, else packed where
-  // three 8-warp CTAs fit, else scalar), 0 scalar, 1 packed, 2 pipelined (zpass_pipe.cuh)
+  // pass C kernel: -1 the default rule (f = 3: zpass_cols.cuh below kFusedWideMinN points, else pipelined where the
+  // plan and shared memory allow, else scalar), 0 scalar, 1 packed (right-hand sides in pairs), 2 pipelined (zpass_pipe.cuh)
   int zkern = -1;
   int ywaves = 4;    // passes B, D: grid of this many waves of the CTAs resident per SM
   int ybuf = 2;      // passes B, D: buffers per CTA (2: the next task's rows are prefetched; 1: more CTAs)
@@ -93,7 +106,7 @@ template <typename T> struct MvpPrec {
   const C* twz;
   const C* ghat;  // [Px][Py][6 or 9][Pz] (digit-reversed frequencies), divided by Px*Py*Pz
   const float4* twzp = nullptr;  // complex FP32: z twiddle pairs {wx, wx, wy, wy} (packed z pass)
-  // staged tables (stage_twiddles) of the compile-time-plan kernels: x, y pairs, z, z pairs (packed z pass)
+  // staged tables (stage_twiddles) of the compile-time-plan kernels: x, y pairs, z, z pairs (zpass_cols.cuh)
   const float4* twxps = nullptr;
   const float4* twyps = nullptr;
   const C* twzs = nullptr;
@@ -269,14 +282,15 @@ inline int x_field_groups(int nfield, int ntiles, int sms, int* fpg, int xcta = 
 bool launch_tile_static(int pass, const TileArgs& a, cudaError_t* err);
 
 // Pass C for complex FP32 with the compile-time z plan of g.Pz (zplans.inc);
-// returns false (nothing launched) when g.Pz has none.  With twzp (the z
-// twiddle pair table {wx, wx, wy, wy}) and f = 3 the packed-pair kernel runs.
+// returns false (nothing launched) when g.Pz has none.  twz: the plan's staged
+// twiddles; twzp: those of the column kernels' plan (z_col_last_radix) as
+// {wx, wx, wy, wy}.
 // *err: launch status.
 bool launch_pass_c_static(const MvpGeom& g, float2* t2, int L, const float2* twz, const float4* twzp, const float2* ghat,
                           cudaStream_t st, const int* done, cudaError_t* err);
 
-// Whether the packed-pair pass C can run for z length Pz and f (an autotuner
-// candidate besides the scalar kernel).
+// Whether pass C can run right-hand sides in pairs for z length Pz and f (an
+// autotuner candidate besides the scalar kernel).
 bool packed_z_available(int Pz, int f);
 // Whether the pipelined z pass (zpass_pipe.cuh) can run this geometry at nrhs
 // L (an autotuner candidate; the default rule also wants two CTAs per SM).

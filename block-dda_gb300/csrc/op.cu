@@ -417,17 +417,26 @@ int bdda_op_create(bdda_op** out, const int n[3], int f, double lf, double k_re,
     }
     // staged tables of the complex FP32 compile-time-plan kernels
     std::vector<double2> ts;
-    stage_twiddles(op->plan[i], &ts);
-    const size_t nts = std::max<size_t>(ts.size(), 1);
-    std::vector<float2> tsf(nts, make_float2(1.f, 0.f));
-    std::vector<float4> tsp(nts, make_float4(1.f, 1.f, 0.f, 0.f));
-    for (size_t t = 0; t < ts.size(); ++t) {
-      tsf[t] = make_float2((float)ts[t].x, (float)ts[t].y);
-      tsp[t] = make_float4(tsf[t].x, tsf[t].x, tsf[t].y, tsf[t].y);
+    AxisPlan col = op->plan[i];  // the column kernels' plan
+    if (i == 2 && col.nst == 2 && col.N < kFusedWideMinN) {
+      col.radix[1] = z_col_last_radix(col.N);
+      col.radix[0] = col.N / col.radix[1];
     }
-    BDDA_CUDA(op->tws32p[i].ensure(nts * sizeof(float4), op->stream));
-    BDDA_CUDA(cudaMemcpyAsync(op->tws32p[i].p, tsp.data(), nts * sizeof(float4), cudaMemcpyHostToDevice, op->stream));
+    stage_twiddles(col, &ts);
+    const size_t ntp = std::max<size_t>(ts.size(), 1);
+    std::vector<float4> tsp(ntp, make_float4(1.f, 1.f, 0.f, 0.f));
+    for (size_t t = 0; t < ts.size(); ++t) {
+      const float wx = (float)ts[t].x, wy = (float)ts[t].y;
+      tsp[t] = make_float4(wx, wx, wy, wy);
+    }
+    BDDA_CUDA(op->tws32p[i].ensure(ntp * sizeof(float4), op->stream));
+    BDDA_CUDA(cudaMemcpyAsync(op->tws32p[i].p, tsp.data(), ntp * sizeof(float4), cudaMemcpyHostToDevice, op->stream));
+    std::vector<float2> tsf;
     if (i == 2) {
+      stage_twiddles(op->plan[i], &ts);
+      const size_t nts = std::max<size_t>(ts.size(), 1);
+      tsf.assign(nts, make_float2(1.f, 0.f));
+      for (size_t t = 0; t < ts.size(); ++t) tsf[t] = make_float2((float)ts[t].x, (float)ts[t].y);
       BDDA_CUDA(op->tws32z.ensure(nts * sizeof(float2), op->stream));
       BDDA_CUDA(cudaMemcpyAsync(op->tws32z.p, tsf.data(), nts * sizeof(float2), cudaMemcpyHostToDevice, op->stream));
     }

@@ -11,8 +11,7 @@
 // The radix kernels compute the same DFTs as fft_core.cuh (same directions:
 // forward exp(-2 pi i / R), inverse exp(+2 pi i / R); same output order), with
 // the multiplications by +-i folded into the adjacent additions (packed
-// arithmetic has no lane swap).  The stage functions mirror static_fft.cuh
-// (same plans, digit order and pruning) on 16-byte elements.
+// arithmetic has no lane swap).
 #pragma once
 
 #include "fft_core.cuh"
@@ -208,232 +207,6 @@ template <int R, bool INV> __device__ __forceinline__ void dft(cp* v) {
   else if constexpr (R == 12) dct<4, 3, INV>(v);
   else if constexpr (R == 15) dct<3, 5, INV>(v);
   else dct<4, 4, INV>(v);  // 16
-}
-
-// ---- stages on 16-byte shared-memory elements (compile-time plan P) -------------
-// NP line pairs per warp; pair j's element idx at sm[j * P::LW + P::addr(idx)].
-// tw: staged twiddle pair table ({wx, wx, wy, wy} entries, same layout as
-// sfft's staged table: stage s at P::TWO(s), entry (k - 1) M_s + n1).
-template <class P, int s, bool INV, int NP>
-__device__ __forceinline__ void stage(ulonglong2* __restrict__ sm, const float4* __restrict__ tw, int lane, int nv) {
-  constexpr int R = P::rad[s];
-  constexpr int M = P::M(s);
-  constexpr int Ls = M * R;
-  constexpr int B = P::N / R;
-  constexpr int T = NP * B;
-  constexpr int off = (s == P::nst - 1) ? 1 : (M / P::Rl) * P::S;
-  constexpr bool prune_in = !INV && s == 0;
-  constexpr bool prune_out = INV && s == 0;
-  for (int t = lane; t < T; t += 32) {
-    const int j = NP == 1 ? 0 : t / B;
-    const int u = t - j * B;
-    const int b = u / M, n1 = u - b * M;
-    const int idx0 = b * Ls + n1;
-    ulonglong2* p = sm + j * P::LW + P::addr(idx0);
-    cp v[R];
-#pragma unroll
-    for (int i = 0; i < R; ++i) {
-      if (prune_in) v[i] = (2 * i < R && idx0 + i * M < nv) ? lds(p + i * off) : cp{0ull, 0ull};
-      else v[i] = lds(p + i * off);
-    }
-    if (!INV) {
-      dft<R, false>(v);
-      if (M > 1 && n1 != 0) {
-        const float4* tws = tw + P::TWO(s) + n1;
-#pragma unroll
-        for (int k = 1; k < R; ++k) {
-          u64 c, sn;
-          ld_tw(tws + (k - 1) * M, c, sn);
-          v[k] = tw_mul(v[k], c, sn);
-        }
-      }
-    } else {
-      if (M > 1 && n1 != 0) {
-        const float4* tws = tw + P::TWO(s) + n1;
-#pragma unroll
-        for (int k = 1; k < R; ++k) {
-          u64 c, sn;
-          ld_tw(tws + (k - 1) * M, c, sn);
-          v[k] = tw_mulc(v[k], c, sn);
-        }
-      }
-      dft<R, true>(v);
-    }
-#pragma unroll
-    for (int i = 0; i < R; ++i) {
-      if (prune_out) {
-        if (2 * i < R && idx0 + i * M < nv) sts(p + i * off, v[i]);
-      } else {
-        sts(p + i * off, v[i]);
-      }
-    }
-  }
-  __syncwarp();
-}
-
-// First forward stage reading the two lines of each pair from global memory:
-// pair j's lines at ga + j * gstride and ga + j * gstride + boff, elements
-// idx < nv (the zero padding is never read).
-template <class P, int NP>
-__device__ __forceinline__ void stage0_from_global(ulonglong2* __restrict__ sm, const float4* __restrict__ tw, int lane,
-                                                   int nv, const float2* __restrict__ ga, size_t gstride, ptrdiff_t boff) {
-  constexpr int R = P::rad[0];
-  constexpr int M = P::M(0);
-  constexpr int T = NP * M;
-  constexpr int off = (P::nst == 1) ? 1 : (M / P::Rl) * P::S;
-  for (int t = lane; t < T; t += 32) {
-    const int j = NP == 1 ? 0 : t / M;
-    const int n1 = t - j * M;
-    const float2* g = ga + (size_t)j * gstride + n1;
-    cp v[R];
-#pragma unroll
-    for (int i = 0; i < R; ++i) {
-      if (2 * i < R && n1 + i * M < nv) {  // nv <= N / 2, as in sfft::stage
-        const float2 x = g[i * M], y = g[i * M + boff];
-        v[i] = {p2(x.x, y.x), p2(x.y, y.y)};
-      } else {
-        v[i] = {0ull, 0ull};
-      }
-    }
-    dft<R, false>(v);
-    if (M > 1 && n1 != 0) {
-#pragma unroll
-      for (int k = 1; k < R; ++k) {
-        u64 c, sn;
-        ld_tw(tw + (k - 1) * M + n1, c, sn);
-        v[k] = tw_mul(v[k], c, sn);
-      }
-    }
-    ulonglong2* p = sm + j * P::LW + P::addr(n1);
-#pragma unroll
-    for (int i = 0; i < R; ++i) sts(p + i * off, v[i]);
-  }
-  __syncwarp();
-}
-
-// Last inverse stage writing the pairs' lines to global memory (elements
-// idx < nv; the second line only when write_b).
-template <class P, int NP>
-__device__ __forceinline__ void stage0_to_global(const ulonglong2* __restrict__ sm, const float4* __restrict__ tw,
-                                                 int lane, int nv, float2* __restrict__ ga, size_t gstride,
-                                                 ptrdiff_t boff, bool write_b) {
-  constexpr int R = P::rad[0];
-  constexpr int M = P::M(0);
-  constexpr int T = NP * M;
-  constexpr int off = (P::nst == 1) ? 1 : (M / P::Rl) * P::S;
-  for (int t = lane; t < T; t += 32) {
-    const int j = NP == 1 ? 0 : t / M;
-    const int n1 = t - j * M;
-    const ulonglong2* p = sm + j * P::LW + P::addr(n1);
-    cp v[R];
-#pragma unroll
-    for (int i = 0; i < R; ++i) v[i] = lds(p + i * off);
-    if (M > 1 && n1 != 0) {
-#pragma unroll
-      for (int k = 1; k < R; ++k) {
-        u64 c, sn;
-        ld_tw(tw + (k - 1) * M + n1, c, sn);
-        v[k] = tw_mulc(v[k], c, sn);
-      }
-    }
-    dft<R, true>(v);
-    float2* g = ga + (size_t)j * gstride + n1;
-#pragma unroll
-    for (int i = 0; i < R; ++i)
-      if (2 * i < R && n1 + i * M < nv) {
-        float ra, rb, ia, ib;
-        unp(v[i].re, ra, rb);
-        unp(v[i].im, ia, ib);
-        g[i * M] = make_float2(ra, ia);
-        if (write_b) g[i * M + boff] = make_float2(rb, ib);
-      }
-  }
-  __syncwarp();
-}
-
-// Forward stages s .. end - 1.
-template <class P, int NP, int s, int end>
-__device__ __forceinline__ void forward_to(ulonglong2* sm, const float4* tw, int lane, int nv) {
-  if constexpr (s < end) {
-    stage<P, s, false, NP>(sm, tw, lane, nv);
-    forward_to<P, NP, s + 1, end>(sm, tw, lane, nv);
-  }
-}
-
-// Last forward stage, Green product and first inverse stage of a task's three
-// line pairs in one sweep (the packed form of sfft::middle3): butterfly b of
-// the last stage (M = 1, no twiddles) in all three component pairs, the
-// symmetric 3 x 3 spectrum (last-radix-major, green_pos) of each of its R
-// frequencies applied in registers, the inverse DFT, one store.  Used for
-// R <= 5 (3 R pair elements, 12 R registers; zpacked::supported).
-template <class P>
-__device__ __forceinline__ void middle3(ulonglong2* __restrict__ sm, const float2* __restrict__ gl, int lane) {
-  constexpr int R = P::Rl;
-  constexpr int B = P::N / R;
-  constexpr int m[3][3] = {{0, 1, 2}, {1, 3, 4}, {2, 4, 5}};
-  for (int b = lane; b < B; b += 32) {
-    const int idx0 = b * R;
-    ulonglong2* p = sm + P::addr(idx0);
-    cp e[3][R];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-#pragma unroll
-      for (int i = 0; i < R; ++i) e[c][i] = lds(p + c * P::LW + i);
-      dft<R, false>(e[c]);
-    }
-#pragma unroll
-    for (int i = 0; i < R; ++i) {
-      u64 gr[6], gi[6];
-#pragma unroll
-      for (int c = 0; c < 6; ++c) {
-        const float2 g = ldg_c(gl + c * P::N + i * B + b);
-        gr[c] = dup(g.x);
-        gi[c] = dup(g.y);
-      }
-      cp o3[3];
-#pragma unroll
-      for (int o = 0; o < 3; ++o) {
-        // re' = sum re_d gr - sum im_d gi ; im' = sum im_d gr + re_d gi
-        u64 ar = mul(e[0][i].re, gr[m[o][0]]);
-        ar = fma(e[1][i].re, gr[m[o][1]], ar);
-        ar = fma(e[2][i].re, gr[m[o][2]], ar);
-        u64 ai = mul(e[0][i].im, gi[m[o][0]]);
-        ai = fma(e[1][i].im, gi[m[o][1]], ai);
-        ai = fma(e[2][i].im, gi[m[o][2]], ai);
-        u64 bi = mul(e[0][i].im, gr[m[o][0]]);
-        bi = fma(e[1][i].im, gr[m[o][1]], bi);
-        bi = fma(e[2][i].im, gr[m[o][2]], bi);
-        bi = fma(e[0][i].re, gi[m[o][0]], bi);
-        bi = fma(e[1][i].re, gi[m[o][1]], bi);
-        bi = fma(e[2][i].re, gi[m[o][2]], bi);
-        o3[o] = cp{sub(ar, ai), bi};
-      }
-#pragma unroll
-      for (int c = 0; c < 3; ++c) e[c][i] = o3[c];
-    }
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      dft<R, true>(e[c]);
-#pragma unroll
-      for (int i = 0; i < R; ++i) sts(p + c * P::LW + i, e[c][i]);
-    }
-  }
-  __syncwarp();
-}
-
-template <class P, int NP, int s = 0>
-__device__ __forceinline__ void forward(ulonglong2* sm, const float4* tw, int lane, int nv) {
-  if constexpr (s < P::nst) {
-    stage<P, s, false, NP>(sm, tw, lane, nv);
-    forward<P, NP, s + 1>(sm, tw, lane, nv);
-  }
-}
-template <class P, int NP, int s = P::nst - 1, int last = 0>
-__device__ __forceinline__ void inverse(ulonglong2* sm, const float4* tw, int lane, int nv) {
-  if constexpr (s >= last) {
-    stage<P, s, true, NP>(sm, tw, lane, nv);
-    inverse<P, NP, s - 1, last>(sm, tw, lane, nv);
-  }
 }
 
 }  // namespace pk

@@ -46,7 +46,7 @@ bool packed_z_available(int Pz, int f) {
   switch (Pz) {
 #define BDDA_ZPLAN(I, N, S, LW, ...) \
   case N:                            \
-    return zpacked::supported<sfft::Plan<N, S, LW, __VA_ARGS__>>() && zpacked::fits<sfft::Plan<N, S, LW, __VA_ARGS__>>();
+    return zcol::supported<sfft::Plan<N, S, LW, __VA_ARGS__>>();
 #include "zplans.inc"
 #undef BDDA_ZPLAN
     default:

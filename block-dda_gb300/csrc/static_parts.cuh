@@ -4,7 +4,7 @@
 #pragma once
 
 #include "xpass_cols.cuh"
-#include "zpass_packed.cuh"
+#include "zpass_cols.cuh"
 #include "zpass_pipe.cuh"
 #include "zpass_static.cuh"
 
@@ -21,15 +21,11 @@ bool dispatch_z(const MvpGeom& g, float2* t2, int L, const float2* twz, const fl
   case N:                                                                                \
     if constexpr ((I) % kParts == PART) {                                                \
       using Pl = sfft::Plan<N, S, LW, __VA_ARGS__>;                                      \
-      if constexpr (zpacked::supported<Pl>())                                            \
-        if (zpacked::chosen<Pl>(g, twzp)) {                                              \
-          *err = zpacked::launch<Pl>(g, t2, L, twzp, ghat, st, done);                    \
-          return true;                                                                   \
-        }                                                                                \
-      if ((g.tune.zkern < 0 || g.tune.zkern == 2) &&                                     \
+      if ((g.tune.zkern == 2 || (g.tune.zkern < 0 && (N) >= kFusedWideMinN)) &&          \
           zpipe::launch<Pl>(g, t2, L, twz, ghat, st, done, err))                         \
         return true;                                                                     \
-      *err = zstatic::launch<Pl>(g, t2, L, twz, ghat, st, done);                         \
+      if (zcol::launch<Pl>(g, t2, L, twzp, ghat, st, done, err)) return true;            \
+      *err = zstatic::launch<Pl, !zcol::supported<Pl>()>(g, t2, L, twz, ghat, st, done); \
       return true;                                                                       \
     }                                                                                    \
     return false;

@@ -78,10 +78,14 @@ cudaError_t launch_f(const MvpGeom& g, C* t2, int L, const C* twz, const C* ghat
   return cudaGetLastError();
 }
 
-template <class P>
+// THREE: the operator may have f = 3 (else those lines run in zpass_cols.cuh)
+template <class P, bool THREE>
 cudaError_t launch(const MvpGeom& g, float2* t2, int L, const float2* twz, const float2* ghat, cudaStream_t st,
                    const int* done) {
-  return g.f == 6 ? launch_f<P, true>(g, t2, L, twz, ghat, st, done) : launch_f<P, false>(g, t2, L, twz, ghat, st, done);
+  if constexpr (THREE) {
+    if (g.f == 3) return launch_f<P, false>(g, t2, L, twz, ghat, st, done);
+  }
+  return launch_f<P, true>(g, t2, L, twz, ghat, st, done);
 }
 
 }  // namespace zstatic
