@@ -15,10 +15,9 @@ namespace bdda {
 
 // ---------------------------------------------------------------------------
 // Double-float scalar: value = hi + lo with |lo| <= ulp(hi)/2 (about 48
-// significant bits), computed with FP32 instructions only.  GB300's FP32 pipes
-// run ~64x the FP64 rate, so an FFT in double-float arithmetic is several
-// times faster than in FP64 while keeping the refinement residual accurate to
-// ~1e-14.  Sums use the two-sum of Knuth, products the FMA-based two-product;
+// significant bits), computed with FP32 instructions only (GB300's FP32 pipes
+// run ~64x the FP64 rate): the L x L steps and Gram sums of FP32 solves, and
+// the storage of the refinement's residual vectors.  Sums use the two-sum of Knuth, products the FMA-based two-product;
 // the addition is the short ("sloppy") variant whose error is bounded
 // relative to |a| + |b|, which is what FFT error analysis needs.
 // ---------------------------------------------------------------------------
@@ -56,8 +55,8 @@ struct __align__(16) dfc {
   dfl x, y;
 };
 
-// Double-float without renormalisation, the arithmetic of the double-float
-// block MVP.  The leading parts are summed with the exact two-sum and the
+// Double-float without renormalisation, an arithmetic of the host line
+// transform (bdda_host_fft_line).  The leading parts are summed with the exact two-sum and the
 // products formed with the FMA two-product, as in dfl, but the result keeps
 // the error term as the trailing part (|lo| may exceed ulp(hi) / 2 by the few
 // rounding errors of a butterfly chain) instead of being renormalised by a

@@ -105,7 +105,6 @@ template <typename T> struct MvpPrec {
   const C* twy;
   const C* twz;
   const C* ghat;  // [Px][Py][6 or 9][Pz] (digit-reversed frequencies), divided by Px*Py*Pz
-  const float4* twzp = nullptr;  // complex FP32: z twiddle pairs {wx, wx, wy, wy} (packed z pass)
   // staged tables (stage_twiddles) of the compile-time-plan kernels: x, y pairs, z, z pairs (zpass_cols.cuh)
   const float4* twxps = nullptr;
   const float4* twyps = nullptr;
@@ -257,11 +256,8 @@ enum TilePass { kTileA = 0, kTileB, kTileD, kTileE };
 
 // Grid of the y passes (B, D), whose CTAs take tasks (field, x, z tile) in a
 // fixed stride: by default four waves of the CTAs resident per SM
-// (MvpTune::ywaves).  Measured on the
-// column-pair passes (N=16384 / 8192, tasks of uneven cost: empty rows are
-// skipped): one exact wave 0.244 / 0.146 ms (forward), two 0.239 / 0.138,
-// four 0.233 / 0.135; the earlier fixed 8 CTAs per SM (1.1-1.6 waves) 0.239 /
-// 0.159.
+// (MvpTune::ywaves): tasks are of uneven cost (empty rows are skipped), so one
+// wave of them ends raggedly.  The autotuner times 2 to 16 waves.
 constexpr int kYWaves = 4;
 
 // Fields per CTA of the x passes (A, E), an even number: a tile's fields are

@@ -82,7 +82,7 @@ Op::~Op() {
   solver.reset();
   for (auto* o : {&dip, &cub}) { o->occ.release(); o->tiles.release(); o->tmask.release(); }
   for (int i = 0; i < 3; ++i) {
-    tw32[i].release(); twfx[i].release(); tw32p[i].release(); tws32p[i].release();
+    tw32[i].release(); twfx[i].release(); tws32p[i].release();
   }
   tws32z.release(); fxpos.release();
   ghat32.release(); ghatfx.release(); gexpfx.release();
@@ -409,12 +409,6 @@ int bdda_op_create(bdda_op** out, const int n[3], int f, double lf, double k_re,
     for (size_t t = 0; t < tw.size(); ++t) tf[t] = make_float2((float)tw[t].x, (float)tw[t].y);
     BDDA_CUDA(op->tw32[i].ensure(tf.size() * sizeof(float2), op->stream));
     BDDA_CUDA(cudaMemcpyAsync(op->tw32[i].p, tf.data(), tf.size() * sizeof(float2), cudaMemcpyHostToDevice, op->stream));
-    std::vector<float4> tp(tw.size());
-    for (size_t t = 0; t < tw.size(); ++t) tp[t] = make_float4(tf[t].x, tf[t].x, tf[t].y, tf[t].y);
-    if (i == 2 && !std::getenv("BDDA_NO_PACK")) {
-      BDDA_CUDA(op->tw32p[i].ensure(tp.size() * sizeof(float4), op->stream));
-      BDDA_CUDA(cudaMemcpyAsync(op->tw32p[i].p, tp.data(), tp.size() * sizeof(float4), cudaMemcpyHostToDevice, op->stream));
-    }
     // staged tables of the complex FP32 compile-time-plan kernels
     std::vector<double2> ts;
     AxisPlan col = op->plan[i];  // the column kernels' plan

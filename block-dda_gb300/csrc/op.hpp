@@ -90,7 +90,6 @@ struct Op {
   fx::Plan fxplan[3];
   DevBuf tw32[3], twfx[3];
   DevBuf fxpos;     // int [3][kMaxLine]: the complex FP32 order's positions in the fixed-point order
-  DevBuf tw32p[3];  // complex FP32 twiddle pairs {wx, wx, wy, wy} of the packed z pass ([2] only)
   // staged twiddles (stage_twiddles) of the compile-time-plan kernels: complex
   // FP32 along z, and per axis as pairs {wx, wx, wy, wy}.  Every DevBuf of the operator is
   // released in ~Op, before its stream is destroyed.
@@ -122,7 +121,7 @@ struct Op {
   unsigned long long buffer_sig() const {
     unsigned long long h = 0;
     for (int i = 0; i < 3; ++i)
-      for (const DevBuf* b : {&tw32[i], &twfx[i], &tw32p[i], &tws32p[i]}) h = sig_add(h, *b);
+      for (const DevBuf* b : {&tw32[i], &twfx[i], &tws32p[i]}) h = sig_add(h, *b);
     for (int i = 0; i < 2; ++i)
       for (const DevBuf* b : {&t1[i], &t2[i]}) h = sig_add(h, *b);
     for (const DevBuf* b : {&texp, &ghat32, &ghatfx, &gexpfx, &tws32z, &kstat, &dip.occ, &dip.tiles, &dip.tmask})
@@ -150,7 +149,7 @@ struct Op {
     return g;
   }
   MvpPrec<float> tables32() const {
-    return {tw32[0].as<float2>(), tw32[1].as<float2>(), tw32[2].as<float2>(), ghat32.as<float2>(), tw32p[2].as<float4>(),
+    return {tw32[0].as<float2>(), tw32[1].as<float2>(), tw32[2].as<float2>(), ghat32.as<float2>(),
             tws32p[0].as<float4>(), tws32p[1].as<float4>(), tws32z.as<float2>(), tws32p[2].as<float4>()};
   }
   FxTables tables_fx() const {
