@@ -105,11 +105,11 @@ template <typename T> struct MvpPrec {
   const C* twy;
   const C* twz;
   const C* ghat;  // [Px][Py][6 or 9][Pz] (digit-reversed frequencies), divided by Px*Py*Pz
-  // staged tables (stage_twiddles) of the compile-time-plan kernels: x, y pairs, z, z pairs (zpass_cols.cuh)
+  // staged tables (stage_twiddles) of the compile-time-plan kernels: x, y pairs, z, z of zpass_cols.cuh
   const float4* twxps = nullptr;
   const float4* twyps = nullptr;
   const C* twzs = nullptr;
-  const float4* twzps = nullptr;
+  const C* twzc = nullptr;
 };
 
 // Tables of the fixed-point MVP (FP64 and double-float, mvp_fx.cu): axis plans,
@@ -279,10 +279,9 @@ bool launch_tile_static(int pass, const TileArgs& a, cudaError_t* err);
 
 // Pass C for complex FP32 with the compile-time z plan of g.Pz (zplans.inc);
 // returns false (nothing launched) when g.Pz has none.  twz: the plan's staged
-// twiddles; twzp: those of the column kernels' plan (z_col_last_radix) as
-// {wx, wx, wy, wy}.
+// twiddles; twzc: those of the column kernels' plan (z_col_last_radix).
 // *err: launch status.
-bool launch_pass_c_static(const MvpGeom& g, float2* t2, int L, const float2* twz, const float4* twzp, const float2* ghat,
+bool launch_pass_c_static(const MvpGeom& g, float2* t2, int L, const float2* twz, const float2* twzc, const float2* ghat,
                           cudaStream_t st, const int* done, cudaError_t* err);
 
 // Whether pass C can run right-hand sides in pairs for z length Pz and f (an

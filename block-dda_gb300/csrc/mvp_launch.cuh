@@ -169,7 +169,7 @@ cudaError_t launch_block_mvp(const MvpGeom& g, const MvpPrec<T>& p, const typena
     bool launched = false;
     if constexpr (std::is_same<T, float>::value) {
       cudaError_t e = cudaSuccess;
-      launched = launch_pass_c_static(g, t2, L, p.twzs, p.twzps, p.ghat, st, done, &e);
+      launched = launch_pass_c_static(g, t2, L, p.twzs, p.twzc, p.ghat, st, done, &e);
       if (launched && e != cudaSuccess) return e;
     }
     if (!launched) {

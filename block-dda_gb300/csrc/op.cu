@@ -84,7 +84,7 @@ Op::~Op() {
   for (int i = 0; i < 3; ++i) {
     tw32[i].release(); twfx[i].release(); tws32p[i].release();
   }
-  tws32z.release(); fxpos.release();
+  tws32z.release(); tws32c.release(); fxpos.release();
   ghat32.release(); ghatfx.release(); gexpfx.release();
   kstat.release();
   for (int i = 0; i < 2; ++i) { t1[i].release(); t2[i].release(); }
@@ -212,7 +212,7 @@ static cudaError_t autotune_f32(MvpGeom g, const MvpPrec<float>& p, const float2
     t.ywaves = yw[best % 4];
   }
   {  // pass C: scalar, packed and pipelined kernels where they run this geometry
-    const bool packed = packed_z_available(g.Pz, g.f) && p.twzps;
+    const bool packed = packed_z_available(g.Pz, g.f) && p.twzc;
     const bool pipe = pipe_z_available(g.Pz, g.f, g.nzp, L);
     if (e == cudaSuccess && (packed || pipe)) {
       MvpTune c = t;
@@ -411,28 +411,34 @@ int bdda_op_create(bdda_op** out, const int n[3], int f, double lf, double k_re,
     BDDA_CUDA(cudaMemcpyAsync(op->tw32[i].p, tf.data(), tf.size() * sizeof(float2), cudaMemcpyHostToDevice, op->stream));
     // staged tables of the complex FP32 compile-time-plan kernels
     std::vector<double2> ts;
-    AxisPlan col = op->plan[i];  // the column kernels' plan
-    if (i == 2 && col.nst == 2 && col.N < kFusedWideMinN) {
-      col.radix[1] = z_col_last_radix(col.N);
-      col.radix[0] = col.N / col.radix[1];
-    }
-    stage_twiddles(col, &ts);
-    const size_t ntp = std::max<size_t>(ts.size(), 1);
-    std::vector<float4> tsp(ntp, make_float4(1.f, 1.f, 0.f, 0.f));
-    for (size_t t = 0; t < ts.size(); ++t) {
-      const float wx = (float)ts[t].x, wy = (float)ts[t].y;
-      tsp[t] = make_float4(wx, wx, wy, wy);
-    }
-    BDDA_CUDA(op->tws32p[i].ensure(ntp * sizeof(float4), op->stream));
-    BDDA_CUDA(cudaMemcpyAsync(op->tws32p[i].p, tsp.data(), ntp * sizeof(float4), cudaMemcpyHostToDevice, op->stream));
-    std::vector<float2> tsf;
-    if (i == 2) {
-      stage_twiddles(op->plan[i], &ts);
-      const size_t nts = std::max<size_t>(ts.size(), 1);
-      tsf.assign(nts, make_float2(1.f, 0.f));
-      for (size_t t = 0; t < ts.size(); ++t) tsf[t] = make_float2((float)ts[t].x, (float)ts[t].y);
-      BDDA_CUDA(op->tws32z.ensure(nts * sizeof(float2), op->stream));
-      BDDA_CUDA(cudaMemcpyAsync(op->tws32z.p, tsf.data(), nts * sizeof(float2), cudaMemcpyHostToDevice, op->stream));
+    stage_twiddles(op->plan[i], &ts);
+    std::vector<float4> tsp;
+    std::vector<float2> tsf, tsc;
+    if (i < 2) {  // pairs of adjacent columns
+      tsp.assign(std::max<size_t>(ts.size(), 1), make_float4(1.f, 1.f, 0.f, 0.f));
+      for (size_t t = 0; t < ts.size(); ++t) {
+        const float wx = (float)ts[t].x, wy = (float)ts[t].y;
+        tsp[t] = make_float4(wx, wx, wy, wy);
+      }
+      BDDA_CUDA(op->tws32p[i].ensure(tsp.size() * sizeof(float4), op->stream));
+      BDDA_CUDA(cudaMemcpyAsync(op->tws32p[i].p, tsp.data(), tsp.size() * sizeof(float4), cudaMemcpyHostToDevice, op->stream));
+    } else {
+      auto to_float = [&ts](std::vector<float2>* out) {
+        out->assign(std::max<size_t>(ts.size(), 1), make_float2(1.f, 0.f));
+        for (size_t t = 0; t < ts.size(); ++t) (*out)[t] = make_float2((float)ts[t].x, (float)ts[t].y);
+      };
+      to_float(&tsf);
+      BDDA_CUDA(op->tws32z.ensure(tsf.size() * sizeof(float2), op->stream));
+      BDDA_CUDA(cudaMemcpyAsync(op->tws32z.p, tsf.data(), tsf.size() * sizeof(float2), cudaMemcpyHostToDevice, op->stream));
+      AxisPlan col = op->plan[i];  // the column kernels' plan
+      if (col.nst == 2 && col.N < kFusedWideMinN) {
+        col.radix[1] = z_col_last_radix(col.N);
+        col.radix[0] = col.N / col.radix[1];
+      }
+      stage_twiddles(col, &ts);
+      to_float(&tsc);
+      BDDA_CUDA(op->tws32c.ensure(tsc.size() * sizeof(float2), op->stream));
+      BDDA_CUDA(cudaMemcpyAsync(op->tws32c.p, tsc.data(), tsc.size() * sizeof(float2), cudaMemcpyHostToDevice, op->stream));
     }
     BDDA_CUDA(wait_stream(op->stream));  // tw / tf / ts die at the end of this iteration
   }

@@ -91,9 +91,9 @@ struct Op {
   DevBuf tw32[3], twfx[3];
   DevBuf fxpos;     // int [3][kMaxLine]: the complex FP32 order's positions in the fixed-point order
   // staged twiddles (stage_twiddles) of the compile-time-plan kernels: complex
-  // FP32 along z, and per axis as pairs {wx, wx, wy, wy}.  Every DevBuf of the operator is
+  // FP32 along z (tws32c: zpass_cols.cuh), and of x and y as pairs {wx, wx, wy, wy}.  Every DevBuf of the operator is
   // released in ~Op, before its stream is destroyed.
-  DevBuf tws32z, tws32p[3];
+  DevBuf tws32z, tws32c, tws32p[3];
   DevBuf ghat32, ghatfx, gexpfx;  // Green spectra: complex FP32; Q62 with its exponents
   DevBuf kstat;     // int: status word of the pipelined z pass (take_kernel_status)
   Occupancy dip;    // dipole occupancy (set_dipoles)
@@ -124,7 +124,7 @@ struct Op {
       for (const DevBuf* b : {&tw32[i], &twfx[i], &tws32p[i]}) h = sig_add(h, *b);
     for (int i = 0; i < 2; ++i)
       for (const DevBuf* b : {&t1[i], &t2[i]}) h = sig_add(h, *b);
-    for (const DevBuf* b : {&texp, &ghat32, &ghatfx, &gexpfx, &tws32z, &kstat, &dip.occ, &dip.tiles, &dip.tmask})
+    for (const DevBuf* b : {&texp, &ghat32, &ghatfx, &gexpfx, &tws32z, &tws32c, &kstat, &dip.occ, &dip.tiles, &dip.tmask})
       h = sig_add(h, *b);
     return h;
   }
@@ -150,7 +150,7 @@ struct Op {
   }
   MvpPrec<float> tables32() const {
     return {tw32[0].as<float2>(), tw32[1].as<float2>(), tw32[2].as<float2>(), ghat32.as<float2>(),
-            tws32p[0].as<float4>(), tws32p[1].as<float4>(), tws32z.as<float2>(), tws32p[2].as<float4>()};
+            tws32p[0].as<float4>(), tws32p[1].as<float4>(), tws32z.as<float2>(), tws32c.as<float2>()};
   }
   FxTables tables_fx() const {
     return {{fxplan[0], fxplan[1], fxplan[2]},

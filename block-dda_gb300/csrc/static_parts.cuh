@@ -14,7 +14,7 @@ namespace sparts {
 constexpr int kParts = 4;
 
 template <int PART>
-bool dispatch_z(const MvpGeom& g, float2* t2, int L, const float2* twz, const float4* twzp, const float2* ghat,
+bool dispatch_z(const MvpGeom& g, float2* t2, int L, const float2* twz, const float2* twzc, const float2* ghat,
                 cudaStream_t st, const int* done, cudaError_t* err) {
   switch (g.Pz) {
 #define BDDA_ZPLAN(I, N, S, LW, ...)                                                     \
@@ -24,7 +24,7 @@ bool dispatch_z(const MvpGeom& g, float2* t2, int L, const float2* twz, const fl
       if ((g.tune.zkern == 2 || (g.tune.zkern < 0 && (N) >= kFusedWideMinN)) &&          \
           zpipe::launch<Pl>(g, t2, L, twz, ghat, st, done, err))                         \
         return true;                                                                     \
-      if (zcol::launch<Pl>(g, t2, L, twzp, ghat, st, done, err)) return true;            \
+      if (zcol::launch<Pl>(g, t2, L, twzc, ghat, st, done, err)) return true;            \
       *err = zstatic::launch<Pl, !zcol::supported<Pl>()>(g, t2, L, twz, ghat, st, done); \
       return true;                                                                       \
     }                                                                                    \

@@ -23,9 +23,11 @@
 // Bound by issue and latency (T2 at its copy rate would take 2.4 ps per point).
 // Lines of 9216 (x, y) and L = 16 right-hand sides, ms, one warp per pair of
 // right-hand sides -> now: 64
-// 0.127 -> 0.082, 80 0.154 -> 0.123, 90 0.154 -> 0.147, 96 0.183 -> 0.133, 100
-// 0.194 -> 0.164, 120 0.195 -> 0.175, 128 0.220 -> 0.173, 135 0.287 -> 0.202,
-// 144 0.268 -> 0.201, 150 0.251 -> 0.215, 160 0.261 -> 0.216, 180 0.388 -> 0.288.
+// 0.127 -> 0.085, 80 0.154 -> 0.121, 90 0.154 -> 0.139, 96 0.183 -> 0.132, 100
+// 0.194 -> 0.158, 120 0.195 -> 0.171, 128 0.220 -> 0.168, 135 0.287 -> 0.192,
+// 144 0.268 -> 0.190, 150 0.251 -> 0.205, 160 0.261 -> 0.205, 180 0.388 -> 0.278.
+// The L1 data pipe is 86% busy (120 = 15 8): twiddles are loaded as 8 bytes and
+// duplicated in registers (as 16-byte pairs 150 took 0.215, 180 0.290).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -121,9 +123,8 @@ template <> struct El<false> {
   static __device__ __forceinline__ V load(const float2* g, long long) { return *g; }
   static __device__ __forceinline__ void store(float2* g, long long, int, V v) { *g = v; }
   template <int R, bool INV> static __device__ __forceinline__ void fft(V* v) { dft<R, INV>(v); }
-  template <bool CONJ> static __device__ __forceinline__ V tw(V v, const float4* p) {
-    const float4 t = __ldg(p);
-    const float2 w = make_float2(t.x, t.z);
+  template <bool CONJ> static __device__ __forceinline__ V tw(V v, const float2* p) {
+    const float2 w = ldg_c(p);
     return CONJ ? cmulc(v, w) : cmul(v, w);
   }
 };
@@ -153,22 +154,22 @@ template <> struct El<true> {
     if (n > 1) g[rhs] = b;
   }
   template <int R, bool INV> static __device__ __forceinline__ void fft(V* v) { pk::dft<R, INV>(v); }
-  template <bool CONJ> static __device__ __forceinline__ V tw(V v, const float4* p) {
-    pk::u64 c, s;
-    pk::ld_tw(p, c, s);
+  template <bool CONJ> static __device__ __forceinline__ V tw(V v, const float2* p) {
+    const float2 w = ldg_c(p);
+    const pk::u64 c = pk::dup(w.x), s = pk::dup(w.y);
     return CONJ ? pk::tw_mulc(v, c, s) : pk::tw_mul(v, c, s);
   }
 };
 
 // Stage 0 < s < last, in place.
 template <class P, bool PAIR, int NT, int s, bool INV>
-__device__ __forceinline__ void stage(typename El<PAIR>::E* sm, const float4* __restrict__ tw, int tid, int nthr) {
+__device__ __forceinline__ void stage(typename El<PAIR>::E* sm, const float2* __restrict__ tw, int tid, int nthr) {
   using X = El<PAIR>;
   constexpr int R = P::rad[s], M = P::M(s), Ls = M * R, B = P::N / R, off = Lay<P>::off(s);
   for (int t = tid; t < NT * 3 * B; t += nthr) {
     const int j = t / B, u = t - j * B, b = u / M, n1 = u - b * M;
     typename X::E* p = sm + j * Lay<P>::LW + Lay<P>::addr(b * Ls + n1);
-    const float4* tws = tw + P::TWO(s) + n1;
+    const float2* tws = tw + P::TWO(s) + n1;
     typename X::V v[R];
 #pragma unroll
     for (int i = 0; i < R; ++i) v[i] = X::get(p + i * off);
@@ -185,7 +186,7 @@ __device__ __forceinline__ void stage(typename El<PAIR>::E* sm, const float4* __
   __syncthreads();
 }
 template <class P, bool PAIR, int NT, int s, bool INV>
-__device__ __forceinline__ void inner(typename El<PAIR>::E* sm, const float4* tw, int tid, int nthr) {
+__device__ __forceinline__ void inner(typename El<PAIR>::E* sm, const float2* tw, int tid, int nthr) {
   if constexpr (s > 0 && s < P::nst - 1) {
     stage<P, PAIR, NT, s, INV>(sm, tw, tid, nthr);
     inner<P, PAIR, NT, INV ? s - 1 : s + 1, INV>(sm, tw, tid, nthr);
@@ -194,7 +195,7 @@ __device__ __forceinline__ void inner(typename El<PAIR>::E* sm, const float4* tw
 
 template <class P, bool PAIR, int NT>
 __global__ void __launch_bounds__(threads<P, PAIR>(NT), std::max(1, sm_threads<P, PAIR>() / threads<P, PAIR>(NT)))
-k_pass_c(float2* __restrict__ t2, int L, int nlines, int nz, int nzp, const float4* __restrict__ tw,
+k_pass_c(float2* __restrict__ t2, int L, int nlines, int nz, int nzp, const float2* __restrict__ tw,
          const float2* __restrict__ ghat, const int* done) {
   using X = El<PAIR>;
   constexpr int nthr = threads<P, PAIR>(NT);
@@ -303,7 +304,7 @@ k_pass_c(float2* __restrict__ t2, int L, int nlines, int nz, int nzp, const floa
 }
 
 template <class P, bool PAIR, int NT>
-cudaError_t launch_nt(const MvpGeom& g, float2* t2, int L, const float4* tw, const float2* ghat, long long ntask,
+cudaError_t launch_nt(const MvpGeom& g, float2* t2, int L, const float2* tw, const float2* ghat, long long ntask,
                       cudaStream_t st, const int* done) {
   constexpr int smem = smem_bytes<P, PAIR>(NT);
   static std::once_flag once;
@@ -318,7 +319,7 @@ cudaError_t launch_nt(const MvpGeom& g, float2* t2, int L, const float4* tw, con
 }
 
 template <class P, bool PAIR>
-cudaError_t launch(const MvpGeom& g, float2* t2, int L, const float4* tw, const float2* ghat, cudaStream_t st,
+cudaError_t launch(const MvpGeom& g, float2* t2, int L, const float2* tw, const float2* ghat, cudaStream_t st,
                    const int* done) {
   const long long ntask = (long long)g.Px * g.Py * (PAIR ? (L + 1) / 2 : L);
   return launch_nt<P, PAIR, tasks<P, PAIR>()>(g, t2, L, tw, ghat, ntask, st, done);
@@ -326,9 +327,9 @@ cudaError_t launch(const MvpGeom& g, float2* t2, int L, const float4* tw, const 
 
 // Runs pass C when the length is in range and f = 3.  MvpTune::zkern 1 runs pairs, 0 does not; by default pairs for even
 // L and from L = 7: an empty half costs less than the pairs save there (9216 lines of 150, per right-hand side: pairs
-// 13.5 us at L = 16, single 14.5; at L = 3 19.9 and 17.3).
+// 12.8 us at L = 16, single 13.9; at L = 3 19.0 and 16.4).
 template <class P>
-bool launch(const MvpGeom& g, float2* t2, int L, const float4* tw, const float2* ghat, cudaStream_t st, const int* done,
+bool launch(const MvpGeom& g, float2* t2, int L, const float2* tw, const float2* ghat, cudaStream_t st, const int* done,
             cudaError_t* err) {
   if constexpr (supported<P>()) {
     if (g.f != 3) return false;
