@@ -840,6 +840,8 @@ static int ensure_work(Op* op, int n, int L, int itermax, bool need64, bool need
     set((const void*)k_small_cocg_alpha<double, double2>, mx);
     set((const void*)k_small_solve<double, double2>, mx);
     set((const void*)k_small_solve<double, dfc>, mx);
+    set((const void*)k_small_store_reduce<double2>, mx);
+    set((const void*)k_small_store_reduce<dfc>, mx);
     set((const void*)k_small_chol1<dfl, dfc>, mx);
     set((const void*)k_small_chol2<dfl, dfc>, mx);
     set((const void*)k_small_cocg_alpha<dfl, dfc>, mx);
