@@ -107,6 +107,32 @@ template <int D, bool CJ> BDDA_FX_FN Val cmul(Val z, int rh, int rl, int ih, int
   else return {(mr + (cr >> 32) + (1ll << (D - 3))) >> (D - 2), (mi + (ci >> 32) + (1ll << (D - 3))) >> (D - 2)};
 }
 
+// Sum of complex products Fac x Val, scaled as its Val operands; one shift and rounding at the end.
+struct Split { int xh, xl, yh, yl; };
+BDDA_FX_FN Split split(Val v) {
+  Split s;
+  split(v.x, s.xh, s.xl);
+  split(v.y, s.yh, s.yl);
+  return s;
+}
+struct Acc {
+  long long cr = 1ll << 29, ci = 1ll << 29, mr = 0, mi = 0;
+  BDDA_FX_FN void mad(const Fac& g, const Split& s) {
+    cr += (mw(s.xh, g.rl) + mw(s.xl, g.rh)) - (mw(s.yh, g.il) + mw(s.yl, g.ih));
+    mr += mw(s.xh, g.rh) - mw(s.yh, g.ih);
+    ci += (mw(s.xh, g.il) + mw(s.xl, g.ih)) + (mw(s.yh, g.rl) + mw(s.yl, g.rh));
+    mi += mw(s.xh, g.ih) + mw(s.yh, g.rh);
+  }
+  // the products are subtracted: a low half of -2^31 has no negative in 32 bits
+  BDDA_FX_FN void msub(const Fac& g, const Split& s) {
+    cr -= (mw(s.xh, g.rl) + mw(s.xl, g.rh)) - (mw(s.yh, g.il) + mw(s.yl, g.ih));
+    mr -= mw(s.xh, g.rh) - mw(s.yh, g.ih);
+    ci -= (mw(s.xh, g.il) + mw(s.xl, g.ih)) + (mw(s.yh, g.rl) + mw(s.yl, g.rh));
+    mi -= mw(s.xh, g.ih) + mw(s.yh, g.rh);
+  }
+  BDDA_FX_FN Val get() const { return {shl(mr, 2) + (cr >> 30), shl(mi, 2) + (ci >> 30)}; }
+};
+
 // ---- butterflies: forward exp(-2 pi i / R), INV exp(+2 pi i / R) --------------
 constexpr long long kS60 = 3993837246235628775ll;   // sin 60, Q62
 constexpr long long kHalfRt = 3260954456333195553ll;  // sqrt(1/2)

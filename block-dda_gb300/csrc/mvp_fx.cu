@@ -38,7 +38,9 @@ namespace bdda {
 
 namespace {
 
+using fx::Acc;
 using fx::Fac;
+using fx::Split;
 using fx::Val;
 
 constexpr int kFxWarps = 4;                    // warps of a strided pass's CTA
@@ -314,27 +316,6 @@ k_fx_e(const Val* __restrict__ t1, const int* __restrict__ ein, int nfield, int 
 }
 
 // ---------------------------------------------------------------- pass C
-// Sum of complex products Fac x Val, scaled as its Val operands; one shift and rounding at the end.
-struct Split { int xh, xl, yh, yl; };
-__device__ __forceinline__ Split split(Val v) {
-  Split s;
-  fx::split(v.x, s.xh, s.xl);
-  fx::split(v.y, s.yh, s.yl);
-  return s;
-}
-struct Acc {
-  long long cr = 1ll << 29, ci = 1ll << 29, mr = 0, mi = 0;
-  __device__ __forceinline__ void mad(const Fac& g, const Split& s) {
-    using fx::mw;
-    cr += (mw(s.xh, g.rl) + mw(s.xl, g.rh)) - (mw(s.yh, g.il) + mw(s.yl, g.ih));
-    mr += mw(s.xh, g.rh) - mw(s.yh, g.ih);
-    ci += (mw(s.xh, g.il) + mw(s.xl, g.ih)) + (mw(s.yh, g.rl) + mw(s.yl, g.rh));
-    mi += mw(s.xh, g.ih) + mw(s.yh, g.rh);
-  }
-  __device__ __forceinline__ void msub(const Fac& g, const Split& s) { mad(Fac{-g.rh, -g.rl, -g.ih, -g.il}, s); }
-  __device__ __forceinline__ Val get() const { return {fx::shl(mr, 2) + (cr >> 30), fx::shl(mi, 2) + (ci >> 30)}; }
-};
-
 // One warp per (x = q, y = qy, rhs l): fc component lines, blockDim.x / 32 warps per CTA.
 template <bool SIX, int MB>
 __global__ void __launch_bounds__(kZWarps * 32, MB)
@@ -393,7 +374,7 @@ k_fx_c(Val* __restrict__ t2, int L, int Px, int Py, int nz, int nzp, fx::Plan p,
     for (int c = 0; c < nc; ++c) g[c] = fx::ldfac(gl + (size_t)c * Pz + f);
     Split e[fc];
 #pragma unroll
-    for (int c = 0; c < fc; ++c) e[c] = split(s0[c * LW + a]);
+    for (int c = 0; c < fc; ++c) e[c] = fx::split(s0[c * LW + a]);
     auto put = [&](int c, const Acc& acc) {
       const Val v = acc.get();
       used |= fx::bits_of(v);

@@ -1,0 +1,27 @@
+// The fixed-point arithmetic of the FP64 and double-float block MVPs, compiled for the host from the device source
+// (tests/test_fixed_point_arith.py).
+#include <cmath>
+
+#include "fx_fft.cuh"
+
+using namespace bdda;
+
+extern "C" {
+
+// Sum of n products of Q62 factors g (re, im) and values z, those with sub[i] subtracted.
+void fx_products(int n, const long long* g, const long long* z, const int* sub, long long* out) {
+  fx::Acc acc;
+  for (int i = 0; i < n; ++i) {
+    fx::Fac f;
+    fx::split(g[2 * i], f.rh, f.rl);
+    fx::split(g[2 * i + 1], f.ih, f.il);
+    const fx::Split s = fx::split(fx::Val{z[2 * i], z[2 * i + 1]});
+    if (sub[i]) acc.msub(f, s);
+    else acc.mad(f, s);
+  }
+  const fx::Val v = acc.get();
+  out[0] = v.x;
+  out[1] = v.y;
+}
+
+}  // extern "C"

@@ -1,0 +1,45 @@
+"""Arithmetic of the fixed-point block MVPs (fx_fft.cuh) on the host, against exact integers."""
+import ctypes as ct
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+from conftest import ROOT
+
+
+@pytest.fixture(scope="module")
+def fx(tmp_path_factory):
+    so = str(tmp_path_factory.mktemp("fx") / "fx_arith.so")
+    subprocess.run(["g++", "-std=c++17", "-O2", "-ffp-contract=off", "-shared", "-fPIC",
+                    "-I", os.path.join(ROOT, "block-dda_gb300", "csrc"), "-I", "/usr/local/cuda/include",
+                    os.path.join(ROOT, "tests", "cpp", "fx_arith.cpp"), "-o", so], check=True)
+    return ct.CDLL(so)
+
+
+def _ll(v):
+    return np.ascontiguousarray(v, dtype=np.int64).ctypes.data_as(ct.POINTER(ct.c_longlong))
+
+
+# A product drops the two low x low terms of each part (below 2^31 2^31 / 2^62 = 1 unit each) and a sum is rounded once.
+@pytest.mark.parametrize("low", [0x80000000, 0x7FFFFFFF, 0x80000001, 0, 0xFFFFFFFF])
+@pytest.mark.parametrize("sub", [0, 1])
+def test_products_at_the_ends_of_the_low_half(fx, low, sub):
+    rng = np.random.default_rng(low % 1000 + sub)
+    for part in range(4):                      # which of g.re, g.im, z.re, z.im has the low word
+        for _ in range(50):
+            v = [int(a) for a in rng.integers(-2 ** 59, 2 ** 59, 8)]
+            v[part] = (v[part] >> 32 << 32) | low
+            g, z = v[0:2] + v[4:6], v[2:4] + v[6:8]
+            s = [sub, 0]
+            out = np.zeros(2, np.int64)
+            fx.fx_products(2, _ll(g), _ll(z), np.array(s, np.int32).ctypes.data_as(ct.POINTER(ct.c_int)), _ll(out))
+            re = im = 0
+            for i in range(2):
+                sg = -1 if s[i] else 1
+                a, b, c, d = g[2 * i], g[2 * i + 1], z[2 * i], z[2 * i + 1]
+                re += sg * (a * c - b * d)
+                im += sg * (a * d + b * c)
+            assert abs(int(out[0]) * 2 ** 62 - re) <= 5 * 2 ** 62
+            assert abs(int(out[1]) * 2 ** 62 - im) <= 5 * 2 ** 62
