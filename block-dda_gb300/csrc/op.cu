@@ -87,8 +87,7 @@ Op::~Op() {
   tws32z.release(); tws32c.release(); fxpos.release();
   ghat32.release(); ghatfx.release(); gexpfx.release();
   kstat.release();
-  for (int i = 0; i < 2; ++i) { t1[i].release(); t2[i].release(); }
-  texp.release();
+  for (int i = 0; i < 3; ++i) { t1[i].release(); t2[i].release(); texp[i].release(); }
   if (stream) {
     wait_stream(stream);
     cudaStreamDestroy(stream);
@@ -280,11 +279,11 @@ int op_block_mvp(Op* op, const Occupancy& o, const typename cplx<T>::type* x, in
   MvpGeom g = op->geom(o);
   const size_t eb = std::is_same<T, float>::value ? 0 : FxWork::exp_elems(g, L) * sizeof(int);
   const bool grow = op->t1[pi].bytes < mvp_t1_elems(g, L) * sizeof(C) || op->t2[pi].bytes < mvp_t2_elems(g, L) * sizeof(C) ||
-                    op->texp.bytes < eb;
+                    op->texp[pi].bytes < eb;
   if (grow && st != op->stream) BDDA_TRY_CUDA(order_after(op->stream, st));  // old buffers may be in use on st
   BDDA_CUDA(op->t1[pi].ensure(mvp_t1_elems(g, L) * sizeof(C), op->stream));
   BDDA_CUDA(op->t2[pi].ensure(mvp_t2_elems(g, L) * sizeof(C), op->stream));
-  if (eb) BDDA_CUDA(op->texp.ensure(eb, op->stream));
+  if (eb) BDDA_CUDA(op->texp[pi].ensure(eb, op->stream));
   if (grow && st != op->stream) BDDA_TRY_CUDA(order_after(st, op->stream));  // new buffers exist before st uses them
   cudaError_t e;
   if constexpr (std::is_same<T, float>::value) {
@@ -318,7 +317,7 @@ int op_block_mvp(Op* op, const Occupancy& o, const typename cplx<T>::type* x, in
                                 &op->timer, done);
   } else {
     e = launch_block_mvp_fx(g, op->tables_fx(), std::is_same<T, dfl>::value, x, ldx, y, ldy, L, diag, jpre,
-                            FxWork(op->t1[pi].p, op->t2[pi].p, op->texp.as<int>(), g, L), st, &op->timer, done);
+                            FxWork(op->t1[pi].p, op->t2[pi].p, op->texp[pi].as<int>(), g, L), st, &op->timer, done);
   }
   if (e != cudaSuccess) return cuda_fail(e, "block MVP launch");
   return BDDA_OK;

@@ -99,8 +99,9 @@ struct Op {
   Occupancy dip;    // dipole occupancy (set_dipoles)
   unsigned long long dip_epoch = 0;  // bumped whenever dip is rebuilt (captured MVPs hold its sizes)
   Occupancy cub;    // every cuboid site (the reference's MBT_fft_mvp vector)
-  DevBuf t1[2], t2[2];   // MVP workspace (0 = FP64 and double-float, 1 = FP32)
-  DevBuf texp;           // line exponents of workspace 0 (FxWork)
+  // MVP workspace per precision (0 = FP64, 1 = FP32, 2 = double-float): MVPs of two precisions may be in flight on two streams
+  DevBuf t1[3], t2[3];
+  DevBuf texp[3];        // line exponents of workspaces 0 and 2 (FxWork)
   cudaStream_t stream = nullptr;
   KernelTimer timer;
   std::mutex mu;
@@ -121,10 +122,8 @@ struct Op {
   unsigned long long buffer_sig() const {
     unsigned long long h = 0;
     for (int i = 0; i < 3; ++i)
-      for (const DevBuf* b : {&tw32[i], &twfx[i], &tws32p[i]}) h = sig_add(h, *b);
-    for (int i = 0; i < 2; ++i)
-      for (const DevBuf* b : {&t1[i], &t2[i]}) h = sig_add(h, *b);
-    for (const DevBuf* b : {&texp, &ghat32, &ghatfx, &gexpfx, &tws32z, &tws32c, &kstat, &dip.occ, &dip.tiles, &dip.tmask})
+      for (const DevBuf* b : {&tw32[i], &twfx[i], &tws32p[i], &t1[i], &t2[i], &texp[i]}) h = sig_add(h, *b);
+    for (const DevBuf* b : {&ghat32, &ghatfx, &gexpfx, &tws32z, &tws32c, &kstat, &dip.occ, &dip.tiles, &dip.tmask})
       h = sig_add(h, *b);
     return h;
   }
@@ -161,11 +160,11 @@ struct Op {
   ~Op();
 };
 
-// Workspace slot and precision bit of each vector type (FP64 and double-float share the fixed-point MVP's workspace).
+// Workspace slot and precision bit of each vector type.
 template <typename T> struct PrecInfo;
 template <> struct PrecInfo<double> { static constexpr int slot = 0, bit = 1; };
 template <> struct PrecInfo<float> { static constexpr int slot = 1, bit = 2; };
-template <> struct PrecInfo<dfl> { static constexpr int slot = 0, bit = 4; };
+template <> struct PrecInfo<dfl> { static constexpr int slot = 2, bit = 4; };
 
 // Make stream 'later' wait for the work enqueued so far on 'earlier'.
 cudaError_t order_after(cudaStream_t later, cudaStream_t earlier);
