@@ -219,18 +219,24 @@ struct WarpTeam {
   __device__ void sync() const { __syncwarp(); }
 };
 
-// Integer that orders values by |a|^2 (the top 32 bits of its FP64 or FP32 pattern; NaN is the largest).
-__device__ __forceinline__ unsigned mag_key(double2 a) { return (unsigned)__double2hiint(m_abs2(a)); }
+// Integer that orders values by |a|^2 (the top 32 bits of its FP64 or FP32 pattern; NaN is the largest), 0 only where
+// |a|^2 is.
+__device__ __forceinline__ unsigned mag_key(double2 a) {
+  const double m = m_abs2(a);
+  const unsigned h = (unsigned)__double2hiint(m);
+  return h != 0 ? h : __double2loint(m) != 0 ? 1u : 0u;
+}
 __device__ __forceinline__ unsigned mag_key(dfc a) { return __float_as_uint(a.x.hi * a.x.hi + a.y.hi * a.y.hi); }
 
 // Pivot of step k by one warp: the largest |a| (to the 20 or 23 bits of mag_key; the first in row order among equals, with
-// full in column order first) of the rows and columns not used yet.  Lane r holds row r.
+// full in column order first) of the rows and columns not used yet.  Lane r holds row r.  Where all of them are zero the
+// pivot is one of these zeros (used columns keep old values), which the caller's test of it refuses.
 template <typename M>
 __device__ __forceinline__ void find_pivot(const M* A, int L, int k, bool full, unsigned rows, unsigned cols, int* pr, int* pc) {
   const int lane = threadIdx.x & 31;
   const bool row = lane < L && ((rows >> lane) & 1u);
   unsigned best = 0;
-  int bc = k;
+  int bc = full ? __ffs((int)cols) - 1 : k;
   if (!full) {
     best = row ? mag_key(A[lane + k * L]) : 0;
   } else if (row) {
