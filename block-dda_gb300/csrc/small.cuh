@@ -92,14 +92,25 @@ template <typename M> __device__ __forceinline__ M m_neg(M a) { return cmake(-a.
 template <typename M> __device__ __forceinline__ bool m_finite(M a) {
   return isfinite(r_to_double(a.x)) && isfinite(r_to_double(a.y));
 }
-// 1 / b; operands are O(1) pivots (no scaling against overflow)
+// Whether 1 / a keeps FP64's precision (solves of very small or large right-hand sides have Gram sums near its ends).
+__device__ __forceinline__ bool r_recip_ok(double a) { return a > 0x1p-1000 && a < 0x1p1000; }
+__device__ __forceinline__ bool r_recip_ok(dfl) { return true; }
+// 1 / b; operands are O(1) pivots (no scaling against overflow of |b|^2)
 __device__ __forceinline__ double2 m_recip(double2 b) {
-  const double d = 1.0 / (b.x * b.x + b.y * b.y);
+  const double n = b.x * b.x + b.y * b.y;
+  if (!r_recip_ok(n)) return make_double2(b.x / n, -b.y / n);
+  const double d = 1.0 / n;
   return make_double2(b.x * d, -b.y * d);
 }
 __device__ __forceinline__ dfc m_recip(dfc b) {
   const dfl d = df_recip(b.x * b.x + b.y * b.y);
   return cmake(b.x * d, -(b.y * d));
+}
+// conj(a) / b, b real
+__device__ __forceinline__ double2 m_over(double2 a, double b) { return make_double2(a.x / b, -a.y / b); }
+__device__ __forceinline__ dfc m_over(dfc a, dfl b) {
+  const dfl q = df_recip(b);
+  return cmake(a.x * q, -(a.y * q));
 }
 // a / b; operands are O(1) pivots (no scaling against overflow)
 __device__ __forceinline__ double2 m_div(double2 a, double2 b) {
@@ -388,7 +399,7 @@ __device__ void ldl_team(const Team tm, typename SmallMat<R>::M* U, int L, R* di
     }
     if (c.i > k && c.i < L) {
       const M u = U[k + c.i * L];
-      const M l = cmake(u.x * di, -(u.y * di));  // L_ik
+      const M l = r_recip_ok(d) ? cmake(u.x * di, -(u.y * di)) : m_over(u, d);  // L_ik
       for (int j = c.j0; j < L; j += c.step) {
         if (j > k && j < c.i) continue;  // neither triangle has (i, j) at this step
         M* col = U + j * L;

@@ -1,6 +1,7 @@
 """The one-CTA L x L routines of the block solvers on matrices of the test's
-own: singular ones that complete pivoting has to refuse, for the widths of one
-warp (up to 8) and of the whole CTA."""
+own: singular ones that complete pivoting has to refuse, and FP64 values whose
+reciprocal is beyond its range, for the widths of one warp (up to 8) and of the
+whole CTA."""
 import ctypes as ct
 import os
 import subprocess
@@ -63,4 +64,37 @@ def test_lu_solves(steps, L, full, df):
     assert ok == 1
     want = np.linalg.solve(A, B)
     eps = 2.0 ** -44 if df else 2.0 ** -52
+    assert np.linalg.norm(x - want) <= 8 * L * eps * np.linalg.cond(A) * np.linalg.norm(want)
+
+
+# The Gram sums of a solve whose right-hand sides are about 1e-155 or 1e153: 2^-1034 (40 bits left) and 2^1018.
+# Cholesky factor and inverse of s H are those of H times sqrt(s) and its inverse; both are compared with H's.
+@pytest.mark.parametrize("L", [1, 2, 8, 9, 32])
+@pytest.mark.parametrize("e, eps", [(-1034, 2.0 ** -40), (0, 2.0 ** -52), (1018, 2.0 ** -52)])
+def test_cholesky_over_the_range_of_fp64(steps, L, e, eps):
+    rng = np.random.default_rng(L)
+    W = rng.standard_normal((4 * L, L)) + 1j * rng.standard_normal((4 * L, L))
+    H = W.conj().T @ W / L
+    h = np.ldexp(H.real, e) + 1j * np.ldexp(H.imag, e)
+    H = np.ldexp(h.real, -e) + 1j * np.ldexp(h.imag, -e)            # as rounded
+    h, r, ri, ok = np.asfortranarray(h), np.zeros((L, L), complex, "F"), np.zeros((L, L), complex, "F"), ct.c_int(-1)
+    assert steps.chol(_ptr(h), _ptr(r), _ptr(ri), L, 0, ct.byref(ok)) == 0
+    assert ok.value == 1
+    R = np.linalg.cholesky(H).conj().T
+    tol = 8 * L * eps * np.linalg.cond(H)
+    assert np.linalg.norm(r * 2.0 ** (-e // 2) - R) <= tol * np.linalg.norm(R)
+    assert np.linalg.norm(ri * 2.0 ** (e // 2) - np.linalg.inv(R)) <= tol * np.linalg.norm(np.linalg.inv(R))
+
+
+# A pivot of 2^-520 has a square of 2^-1040, 34 bits; its reciprocal is within FP64.
+@pytest.mark.parametrize("full", [False, True])
+@pytest.mark.parametrize("L", [1, 2, 8, 9, 32])
+@pytest.mark.parametrize("e, eps", [(-520, 2.0 ** -32), (-505, 2.0 ** -52), (505, 2.0 ** -52)])
+def test_lu_over_the_range_of_fp64(steps, L, full, e, eps):
+    rng = np.random.default_rng(L)
+    A = rng.standard_normal((L, L)) + 1j * rng.standard_normal((L, L)) + 3 * np.sqrt(L) * np.eye(L)[rng.permutation(L)]
+    B = rng.standard_normal((L, L)) + 1j * rng.standard_normal((L, L))
+    x, ok = _lu(steps, A * 2.0 ** e, B * 2.0 ** e, full, False)
+    assert ok == 1
+    want = np.linalg.solve(A, B)
     assert np.linalg.norm(x - want) <= 8 * L * eps * np.linalg.cond(A) * np.linalg.norm(want)
