@@ -133,6 +133,20 @@ struct Acc {
   BDDA_FX_FN Val get() const { return {shl(mr, 2) + (cr >> 30), shl(mi, 2) + (ci >> 30)}; }
 };
 
+// Spectrum component that couples component c to row r of the block: symmetric A (xx xy xz yy yz zz), and with SIX
+// [A B; -B A], B antisymmetric (xy xz yz): index, -1 for none, and whether its product is subtracted.
+template <bool SIX> BDDA_FX_FN constexpr int green_comp(int r, int c) {
+  const int a = r % 3, b = c % 3;
+  return (r < 3) == (c < 3) ? a + b + (a != 0 && b != 0 ? 1 : 0) : a == b ? -1 : 5 + a + b;
+}
+BDDA_FX_FN constexpr bool green_sub(int r, int c) { return (r < 3) != (c < 3) && (r < 3) == (r % 3 > c % 3); }
+// Bits that a spectrum component stays below 1, and that values are shifted for the products at least: with the 3 (SIX: 5)
+// terms of a row the middle sums of Acc stay below 7.3 (4.8) 2^60 and its result below 2^62.  SIX could do with 2 bits of
+// the first; the exponents, and so the roundings, of the recorded f = 6 runs depend on it, whose loosely converged BiCGSTAB
+// results move by 1e-4 to 1.9e-3 with any rounding: with 3 bits they are within the 1e-3 that their tests ask, with 2 not.
+template <bool SIX> constexpr int kGreenBits = SIX ? 3 : 1;
+template <bool SIX> constexpr int kProductBits = SIX ? 2 : 1;
+
 // ---- butterflies: forward exp(-2 pi i / R), INV exp(+2 pi i / R) --------------
 constexpr long long kS60 = 3993837246235628775ll;   // sin 60, Q62
 constexpr long long kHalfRt = 3260954456333195553ll;  // sqrt(1/2)
@@ -476,7 +490,7 @@ BDDA_FX_FN Val align(Val v, int r) {
 
 // ---- stages ---------------------------------------------------------------------
 // Input of a stage: RAW: FP64 bits to convert with the line's scale (rsh[j]),
-// FIXED, SHIFT: fixed values to shift right by rsh[0] (left where negative),
+// FIXED, SHIFT: fixed values to shift right by rsh[j] (left where negative),
 // ALIGN: stored values of element exponents ex[j * exs + idx], shifted right by rsh[j] - ex.
 enum In { kRaw, kFixed, kShift, kAlign };
 struct InArgs {
@@ -488,8 +502,7 @@ struct InArgs {
 // One stage over NL lines of a warp (line j at s + j p.LW).  PRUNE: only
 // elements idx < nv (nv <= N / 2) are read (forward) or written (inverse), so
 // butterfly elements i with 2 i >= R are compile-time zeros or dead.  used
-// (USED: the last stage): line j's bits in use at used[j], or of all lines at
-// used[0] for NL = 3.
+// (USED: the last stage): line j's bits in use at used[j].
 template <int R, bool INV, int NL, int IN, bool PRUNE, bool USED>
 BDDA_FX_FN void stage(Val* __restrict__ s, const Plan& p, int st, const Fac* __restrict__ tw, int lane, int lanes, int nv,
                       const InArgs& in, int* used) {
@@ -504,7 +517,7 @@ BDDA_FX_FN void stage(Val* __restrict__ s, const Plan& p, int st, const Fac* __r
     const int n1 = u - b * M, idx0 = b * M * R + n1;
     Val* q = s + j * p.LW + p.addr(idx0);
     Val v[R];
-    const int rs = IN == kFixed ? 0 : NL == 2 ? (j ? in.rsh[1] : in.rsh[0]) : in.rsh[0];
+    const int rs = IN == kFixed ? 0 : NL == 3 && j == 2 ? in.rsh[NL - 1] : NL > 1 && j ? in.rsh[NL > 1] : in.rsh[0];  // rsh[j]
     const int* ex = IN == kAlign ? in.ex + j * in.exs + idx0 : nullptr;
 #pragma unroll
     for (int i = 0; i < R; ++i) {
@@ -543,12 +556,8 @@ BDDA_FX_FN void stage(Val* __restrict__ s, const Plan& p, int st, const Fac* __r
       if (USED) o |= bits_of(v[i]);
     }
     if (USED) {
-      if (NL == 2) {
-        used[0] |= j ? 0 : o;
-        used[1] |= j ? o : 0;
-      } else {
-        used[0] |= o;
-      }
+#pragma unroll
+      for (int k = 0; k < NL; ++k) used[k] |= j == k ? o : 0;
     }
   }
   BDDA_FX_SYNCWARP();

@@ -114,7 +114,7 @@ template <typename T> struct MvpPrec {
 
 // Tables of the fixed-point MVP (FP64 and double-float, mvp_fx.cu): axis plans,
 // Q62 twiddles, and the Green spectrum [Px][Py][6 or 9][Pz] / (Px Py Pz) as Q62
-// over one power of two per (x, y) line.
+// over one power of two per (x, y) line and component.
 struct FxTables {
   fx::Plan plan[3];
   const fx::Fac* tw[3];
@@ -293,12 +293,12 @@ bool pipe_z_available(int Pz, int f, int nzp, int L);
 
 // Workspace of the fixed-point MVP: T1 and T2 (16 bytes per element) and the
 // exponents of their lines: after pass A [f L][ny][nzp], after B and D
-// [f L][Px][nzp], after C [L][Px][Py], carved in that order from one array.
+// [f L][Px][nzp], after C [f L][Px][Py], carved in that order from one array.
 struct FxWork {
   void *t1, *t2;
   int *ea, *eb, *ec;
   static size_t exp_elems(const MvpGeom& g, int L) {
-    return (size_t)g.f * L * (g.ny + g.Px) * g.nzp + (size_t)L * g.Px * g.Py;
+    return (size_t)g.f * L * ((size_t)(g.ny + g.Px) * g.nzp + (size_t)g.Px * g.Py);
   }
   FxWork(void* t1_, void* t2_, int* e, const MvpGeom& g, int L)
       : t1(t1_), t2(t2_), ea(e), eb(e + (size_t)g.f * L * g.ny * g.nzp), ec(eb + (size_t)g.f * L * g.Px * g.nzp) {}

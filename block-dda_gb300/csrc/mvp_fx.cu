@@ -5,8 +5,8 @@
 // T1 / T2 hold fixed-point values (2 x 64 bits per element, the size of complex
 // FP64) in lines of the pass that wrote them, each line shifted up to 62 bits
 // with an exponent in a side array (FxExps):
-//   pass A -> ea[f][y][z] (x lines), B -> eb[f][x][z] (y lines), C -> ec[l][x][y]
-//   (z lines, one for the components of a right-hand side), D -> eb again.
+//   pass A -> ea[f][y][z] (x lines), B -> eb[f][x][z] (y lines), C -> ec[f][x][y]
+//   (z lines), D -> eb again.
 // The next pass aligns the elements of its lines, which come from lines of
 // different exponents, to the largest one: two 64-bit shifts and an addition
 // per part, where a conversion to FP64 and back took 80 instructions per
@@ -14,10 +14,12 @@
 // converts from FP64 (the gathered sites) and pass E to FP64 (the scattered
 // ones), so the values between the passes carry more bits than FP64's 53.
 //
-// The Green spectrum is held as Q62 integers with one exponent per (x, y) line,
-// scaled so that every row of the 3 x 3 (6 x 6) block has a modulus sum <= 1
-// and the product cannot grow a line past its bound; before its inverse
-// transform the z pass shifts the lines to that transform's headroom.
+// The Green spectrum is held as Q62 integers with one exponent per (x, y) line
+// and component.  In pass C every component of the vectors and of the product
+// has an exponent of its own too: where components do not couple (the normal
+// one of a flat target, the axial one of a chain; magnetic and electric ones at
+// small k d) a small one keeps its bits beside a large one.  The terms of a row
+// are aligned to its largest term as they are multiplied.
 //
 // The two precisions differ only in the vectors' storage (Io64, IoDf): pass E
 // adds diag o x and scales by jpre in FP64 on the occupied sites (3% of a
@@ -221,8 +223,8 @@ k_fx_a(const typename Io::E* __restrict__ x, int ldx, int nfield, int fpg, int f
 // ---------------------------------------------------------------- pass B / D
 template <bool INV, int MB>
 __global__ void __launch_bounds__(kFxThreads, MB)
-k_fx_y(const Val* __restrict__ src, Val* __restrict__ dst, const unsigned char* __restrict__ tmask, int fc, int Px, int ny,
-       int nz, int nzp, int nzt, fx::Plan p, const Fac* __restrict__ tw, const int* __restrict__ ein, int* __restrict__ eout,
+k_fx_y(const Val* __restrict__ src, Val* __restrict__ dst, const unsigned char* __restrict__ tmask, int Px, int ny, int nz, int nzp,
+       int nzt, fx::Plan p, const Fac* __restrict__ tw, const int* __restrict__ ein, int* __restrict__ eout,
        const int* done) {
   pdl_begin();
   if (skip(done)) return;
@@ -235,9 +237,8 @@ k_fx_y(const Val* __restrict__ src, Val* __restrict__ dst, const unsigned char* 
   const int nin = INV ? p.N : ny, nout = INV ? ny : p.N;
   const int zt = blockIdx.x % nzt, z0 = zt * kTZ;
   const int r = blockIdx.x / nzt;  // f * Px + q
-  const int f = r / Px, q = r - f * Px;
   const bool zval = z0 + col < nz;
-  const int* ei = INV ? ein + ((size_t)(f / fc) * Px + q) * p.N : ein + (size_t)f * ny * nzp + z0 + (zval ? col : 0);
+  const int* ei = INV ? ein + (size_t)r * p.N : ein + (size_t)(r / Px) * ny * nzp + z0 + (zval ? col : 0);
   if constexpr (INV)
     for (int i = tid; i < nin; i += kFxThreads) ex[i] = ei[i];
   fill_tile(lines, p, src + (size_t)r * nin * nzp + z0 + (zval ? col : 0), nzp, nin, col, row, [&](int yy) {
@@ -316,7 +317,11 @@ k_fx_e(const Val* __restrict__ t1, const int* __restrict__ ein, int nfield, int 
 }
 
 // ---------------------------------------------------------------- pass C
-// One warp per (x = q, y = qy, rhs l): fc component lines, blockDim.x / 32 warps per CTA.
+// One warp per (x = q, y = qy, rhs l): fc component lines, blockDim.x / 32 warps per CTA.  Bound by the integer multiplier
+// and the instructions around it.  An exponent per component costs the alignment of nine (f = 6: 30) factors per
+// frequency: 1.84 -> 2.00 ms at Pz=120 (N=8192, L=16), 3.90 -> 4.20 at 150, f = 6 0.151 -> 0.172 at 54 (N=1200, L=4),
+// against one for all of them, whose small components lost the bits between.  One shift for the rows of lines whose
+// spectrum components are close was no faster (4.2 ms): the second product loop cost what it saved.
 template <bool SIX, int MB>
 __global__ void __launch_bounds__(kZWarps * 32, MB)
 k_fx_c(Val* __restrict__ t2, int L, int Px, int Py, int nz, int nzp, fx::Plan p, const Fac* __restrict__ tw,
@@ -336,90 +341,115 @@ k_fx_c(Val* __restrict__ t2, int L, int Px, int Py, int nz, int nzp, fx::Plan p,
   const size_t fstride = (size_t)Px * Py * nzp, estride = (size_t)Px * nzp;
   Val* g0 = t2 + (size_t)(fc * l) * fstride + (size_t)line * nzp;
   const int* ei = ein + (size_t)(fc * l) * estride + (size_t)(line / Py) * nzp;
-  int* eo = eout + (size_t)l * Px * Py + line;
-  int emax = fx::kZeroExp;
+  int* eo = eout + (size_t)(fc * l) * Px * Py + line;
+  const size_t eostride = (size_t)Px * Py;
+  int em[fc];  // largest exponent of a component's elements
+#pragma unroll
+  for (int c = 0; c < fc; ++c) em[c] = fx::kZeroExp;
   for (int z = lane; z < nz; z += 32)
 #pragma unroll
-    for (int c = 0; c < fc; ++c) emax = max(emax, ei[c * estride + z]);
-  emax = __reduce_max_sync(0xffffffffu, emax);
-  const int ge = gexp[line];
-  if (emax <= fx::kZeroExp || emax == fx::kBadExp || ge == fx::kBadExp) {  // zero in, zero out; or not finite
-    if (lane == 0) *eo = ge == fx::kBadExp ? ge : emax;
+    for (int c = 0; c < fc; ++c) em[c] = max(em[c], ei[c * estride + z]);
+  int emax = fx::kZeroExp;
+#pragma unroll
+  for (int c = 0; c < fc; ++c) {
+    em[c] = __reduce_max_sync(0xffffffffu, em[c]);
+    emax = max(emax, em[c]);
+  }
+  const int ge = lane < nc ? gexp[(size_t)line * nc + lane] : fx::kZeroExp;  // lane i: exponent of spectrum component i
+  const bool gbad = __any_sync(0xffffffffu, ge == fx::kBadExp);
+  if (emax <= fx::kZeroExp || emax == fx::kBadExp || gbad) {  // zero in, zero out; or not finite
+    if (lane < fc) eo[lane * eostride] = gbad ? fx::kBadExp : emax;
     return;
   }
-  int in = 0;
+  int in[fc] = {};
   for (int z = lane; z < nz; z += 32) {
     const int a = p.addr(z);
 #pragma unroll
     for (int c = 0; c < fc; ++c) {
-      const Val v = fx::align(g0[c * fstride + z], emax + 1 - ei[c * estride + z]);
-      in |= fx::bits_of(v);
+      const Val v = fx::align(g0[c * fstride + z], em[c] + 1 - ei[c * estride + z]);
+      in[c] |= fx::bits_of(v);
       s0[c * LW + a] = v;
     }
   }
-  // to the forward transform's headroom (the spectral product adds three or five complex products before it shifts: one
-  // or two bits more)
-  in = (int)__reduce_or_sync(0xffffffffu, (unsigned)in);
-  const int fsh[1] = {64 - __clz(in) - (fx::kTopBit - 1 - p.headroom(false, clog2(nz)) - (SIX ? 2 : 1))};
+  // each component to the forward transform's headroom; lane c keeps the exponent of component c's transform
+  int fsh[fc], ev = fx::kZeroExp;
+#pragma unroll
+  for (int c = 0; c < fc; ++c) {
+    fsh[c] = 64 - __clz(__reduce_or_sync(0xffffffffu, (unsigned)in[c])) - (fx::kTopBit - 1 - p.headroom(false, clog2(nz)));
+    if (lane == c && em[c] > fx::kZeroExp) ev = em[c] + 1 + fsh[c] + p.D;
+  }
   __syncwarp();
   constexpr int halves = SIX ? 2 : 1;
+#pragma unroll
   for (int h = 0; h < halves; ++h)
-    fx::forward<3, fx::kShift, true, false>(s0 + 3 * h * LW, p, tw, lane, 32, nz, {fsh, nullptr, 0}, nullptr);
+    fx::forward<3, fx::kShift, true, false>(s0 + 3 * h * LW, p, tw, lane, 32, nz, {fsh + 3 * h, nullptr, 0}, nullptr);
+  // lane r: exponent of row r's products, from its largest term (exponents of its spectrum components and values)
+  int er = fx::kZeroExp;
+#pragma unroll
+  for (int c = 0; c < fc; ++c) {
+    const int i = fx::green_comp<SIX>(lane < fc ? lane : 0, c);
+    const int v = __shfl_sync(0xffffffffu, ev, c), g = __shfl_sync(0xffffffffu, ge, i < 0 ? 0 : i);
+    if (lane < fc && i >= 0 && v > fx::kZeroExp && g > fx::kZeroExp) er = max(er, v + g + fx::kProductBits<SIX>);
+  }
+  unsigned sh[fc][halves];  // shift of component c for row r: byte c % 3 of sh[r][c / 3]
+#pragma unroll
+  for (int r = 0; r < fc; ++r)
+#pragma unroll
+    for (int h = 0; h < halves; ++h) {
+      sh[r][h] = 0;
+#pragma unroll
+      for (int b = 0; b < 3; ++b) {
+        const int c = 3 * h + b, i = fx::green_comp<SIX>(r, c);
+        if (i < 0) continue;
+        const int d = __shfl_sync(0xffffffffu, er, r) - __shfl_sync(0xffffffffu, ev, c) - __shfl_sync(0xffffffffu, ge, i);
+        sh[r][h] |= (unsigned)min(max(d, 1), 62) << (8 * b);  // a zero component's shift does not matter
+      }
+    }
   const Fac* gl = ghat + (size_t)line * nc * Pz;
-  int used = 0;
+  int used[fc] = {};
   for (int f = lane; f < Pz; f += 32) {
     const int a = p.addr(f);
     Fac g[nc];
 #pragma unroll
     for (int c = 0; c < nc; ++c) g[c] = fx::ldfac(gl + (size_t)c * Pz + f);
-    Split e[fc];
+    Val e[fc];
 #pragma unroll
-    for (int c = 0; c < fc; ++c) e[c] = fx::split(s0[c * LW + a]);
-    auto put = [&](int c, const Acc& acc) {
-      const Val v = acc.get();
-      used |= fx::bits_of(v);
-      s0[c * LW + a] = v;
-    };
+    for (int c = 0; c < fc; ++c) e[c] = s0[c * LW + a];
 #pragma unroll
-    for (int r = 0; r < 3; ++r) {
-      // rows of the symmetric A: xx xy xz / xy yy yz / xz yz zz
-      const int i0 = r, i1 = r == 0 ? 1 : r + 2, i2 = r == 0 ? 2 : r + 3;
+    for (int r = 0; r < fc; ++r) {
       Acc acc;
-      acc.mad(g[i0], e[0]);
-      acc.mad(g[i1], e[1]);
-      acc.mad(g[i2], e[2]);
-      if constexpr (SIX) {  // E' = A E + B M, B antisymmetric (xy, xz, yz)
-        if (r == 0) { acc.mad(g[6], e[4]); acc.mad(g[7], e[5]); }
-        if (r == 1) { acc.mad(g[8], e[5]); acc.msub(g[6], e[3]); }
-        if (r == 2) { acc.msub(g[7], e[3]); acc.msub(g[8], e[4]); }
+#pragma unroll
+      for (int c = 0; c < fc; ++c) {
+        const int i = fx::green_comp<SIX>(r, c);
+        if (i < 0) continue;
+        const Split s = fx::split(fx::align(e[c], (int)(sh[r][c / 3] >> (8 * (c % 3)) & 255u)));
+        if (fx::green_sub(r, c)) acc.msub(g[i], s);
+        else acc.mad(g[i], s);
       }
-      put(r, acc);
-      if constexpr (SIX) {  // M' = A M - B E
-        Acc m;
-        m.mad(g[i0], e[3]);
-        m.mad(g[i1], e[4]);
-        m.mad(g[i2], e[5]);
-        if (r == 0) { m.msub(g[6], e[1]); m.msub(g[7], e[2]); }
-        if (r == 1) { m.msub(g[8], e[2]); m.mad(g[6], e[0]); }
-        if (r == 2) { m.mad(g[7], e[0]); m.mad(g[8], e[1]); }
-        put(3 + r, m);
-      }
+      const Val v = acc.get();
+      used[r] |= fx::bits_of(v);
+      s0[r * LW + a] = v;
     }
   }
-  used = (int)__reduce_or_sync(0xffffffffu, (unsigned)used);
   __syncwarp();
-  // bring the largest part (below 2^bits; 2^32 where no high word is in use) to the inverse transform's headroom
-  const int bits = 64 - __clz(used);
-  const int sh[1] = {bits - (fx::kTopBit - 1 - p.headroom(true, clog2(Pz)))};
-  int ou[1] = {0};
+  // bring each row's largest part (below 2^bits; 2^32 where no high word is in use) to the inverse transform's headroom
+  int ish[fc], ou[fc] = {};
+#pragma unroll
+  for (int r = 0; r < fc; ++r)
+    ish[r] = 64 - __clz(__reduce_or_sync(0xffffffffu, (unsigned)used[r])) - (fx::kTopBit - 1 - p.headroom(true, clog2(Pz)));
+#pragma unroll
   for (int h = 0; h < halves; ++h)
-    fx::inverse<3, fx::kShift, true>(s0 + 3 * h * LW, p, tw, lane, 32, nz, {sh, nullptr, 0}, ou);
-  const int s = fx::store_shift((int)__reduce_or_sync(0xffffffffu, (unsigned)ou[0]));
-  if (lane == 0) *eo = emax + 1 + fsh[0] + 2 * p.D + ge + sh[0] - s;
+    fx::inverse<3, fx::kShift, true>(s0 + 3 * h * LW, p, tw, lane, 32, nz, {ish + 3 * h, nullptr, 0}, ou + 3 * h);
+  int s[fc];
+#pragma unroll
+  for (int c = 0; c < fc; ++c) {
+    s[c] = fx::store_shift((int)__reduce_or_sync(0xffffffffu, (unsigned)ou[c]));
+    if (lane == c) eo[c * eostride] = er > fx::kZeroExp ? er + ish[c] + p.D - s[c] : fx::kZeroExp;
+  }
   for (int z = lane; z < nz; z += 32) {
     const int a = p.addr(z);
 #pragma unroll
-    for (int c = 0; c < fc; ++c) g0[c * fstride + z] = lift(s0[c * LW + a], s);
+    for (int c = 0; c < fc; ++c) g0[c * fstride + z] = lift(s0[c * LW + a], s[c]);
   }
 }
 
@@ -483,9 +513,9 @@ k_fx_strided(double2* __restrict__ data, size_t cc, fx::Plan p, const Fac* __res
   for (int i = row; i < p.N; i += kFxRows, out += kFxRows * cc) *out = fx::to_bits(lb[p.addr(i)], e, e == fx::kBadExp);
 }
 
-// g[comp][qx][qy][qz] * scale -> out[qx][qy][comp][qz] as Q62 over the line's
-// power of two 2^gexp >= the largest modulus sum of a row of the block: one
-// warp per (qx, qy) line.
+// g[comp][qx][qy][qz] * scale -> out[qx][qy][comp][qz] as Q62 over a power of
+// two 2^gexp of the line and component that leaves its moduli kGreenBits below
+// 1: one warp per (qx, qy) line.
 template <int NC>
 __global__ void __launch_bounds__(256)
 k_fx_pack(const double2* __restrict__ g, Fac* __restrict__ out, int* __restrict__ gexp, size_t nline, int Pz, double scale) {
@@ -493,40 +523,33 @@ k_fx_pack(const double2* __restrict__ g, Fac* __restrict__ out, int* __restrict_
   if (line >= nline) return;
   const int lane = threadIdx.x & 31;
   const size_t ng = nline * Pz;
-  const double2* gl = g + line * Pz;
-  double m = 0.0;
-  bool bad = false;
-  for (int q = lane; q < Pz; q += 32) {
-    double a[NC];
-#pragma unroll
-    for (int c = 0; c < NC; ++c) {
-      const double2 v = gl[(size_t)c * ng + q];
-      a[c] = fabs(v.x) + fabs(v.y);
+  for (int c = 0; c < NC; ++c) {
+    const double2* gl = g + (size_t)c * ng + line * Pz;
+    double m = 0.0;
+    bool bad = false;
+    for (int q = lane; q < Pz; q += 32) {
+      const double2 v = gl[q];
+      const double a = fabs(v.x) + fabs(v.y);
+      bad = bad || !isfinite(a);
+      m = fmax(m, a * scale);
     }
-    double r0 = a[0] + a[1] + a[2], r1 = a[1] + a[3] + a[4], r2 = a[2] + a[4] + a[5];
-    if constexpr (NC == 9) { r0 += a[6] + a[7]; r1 += a[6] + a[8]; r2 += a[7] + a[8]; }
-    const double r = fmax(r0, fmax(r1, r2)) * scale;
-    bad = bad || !isfinite(r0 + r1 + r2);
-    m = fmax(m, r);
-  }
-  int e = 0;
-  frexp(m, &e);  // m < 2^e
-  e = m > 0.0 ? max(e, -960) : 0;
-  e = (int)__reduce_max_sync(0xffffffffu, m > 0.0 ? e : INT32_MIN);
-  if (e == INT32_MIN) e = 0;
-  bad = __any_sync(0xffffffffu, bad);
-  if (lane == 0) gexp[line] = bad ? fx::kBadExp : e;
-  const double mul = bad ? 0.0 : ldexp(scale, 62 - e);
-  for (int q = lane; q < Pz; q += 32)
-#pragma unroll
-    for (int c = 0; c < NC; ++c) {
-      const double2 v = gl[(size_t)c * ng + q];
+    int e = 0;
+    frexp(m, &e);  // m < 2^e
+    e = __reduce_max_sync(0xffffffffu, m > 0.0 ? max(e, -950) : INT32_MIN);
+    bad = __any_sync(0xffffffffu, bad);
+    const bool zero = e == INT32_MIN;
+    e += fx::kGreenBits<NC == 9>;
+    if (lane == 0) gexp[line * NC + c] = bad ? fx::kBadExp : zero ? fx::kZeroExp : e;
+    const double mul = bad || zero ? 0.0 : ldexp(scale, 62 - e);
+    for (int q = lane; q < Pz; q += 32) {
+      const double2 v = gl[q];
       const long long re = __double2ll_rn(v.x * mul), im = __double2ll_rn(v.y * mul);
       Fac w;
       fx::split(re, w.rh, w.rl);
       fx::split(im, w.ih, w.il);
       out[(line * NC + c) * Pz + q] = w;
     }
+  }
 }
 
 // Shared memory of a strided pass: lines, shifts, ints (exponents, occupancy).
@@ -599,7 +622,7 @@ cudaError_t launch(const MvpGeom& g, const FxTables& t, const void* xv, int ldx,
   end(kPassA64);
   begin(kPassB64);
   auto* kb = fits(kXMany, bsm) ? k_fx_y<false, kXMany> : k_fx_y<false, kXFew>;
-  launch_pdl(kb, ygrid, kFxThreads, bsm, st, t1, t2, g.tmask, g.f, g.Px, g.ny, g.nz, g.nzp, g.nzt, py,
+  launch_pdl(kb, ygrid, kFxThreads, bsm, st, t1, t2, g.tmask, g.Px, g.ny, g.nz, g.nzp, g.nzt, py,
                                                                     t.tw[1], w.ea, w.eb, done);
   end(kPassB64);
   begin(kPassC64);
@@ -614,7 +637,7 @@ cudaError_t launch(const MvpGeom& g, const FxTables& t, const void* xv, int ldx,
   end(kPassC64);
   begin(kPassD64);
   auto* kd = fits(kXMany, dsm) ? k_fx_y<true, kXMany> : k_fx_y<true, kXFew>;
-  launch_pdl(kd, ygrid, kFxThreads, dsm, st, t2, t1, g.tmask, g.f, g.Px, g.ny, g.nz, g.nzp, g.nzt, py, t.tw[1],
+  launch_pdl(kd, ygrid, kFxThreads, dsm, st, t2, t1, g.tmask, g.Px, g.ny, g.nz, g.nzp, g.nzt, py, t.tw[1],
                                                              w.ec, w.eb, done);
   end(kPassD64);
   begin(kPassE64);

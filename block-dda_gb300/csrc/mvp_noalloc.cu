@@ -34,9 +34,10 @@ namespace {
 constexpr size_t kNoAllocScratchBytes = 64ull << 20;  // 64 MiB per device
 constexpr int kMaxDevices = 64;
 
-// Line exponents of the FP64 workspace (FxWork), behind the two workspace buffers.  At 16 bytes an element they are at most
-// 1/8 of T1 (Px >= 2) and of T2 (Py >= 2) and, per right-hand side, 1/48 of T2 (f >= 3, nzp >= 4).
-constexpr size_t kNoAllocExpBytes = kNoAllocScratchBytes / 8 + kNoAllocScratchBytes / 48 + 256;
+// Line exponents of the FP64 workspace (FxWork), behind the two workspace buffers: 4 bytes each against 16 per element, so
+// ((ny + Px) nzp + Px Py) / (4 Px nzp (ny + Py)) of T1 and T2 together.  That is 1/6 for a box of one site (ny = 1,
+// Px = Py = 2, nzp = 4) and falls with every side.
+constexpr size_t kNoAllocExpBytes = kNoAllocScratchBytes / 6 + 256;
 __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratchBytes + kNoAllocExpBytes];
 
 std::mutex g_scratch_mu;

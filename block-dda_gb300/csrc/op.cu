@@ -346,7 +346,7 @@ static int build_spectrum(Op* op, double k_re, double k_im) {
   BDDA_CUDA(work.ensure(nc * ng * sizeof(double2), op->stream));
   if (prec & (BDDA_PREC_FP64 | BDDA_PREC_DF64)) {
     BDDA_CUDA(op->ghatfx.ensure(nc * ng * sizeof(fx::Fac), op->stream));
-    BDDA_CUDA(op->gexpfx.ensure((size_t)Px * Py * sizeof(int), op->stream));
+    BDDA_CUDA(op->gexpfx.ensure(nc * Px * Py * sizeof(int), op->stream));
   }
   if (prec & BDDA_PREC_FP32) BDDA_CUDA(op->ghat32.ensure(nc * ng * sizeof(float2), op->stream));
   // one transform, packed for each precision in the order of its plans

@@ -43,3 +43,25 @@ def test_products_at_the_ends_of_the_low_half(fx, low, sub):
                 im += sg * (a * d + b * c)
             assert abs(int(out[0]) * 2 ** 62 - re) <= 5 * 2 ** 62
             assert abs(int(out[1]) * 2 ** 62 - im) <= 5 * 2 ** 62
+
+
+# The largest terms of a row: 3 with |re| + |im| <= 2^61 and |z| <= 2^61, or 5 with 2^59 and 2^60; no sum may wrap.
+@pytest.mark.parametrize("terms, gbits, zbits", [(3, 61, 61), (5, 59, 60)])
+def test_largest_rows_do_not_wrap(fx, terms, gbits, zbits):
+    rng = np.random.default_rng(terms)
+    for _ in range(400):
+        g, z, s = [], [], []
+        for _ in range(terms):
+            a = int(rng.integers(0, 2 ** gbits)) if rng.random() < 0.5 else int(rng.choice([0, 2 ** gbits - 1, 2 ** (gbits - 1)]))
+            g += [a, 2 ** gbits - 1 - a]
+            z += [int(2 ** zbits * 0.7071)] * 2 if rng.random() < 0.7 else [2 ** zbits - 1, 0]
+            s.append(int(rng.integers(0, 2)))
+        for v in (g, z):      # low halves at both ends, signs at random
+            for i in range(len(v)):
+                v[i] = ((v[i] >> 32 << 32) | int(rng.choice([0x7FFFFFFF, 0x80000001, v[i] & 0xFFFFFFFF]))) * int(rng.choice([-1, 1]))
+        out = np.zeros(2, np.int64)
+        fx.fx_products(terms, _ll(g), _ll(z), np.array(s, np.int32).ctypes.data_as(ct.POINTER(ct.c_int)), _ll(out))
+        re = sum((-1 if s[i] else 1) * (g[2 * i] * z[2 * i] - g[2 * i + 1] * z[2 * i + 1]) for i in range(terms))
+        im = sum((-1 if s[i] else 1) * (g[2 * i] * z[2 * i + 1] + g[2 * i + 1] * z[2 * i]) for i in range(terms))
+        assert abs(int(out[0]) * 2 ** 62 - re) <= (2 * terms + 1) * 2 ** 62
+        assert abs(int(out[1]) * 2 ** 62 - im) <= (2 * terms + 1) * 2 ** 62
