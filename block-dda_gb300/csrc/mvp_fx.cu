@@ -87,7 +87,8 @@ struct IoDf {
 };
 
 // Scale of this warp's line (FP64 bits at line[addr(i)], i < n, element i written by lane i % 32): its largest value and
-// the sum of its parts bound every value of its transform.
+// the sum of its parts bound every value of its transform.  A line of tiny values is rewritten, each element by its lane: a
+// __syncwarp() comes before others read it.
 __device__ __forceinline__ fx::Scale line_scale(Val* line, const fx::Plan& p, int lane, int n) {
   auto largest = [&] {
     int k = 0;
@@ -475,6 +476,7 @@ k_fx_contig(double2* __restrict__ data, size_t nlines, fx::Plan p, const Fac* __
     rsh[j] = s.rsh0;
     eb[j] = s.bad ? fx::kBadExp : s.ebase + p.D;
   }
+  __syncwarp();  // line_scale may have rewritten the lines
   fx::forward<kFxLines, fx::kRaw, false, false>(wl, p, tw, lane, 32, p.N, {rsh, nullptr, 0}, nullptr);
 #pragma unroll
   for (int j = 0; j < kFxLines; ++j) {
@@ -504,6 +506,7 @@ k_fx_strided(double2* __restrict__ data, size_t cc, fx::Plan p, const Fac* __res
     rsh[j] = s.rsh0;
     if (lane == 0) eb[kFxLines * warp + j] = s.bad ? fx::kBadExp : s.ebase + p.D;
   }
+  __syncwarp();  // line_scale may have rewritten the lines
   fx::forward<kFxLines, fx::kRaw, false, false>(wl, p, tw, lane, 32, p.N, {rsh, nullptr, 0}, nullptr);
   __syncthreads();
   if (!ok) return;
