@@ -466,7 +466,8 @@ BDDA_FX_FN Val to_bits(Val v, int eb, bool bad) {
 // own: parts below 2^kStoreBit, the largest in [2^(kStoreBit - 1), 2^kStoreBit)
 // (or, below 2^32, shifted up as far as that takes it), value = v 2^e.
 constexpr int kStoreBit = 62;
-constexpr int kBadExp = INT32_MAX;        // a line that is not finite
+// Both marks are exponents like any other to the shifts of an element against its line's largest, which stay in range.
+constexpr int kBadExp = 1 << 24;          // a line that is not finite
 constexpr int kZeroExp = -(1 << 20);      // a line of zeros
 // OR of the folded high words of values: the bits in use.
 BDDA_FX_FN int bits_of(Val v) {

@@ -49,7 +49,6 @@ constexpr int kFxWarps = 4;                    // warps of a strided pass's CTA
 constexpr int kFxThreads = kFxWarps * 32;
 constexpr int kFxLines = kTZ / kFxWarps;       // lines per warp
 constexpr int kFxRows = kFxThreads / kTZ;      // rows a tile copy moves at once
-constexpr int kBadAlign = 1 << 24;             // stands in for the exponent of a line that is not finite
 
 // CTAs per SM the kernels are compiled for: registers against resident warps.
 // Measured at one CTA fewer / more: y passes N=16384, L=16 (Py=160) 1.97 /
@@ -144,11 +143,10 @@ __device__ __forceinline__ void line_aligns(const Val* wl, const fx::Plan& p, co
     }
     e = __reduce_max_sync(0xffffffffu, e);
     cnt = (int)__reduce_add_sync(0xffffffffu, (unsigned)cnt);
-    const int el = e == fx::kBadExp ? kBadAlign : e;
     int used = 0;
-    for (int i = lane; i < n; i += 32) used |= fx::bits_of(wl[j * p.LW + p.addr(i)]) >> min(el - ex[j * exs + i], 31);
+    for (int i = lane; i < n; i += 32) used |= fx::bits_of(wl[j * p.LW + p.addr(i)]) >> min(e - ex[j * exs + i], 31);
     const int s = fx::fit_shift((int)__reduce_or_sync(0xffffffffu, (unsigned)used), p.headroom(inv, clog2(cnt)));
-    rsh[j] = el + s;
+    rsh[j] = e + s;
     eo[j] = e == fx::kBadExp || e == fx::kZeroExp ? e : e + s + p.D;
   }
 }

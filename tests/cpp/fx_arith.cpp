@@ -24,4 +24,10 @@ void fx_products(int n, const long long* g, const long long* z, const int* sub, 
   out[1] = v.y;
 }
 
+// Exponents that mark a line of zeros and one that is not finite.
+int fx_zero_exp() { return fx::kZeroExp; }
+int fx_bad_exp() { return fx::kBadExp; }
+// v / 2^r, rounded
+long long fx_align(long long v, int r) { return fx::align(fx::Val{v, 0}, r).x; }
+
 }  // extern "C"

@@ -65,3 +65,19 @@ def test_largest_rows_do_not_wrap(fx, terms, gbits, zbits):
         im = sum((-1 if s[i] else 1) * (g[2 * i] * z[2 * i + 1] + g[2 * i + 1] * z[2 * i]) for i in range(terms))
         assert abs(int(out[0]) * 2 ** 62 - re) <= (2 * terms + 1) * 2 ** 62
         assert abs(int(out[1]) * 2 ** 62 - im) <= (2 * terms + 1) * 2 ** 62
+
+
+# Elements are shifted right by e + s - ex: e the largest exponent of their line, ex their own, s from 1 to 64.
+def test_shifts_of_marked_lines_stay_in_range(fx):
+    fx.fx_align.restype = ct.c_longlong
+    zero, bad = fx.fx_zero_exp(), fx.fx_bad_exp()
+    for exps in ([bad, zero, 900, -1100], [bad, bad], [zero, 900], [-1100, zero], [bad, -1100]):
+        e = max(exps)
+        for ex in exps:
+            assert e - ex >= 0 and -2 ** 31 <= e - ex
+            for s in (1, 64):
+                assert 1 <= e + s - ex < 2 ** 31 and e + s < 2 ** 31
+                r = e + s - ex
+                v = 2 ** 61 - 12345
+                assert fx.fx_align(ct.c_longlong(v), r) == (v + 2 ** (min(r, 62) - 1)) >> min(r, 62)
+    assert zero < -5000 and bad > 5000            # beyond every exponent of a value
