@@ -536,15 +536,19 @@ k_fx_pack(const double2* __restrict__ g, Fac* __restrict__ out, int* __restrict_
     }
     int e = 0;
     frexp(m, &e);  // m < 2^e
-    e = __reduce_max_sync(0xffffffffu, m > 0.0 ? max(e, -950) : INT32_MIN);
+    e = __reduce_max_sync(0xffffffffu, m > 0.0 ? e : INT32_MIN);
     bad = __any_sync(0xffffffffu, bad);
     const bool zero = e == INT32_MIN;
     e += fx::kGreenBits<NC == 9>;
     if (lane == 0) gexp[line * NC + c] = bad ? fx::kBadExp : zero ? fx::kZeroExp : e;
-    const double mul = bad || zero ? 0.0 : ldexp(scale, 62 - e);
+    const double mul = bad || zero ? 0.0 : ldexp(scale, min(62 - e, 1000));
+    const bool tiny = !zero && 62 - e > 1000;  // the rest of a factor beyond FP64's range
+    const double more = tiny ? ldexp(1.0, 62 - e - 1000) : 1.0;
     for (int q = lane; q < Pz; q += 32) {
       const double2 v = gl[q];
-      const long long re = __double2ll_rn(v.x * mul), im = __double2ll_rn(v.y * mul);
+      double x = v.x * mul, y = v.y * mul;
+      if (tiny) { x *= more; y *= more; }
+      const long long re = __double2ll_rn(x), im = __double2ll_rn(y);
       Fac w;
       fx::split(re, w.rh, w.rl);
       fx::split(im, w.ih, w.il);

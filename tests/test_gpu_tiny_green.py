@@ -1,5 +1,6 @@
 """Green tensors below 2^-923 (strong absorption between neighbouring sites):
-the spectrum's transforms scale such lines up before they convert them."""
+the spectrum's transforms scale such lines up before they convert them, and it
+is packed with all its bits."""
 import numpy as np
 import pytest
 
@@ -11,7 +12,7 @@ pytestmark = pytest.mark.gpu
 
 
 # exp(-k_im lf) = 2^-bits at one site's distance, and G is |k|^2 / lf = 2^25 times that
-@pytest.mark.parametrize("bits", [958])
+@pytest.mark.parametrize("bits", [958, 985, 1010])
 @pytest.mark.parametrize("n", [(5, 6, 7), (33, 20, 40), (2, 65, 64)])
 def test_strong_absorption(n, bits):
     lf = 0.25
