@@ -60,19 +60,21 @@ int smooth235(int v) {
 
 // Device bytes of one request of f components per dipole: Green spectra (6
 // or 9 components; FP64 or FP32 + double-float), the initialisation's FP64
-// work grid, occupancy, MVP workspace of both precisions, Krylov blocks.
+// work grid, occupancy, MVP workspace of both precisions (with the fixed-point
+// one's exponents), Krylov blocks.
 double footprint_bytes(const int n[3], int nocc, int L, int precision, int f) {
   const double Px = smooth235(2 * n[0]), Py = smooth235(2 * n[1]), Pz = smooth235(2 * n[2]);
   const double Ng = Px * Py * Pz;
   const double nc = (double)n[0] * n[1] * n[2];
   const bool mixed = precision == BDDA_SOLVE_MIXED;
   const double ncomp = f == 6 ? 9.0 : 6.0;
-  const double tables = ncomp * Ng * (16.0 + (mixed ? 8.0 : 0.0));
+  const double tables = ncomp * (Ng * (16.0 + (mixed ? 8.0 : 0.0)) + Px * Py * 4.0);
   const double init_work = ncomp * Ng * 16.0;
   const double occ = nc * 4.0 + (double)n[1] * ((n[2] + 7) / 8) * 5.0;
   const double nzp = (double)((n[2] + 3) & ~3);
   const double t1 = (double)f * L * Px * n[1] * nzp, t2 = (double)f * L * Px * Py * nzp;
-  const double mvp = (t1 + t2) * (16.0 + (mixed ? 8.0 : 0.0));
+  const double exps = (double)f * L * ((n[1] + Px) * nzp + Px * Py);
+  const double mvp = (t1 + t2) * (16.0 + (mixed ? 8.0 : 0.0)) + exps * 4.0;
   const double nu = (double)f * nocc, LL = (double)L * L;
   const double blocks = 10.0 * nu * L * (mixed ? 8.0 : 16.0) + 3.0 * nu * L * 16.0 + nu * 32.0;
   const double small = 2.0 * LL * 152.0 * 16.0 + 2.0 * std::max(608.0 * L, 1216.0) * 16.0 + LL * 16.0 * 20.0 + 8.0 * 4096;

@@ -23,6 +23,18 @@ def test_footprint_grows_with_box_and_nrhs():
     assert bdda.footprint((40, 40, 40), 500, 16, bdda.SOLVE_FP64) != c
 
 
+# flat boxes, whose line exponents are the largest share of the workspace (up to a sixth)
+@pytest.mark.parametrize("n, P", [((600, 1, 600), (1200, 2, 1200)), ((1, 600, 600), (2, 1200, 1200)), ((600, 600, 1), (1200, 1200, 2)),
+                                  ((1, 1, 600), (2, 2, 1200))])
+@pytest.mark.parametrize("precision, size", [(bdda.SOLVE_FP64, 16), (bdda.SOLVE_MIXED, 24)])
+def test_footprint_holds_tables_workspace_and_exponents(n, P, precision, size):
+    L, nzp = 32, (n[2] + 3) // 4 * 4
+    fields = 3 * L * P[0] * nzp
+    tables = 6 * (P[0] * P[1] * P[2] * size + P[0] * P[1] * 4)
+    mvp = fields * (n[1] + P[1]) * size + 3 * L * ((n[1] + P[0]) * nzp + P[0] * P[1]) * 4
+    assert bdda.footprint(n, 1, L, precision) > 1.04 * (tables + mvp)     # next to nothing for one dipole's vectors
+
+
 def test_dry_run_respects_budget_and_completes_everything():
     probs = _probs([64, 300, 1000, 2500, 90, 700, 4000, 150, 2000, 80, 512, 3000], seed=1)
     fps = [bdda.footprint(p.n, p.nocc, p.B.shape[1]) for p in probs]
