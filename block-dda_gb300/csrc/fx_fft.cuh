@@ -130,16 +130,15 @@ struct Acc {
     ci -= (mw(s.xh, g.il) + mw(s.xl, g.ih)) + (mw(s.yh, g.rl) + mw(s.yl, g.rh));
     mi -= mw(s.xh, g.ih) + mw(s.yh, g.rh);
   }
+  BDDA_FX_FN void add(const Acc& o) { cr += o.cr; ci += o.ci; mr += o.mr; mi += o.mi; }
+  BDDA_FX_FN void sub(const Acc& o) { cr -= o.cr; ci -= o.ci; mr -= o.mr; mi -= o.mi; }
   BDDA_FX_FN Val get() const { return {shl(mr, 2) + (cr >> 30), shl(mi, 2) + (ci >> 30)}; }
 };
 
-// Spectrum component that couples component c to row r of the block: symmetric A (xx xy xz yy yz zz), and with SIX
-// [A B; -B A], B antisymmetric (xy xz yz): index, -1 for none, and whether its product is subtracted.
-template <bool SIX> BDDA_FX_FN constexpr int green_comp(int r, int c) {
-  const int a = r % 3, b = c % 3;
-  return (r < 3) == (c < 3) ? a + b + (a != 0 && b != 0 ? 1 : 0) : a == b ? -1 : 5 + a + b;
-}
-BDDA_FX_FN constexpr bool green_sub(int r, int c) { return (r < 3) != (c < 3) && (r < 3) == (r % 3 > c % 3); }
+// Index of the spectrum components that couple component c to row r, r and c < 3: of the symmetric block A (xx xy xz yy yz
+// zz), and with f = 6, [A B; -B A], of the antisymmetric B (xy xz yz, -1 on its diagonal; subtracted where r > c).
+BDDA_FX_FN constexpr int green_a(int r, int c) { return r + c + (r != 0 && c != 0 ? 1 : 0); }
+BDDA_FX_FN constexpr int green_b(int r, int c) { return r == c ? -1 : 5 + r + c; }
 // Bits that a spectrum component stays below 1, and that values are shifted for the products at least: with the 3 (SIX: 5)
 // terms of a row the middle sums of Acc stay below 7.3 (4.8) 2^60 and its result below 2^62.  SIX could do with 2 bits of
 // the first; the exponents, and so the roundings, of the recorded f = 6 runs depend on it, whose loosely converged BiCGSTAB

@@ -316,9 +316,12 @@ k_fx_e(const Val* __restrict__ t1, const int* __restrict__ ein, int nfield, int 
 }
 
 // ---------------------------------------------------------------- pass C
+// v[3 h + c]
+template <int N> __device__ __forceinline__ int half(const int (&v)[N], int h, int c) { return N == 6 && h ? v[N - 3 + c] : v[c]; }
+
 // One warp per (x = q, y = qy, rhs l): fc component lines, blockDim.x / 32 warps per CTA.  Bound by the integer multiplier
 // and the instructions around it.  An exponent per component costs the alignment of nine (f = 6: 30) factors per
-// frequency: 1.84 -> 2.00 ms at Pz=120 (N=8192, L=16), 3.90 -> 4.20 at 150, f = 6 0.151 -> 0.172 at 54 (N=1200, L=4),
+// frequency: 1.84 -> 2.00 ms at Pz=120 (N=8192, L=16), 3.90 -> 4.20 at 150, f = 6 0.151 -> 0.175 at 54 (N=1200, L=4),
 // against one for all of them, whose small components lost the bits between.  One shift for the rows of lines whose
 // spectrum components are close was no faster (4.2 ms): the second product loop cost what it saved.
 template <bool SIX, int MB>
@@ -379,31 +382,37 @@ k_fx_c(Val* __restrict__ t2, int L, int Px, int Py, int nz, int nzp, fx::Plan p,
   }
   __syncwarp();
   constexpr int halves = SIX ? 2 : 1;
-#pragma unroll
-  for (int h = 0; h < halves; ++h)
-    fx::forward<3, fx::kShift, true, false>(s0 + 3 * h * LW, p, tw, lane, 32, nz, {fsh + 3 * h, nullptr, 0}, nullptr);
-  // lane r: exponent of row r's products, from its largest term (exponents of its spectrum components and values)
-  int er = fx::kZeroExp;
-#pragma unroll
-  for (int c = 0; c < fc; ++c) {
-    const int i = fx::green_comp<SIX>(lane < fc ? lane : 0, c);
-    const int v = __shfl_sync(0xffffffffu, ev, c), g = __shfl_sync(0xffffffffu, ge, i < 0 ? 0 : i);
-    if (lane < fc && i >= 0 && v > fx::kZeroExp && g > fx::kZeroExp) er = max(er, v + g + fx::kProductBits<SIX>);
+  // one copy of a transform's code for both halves: small launches wait for their instructions
+#pragma unroll 1
+  for (int h = 0; h < halves; ++h) {
+    const int rsh[3] = {half(fsh, h, 0), half(fsh, h, 1), half(fsh, h, 2)};
+    fx::forward<3, fx::kShift, true, false>(s0 + 3 * h * LW, p, tw, lane, 32, nz, {rsh, nullptr, 0}, nullptr);
   }
-  unsigned sh[fc][halves];  // shift of component c for row r: byte c % 3 of sh[r][c / 3]
+  // Lane 3 r + c: the terms of row r with component c of its own block of rows and, f = 6, of the other one.  All lanes of a
+  // row: the exponent of its products, from its largest term (exponents of spectrum component and value).  Lane 3 r: the
+  // shifts of its terms' values, byte c (a zero component's does not matter).
+  const int tr = lane < 3 * fc ? lane / 3 : 0, tc = lane % 3, ta = tr % 3;
+  auto term = [&](int c, int i) {
+    const int v = __shfl_sync(0xffffffffu, ev, c), g = __shfl_sync(0xffffffffu, ge, i < 0 ? 0 : i);
+    return i >= 0 && v > fx::kZeroExp && g > fx::kZeroExp ? v + g : fx::kZeroExp;
+  };
+  const int own = term(tr - ta + tc, fx::green_a(ta, tc));
+  const int oth = SIX ? term((tr < 3 ? 3 : 0) + tc, fx::green_b(ta, tc)) : fx::kZeroExp;
+  int er = max(own, oth);
+  er = max(er, max(__shfl_down_sync(0xffffffffu, er, 1), __shfl_down_sync(0xffffffffu, er, 2)));
+  er = __shfl_sync(0xffffffffu, er, lane - tc);
+  if (er > fx::kZeroExp) er += fx::kProductBits<SIX>;
+  auto shifts = [&](int e) {
+    const unsigned s = (unsigned)min(max(er - e, 1), 62) << (8 * tc);
+    return s | __shfl_down_sync(0xffffffffu, s, 1) | __shfl_down_sync(0xffffffffu, s, 2);
+  };
+  const unsigned so = shifts(own), st = SIX ? shifts(oth) : 0;
+  unsigned sown[fc], soth[fc];
 #pragma unroll
-  for (int r = 0; r < fc; ++r)
-#pragma unroll
-    for (int h = 0; h < halves; ++h) {
-      sh[r][h] = 0;
-#pragma unroll
-      for (int b = 0; b < 3; ++b) {
-        const int c = 3 * h + b, i = fx::green_comp<SIX>(r, c);
-        if (i < 0) continue;
-        const int d = __shfl_sync(0xffffffffu, er, r) - __shfl_sync(0xffffffffu, ev, c) - __shfl_sync(0xffffffffu, ge, i);
-        sh[r][h] |= (unsigned)min(max(d, 1), 62) << (8 * b);  // a zero component's shift does not matter
-      }
-    }
+  for (int r = 0; r < fc; ++r) {
+    sown[r] = __shfl_sync(0xffffffffu, so, 3 * r);
+    soth[r] = SIX ? __shfl_sync(0xffffffffu, st, 3 * r) : 0;
+  }
   const Fac* gl = ghat + (size_t)line * nc * Pz;
   int used[fc] = {};
   for (int f = lane; f < Pz; f += 32) {
@@ -411,39 +420,67 @@ k_fx_c(Val* __restrict__ t2, int L, int Px, int Py, int nz, int nzp, fx::Plan p,
     Fac g[nc];
 #pragma unroll
     for (int c = 0; c < nc; ++c) g[c] = fx::ldfac(gl + (size_t)c * Pz + f);
-    Val e[fc];
+    Val e[3], w[3];
 #pragma unroll
-    for (int c = 0; c < fc; ++c) e[c] = s0[c * LW + a];
+    for (int c = 0; c < 3; ++c) {
+      e[c] = s0[c * LW + a];
+      w[c] = SIX ? s0[(3 + c) * LW + a] : Val{0, 0};
+    }
+    // one copy of a block row's code: unrolled, an MVP of N=99, f = 6, L=1 took 40.0 us, with the loops 38.6
+#pragma unroll 1
+    for (int h = 0; h < halves; ++h) {
 #pragma unroll
-    for (int r = 0; r < fc; ++r) {
-      Acc acc;
+      for (int r = 0; r < 3; ++r) {
+        Acc acc;
+        const unsigned q = SIX && h ? sown[fc - 3 + r] : sown[r];
 #pragma unroll
-      for (int c = 0; c < fc; ++c) {
-        const int i = fx::green_comp<SIX>(r, c);
-        if (i < 0) continue;
-        const Split s = fx::split(fx::align(e[c], (int)(sh[r][c / 3] >> (8 * (c % 3)) & 255u)));
-        if (fx::green_sub(r, c)) acc.msub(g[i], s);
-        else acc.mad(g[i], s);
+        for (int c = 0; c < 3; ++c) acc.mad(g[fx::green_a(r, c)], fx::split(fx::align(e[c], (int)(q >> (8 * c) & 255u))));
+        if constexpr (SIX) {  // E' = A E + B M, M' = A M - B E
+          Acc t{0, 0, 0, 0};
+          const unsigned u = h ? soth[fc - 3 + r] : soth[r];
+#pragma unroll
+          for (int c = 0; c < 3; ++c) {
+            const int i = fx::green_b(r, c);
+            if (i < 0) continue;
+            const Split s = fx::split(fx::align(w[c], (int)(u >> (8 * c) & 255u)));
+            if (r > c) t.msub(g[i], s);
+            else t.mad(g[i], s);
+          }
+          if (h) acc.sub(t);
+          else acc.add(t);
+        }
+        const Val v = acc.get();
+        const int b = fx::bits_of(v);
+        used[r] |= SIX && h ? 0 : b;
+        if constexpr (SIX) used[3 + r] |= h ? b : 0;
+        s0[(3 * h + r) * LW + a] = v;
       }
-      const Val v = acc.get();
-      used[r] |= fx::bits_of(v);
-      s0[r * LW + a] = v;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        const Val t = e[c];
+        e[c] = w[c];
+        w[c] = t;
+      }
     }
   }
   __syncwarp();
   // bring each row's largest part (below 2^bits; 2^32 where no high word is in use) to the inverse transform's headroom
-  int ish[fc], ou[fc] = {};
+  int ish[fc], s[fc] = {};
 #pragma unroll
   for (int r = 0; r < fc; ++r)
     ish[r] = 64 - __clz(__reduce_or_sync(0xffffffffu, (unsigned)used[r])) - (fx::kTopBit - 1 - p.headroom(true, clog2(Pz)));
+#pragma unroll 1
+  for (int h = 0; h < halves; ++h) {
+    const int rsh[3] = {half(ish, h, 0), half(ish, h, 1), half(ish, h, 2)};
+    int ou[3] = {};
+    fx::inverse<3, fx::kShift, true>(s0 + 3 * h * LW, p, tw, lane, 32, nz, {rsh, nullptr, 0}, ou);
 #pragma unroll
-  for (int h = 0; h < halves; ++h)
-    fx::inverse<3, fx::kShift, true>(s0 + 3 * h * LW, p, tw, lane, 32, nz, {ish + 3 * h, nullptr, 0}, ou + 3 * h);
-  int s[fc];
+    for (int c = 0; c < 3; ++c) {
+      const int t = fx::store_shift((int)__reduce_or_sync(0xffffffffu, (unsigned)ou[c]));
+      if (lane == 3 * (3 * h + c)) eo[(3 * h + c) * eostride] = er > fx::kZeroExp ? er + rsh[c] + p.D - t : fx::kZeroExp;
 #pragma unroll
-  for (int c = 0; c < fc; ++c) {
-    s[c] = fx::store_shift((int)__reduce_or_sync(0xffffffffu, (unsigned)ou[c]));
-    if (lane == c) eo[c * eostride] = er > fx::kZeroExp ? er + ish[c] + p.D - s[c] : fx::kZeroExp;
+      for (int k = c; k < fc; k += 3) s[k] = k == 3 * h + c ? t : s[k];
+    }
   }
   for (int z = lane; z < nz; z += 32) {
     const int a = p.addr(z);
@@ -524,30 +561,44 @@ k_fx_pack(const double2* __restrict__ g, Fac* __restrict__ out, int* __restrict_
   if (line >= nline) return;
   const int lane = threadIdx.x & 31;
   const size_t ng = nline * Pz;
-  for (int c = 0; c < NC; ++c) {
-    const double2* gl = g + (size_t)c * ng + line * Pz;
-    double m = 0.0;
-    bool bad = false;
-    for (int q = lane; q < Pz; q += 32) {
-      const double2 v = gl[q];
+  const double2* gl = g + line * Pz;
+  double m[NC] = {};  // largest modulus sum of a component
+  bool bad = false;
+  for (int q = lane; q < Pz; q += 32)
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      const double2 v = gl[(size_t)c * ng + q];
       const double a = fabs(v.x) + fabs(v.y);
       bad = bad || !isfinite(a);
-      m = fmax(m, a * scale);
+      m[c] = fmax(m[c], a);
     }
-    int e = 0;
-    frexp(m, &e);  // m < 2^e
-    e = __reduce_max_sync(0xffffffffu, m > 0.0 ? e : INT32_MIN);
-    bad = __any_sync(0xffffffffu, bad);
-    const bool zero = e == INT32_MIN;
+  bad = __any_sync(0xffffffffu, bad);
+  // lane c: component c's exponent, the factor to its integers and, where that is beyond FP64's range, the rest of it
+  int e = fx::kZeroExp;
+  double mul = 0.0, more = 1.0;
+#pragma unroll
+  for (int c = 0; c < NC; ++c) {
+    const unsigned h = (unsigned)__double2hiint(m[c]);
+    const unsigned top = __reduce_max_sync(0xffffffffu, h);
+    const unsigned lo = __reduce_max_sync(0xffffffffu, h == top ? (unsigned)__double2loint(m[c]) : 0u);
+    if (lane == c) m[0] = __hiloint2double((int)top, (int)lo);
+  }
+  if (lane < NC && m[0] * scale > 0.0) {
+    frexp(m[0] * scale, &e);  // below 2^e
     e += fx::kGreenBits<NC == 9>;
-    if (lane == 0) gexp[line * NC + c] = bad ? fx::kBadExp : zero ? fx::kZeroExp : e;
-    const double mul = bad || zero ? 0.0 : ldexp(scale, min(62 - e, 1000));
-    const bool tiny = !zero && 62 - e > 1000;  // the rest of a factor beyond FP64's range
-    const double more = tiny ? ldexp(1.0, 62 - e - 1000) : 1.0;
+    mul = ldexp(scale, min(62 - e, 1000));
+    more = ldexp(1.0, max(62 - e - 1000, 0));
+  }
+  if (bad) mul = 0.0;
+  if (lane < NC) gexp[line * NC + lane] = bad ? fx::kBadExp : e;
+  const bool tiny = __any_sync(0xffffffffu, more != 1.0);
+#pragma unroll
+  for (int c = 0; c < NC; ++c) {
+    const double f = __shfl_sync(0xffffffffu, mul, c), f2 = __shfl_sync(0xffffffffu, more, c);
     for (int q = lane; q < Pz; q += 32) {
-      const double2 v = gl[q];
-      double x = v.x * mul, y = v.y * mul;
-      if (tiny) { x *= more; y *= more; }
+      const double2 v = gl[(size_t)c * ng + q];
+      double x = v.x * f, y = v.y * f;
+      if (tiny) { x *= f2; y *= f2; }
       const long long re = __double2ll_rn(x), im = __double2ll_rn(y);
       Fac w;
       fx::split(re, w.rh, w.rl);
