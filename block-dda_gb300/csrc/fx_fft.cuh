@@ -153,7 +153,6 @@ constexpr long long kRt5_4 = 2578010857022246787ll;   // sqrt(5) / 4
 constexpr long long kS72 = 4385974038932618941ll, kS36 = 2710681029835013083ll;
 constexpr long long kC9[3] = {3532756447825785444ll, 800810873071977681ll, -4333567320897763126ll};  // cos 40 k, k = 1, 2, 4
 constexpr long long kS9[3] = {2964334632409774423ll, 4541624145405292212ll, 1577289512995517789ll};
-constexpr long long kC16 = 4260642322793532497ll, kS16 = 1764815834521887442ll;  // cos, sin 22.5
 
 BDDA_FX_FN Val mul_i(Val a) { return {-a.y, a.x}; }
 BDDA_FX_FN Val mul_mi(Val a) { return {a.y, -a.x}; }
@@ -234,7 +233,7 @@ template <bool INV, long long QC, long long QS> BDDA_FX_FN Val rotk(Val z) {
   // forward exp(-i a), inverse exp(+i a), a the angle with cosine QC and sine QS
   return cmul<0, !INV>(z, hi_of(QC), lo_of(QC), hi_of(QS), lo_of(QS));
 }
-// 9 = 3 x 3 and 16 = 4 x 4 with constant twiddles
+// 9 = 3 x 3 with constant twiddles
 template <bool INV> BDDA_FX_FN void dft9(Val* v) {
   Val y[3][3];
 #pragma unroll
@@ -252,30 +251,6 @@ template <bool INV> BDDA_FX_FN void dft9(Val* v) {
     Val u[3] = {y[0][k], y[1][k], y[2][k]};
     dft3<INV>(u);
     v[k] = u[0]; v[k + 3] = u[1]; v[k + 6] = u[2];
-  }
-}
-template <bool INV> BDDA_FX_FN void dft16(Val* v) {
-  Val y[4][4];
-#pragma unroll
-  for (int n = 0; n < 4; ++n) {
-    Val u[4] = {v[n], v[n + 4], v[n + 8], v[n + 12]};
-    dft4<INV>(u);
-    y[n][0] = u[0]; y[n][1] = u[1]; y[n][2] = u[2]; y[n][3] = u[3];
-  }
-  y[1][1] = rotk<INV, kC16, kS16>(y[1][1]);
-  y[1][2] = rot8<INV>(y[1][2]);
-  y[1][3] = rotk<INV, kS16, kC16>(y[1][3]);
-  y[2][1] = rot8<INV>(y[2][1]);
-  y[2][2] = INV ? mul_i(y[2][2]) : mul_mi(y[2][2]);
-  y[2][3] = rot8<INV>(INV ? mul_i(y[2][3]) : mul_mi(y[2][3]));
-  y[3][1] = rotk<INV, kS16, kC16>(y[3][1]);
-  y[3][2] = rot8<INV>(INV ? mul_i(y[3][2]) : mul_mi(y[3][2]));
-  y[3][3] = rotk<INV, -kC16, -kS16>(y[3][3]);
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    Val u[4] = {y[0][k], y[1][k], y[2][k], y[3][k]};
-    dft4<INV>(u);
-    v[k] = u[0]; v[k + 4] = u[1]; v[k + 8] = u[2]; v[k + 12] = u[3];
   }
 }
 
@@ -317,18 +292,15 @@ template <int R, bool INV> BDDA_FX_FN void dft(Val* v) {
   else if constexpr (R == 6) dft_pfa<2, 3, INV>(v);
   else if constexpr (R == 8) dft8<INV>(v);
   else if constexpr (R == 9) dft9<INV>(v);
-  else if constexpr (R == 10) dft_pfa<2, 5, INV>(v);
-  else if constexpr (R == 12) dft_pfa<4, 3, INV>(v);
-  else if constexpr (R == 15) dft_pfa<3, 5, INV>(v);
   else {
-    static_assert(R == 16, "register radix");
-    dft16<INV>(v);
+    static_assert(R == 10, "register radix");
+    dft_pfa<2, 5, INV>(v);
   }
 }
 
 // ---- plan ----------------------------------------------------------------------
 constexpr int kMaxFxStages = 8;
-constexpr BDDA_HD int flog2(int r) { return r >= 16 ? 4 : r >= 8 ? 3 : r >= 4 ? 2 : 1; }
+constexpr BDDA_HD int flog2(int r) { return r >= 8 ? 3 : r >= 4 ? 2 : 1; }
 
 BDDA_HD int div_magic(int q, int m) { return (int)((unsigned)(q * m) >> 21); }
 

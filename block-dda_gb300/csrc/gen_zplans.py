@@ -7,8 +7,9 @@
               the first inverse stage run as one step (sfft::middle3), so
               that a 2-stage plan makes two shared-memory round trips per
               line triple instead of four or more
-  zwplans.inc three-line plans of the 16-byte z passes (FP64 / double-float:
-              register radices <= 16, no fused step)
+  zwplans.inc three-line plans of 16-byte elements (register radices <= 16, no
+              fused step): the FP64 and double-float z lines of the host line
+              transform, which the fixed-point one is compared with
   tplans.inc  plans of the strided x / y passes: the radix sequences of the
               column-pair kernels (column_radices); S and LW are the layout
               for one warp per line, which those kernels do not use

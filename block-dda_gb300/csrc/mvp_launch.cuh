@@ -113,7 +113,6 @@ cudaError_t launch_block_mvp(const MvpGeom& g, const MvpPrec<T>& p, const typena
                              cudaStream_t st, KernelTimer* timer, const int* done) {
   using C = typename cplx<T>::type;
   const int nfield = g.f * L;
-  const int pbase = sizeof(T) == sizeof(double) ? (kPassA64 - kPassA) : 0;
   if (g.ntiles == 0) return cudaSuccess;  // no dipoles
   const int ntask_y = nfield * g.Px * g.nzt;
   // runtime-plan y passes: kYWaves waves of the CTAs resident per SM
@@ -124,9 +123,7 @@ cudaError_t launch_block_mvp(const MvpGeom& g, const MvpPrec<T>& p, const typena
   };
   const tile::RtLine<C> lx{g.px}, ly{g.py};
   // runtime-plan strided passes: tile buffers and shared memory -- one buffer
-  // where two would not fit (long lines of 16-byte elements).  Single
-  // buffering where two fit was measured no faster for the double-float y
-  // passes (N=65536, Py=270: 14.6 / 14.3 vs 14.3 / 14.0 ms).
+  // where two would not fit
   const int xbuf = tile::tile_buffers<T>(plan_lw<C>(g.px), g.nx), ybuf = tile::tile_buffers<T>(plan_lw<C>(g.py), 0);
   const int xsm = tile::smem_tile<T>(plan_lw<C>(g.px), g.nx, xbuf), ysm = tile::smem_tile<T>(plan_lw<C>(g.py), 0, ybuf);
   int xfpg = 0;  // x passes: fields per CTA
@@ -137,41 +134,33 @@ cudaError_t launch_block_mvp(const MvpGeom& g, const MvpPrec<T>& p, const typena
   // false when it was not launched that way.
   cudaError_t serr = cudaSuccess;
   auto static_tile = [&](int pass) -> bool {
-    if constexpr (std::is_same<T, float>::value) {
-      const TileArgs a{&g, x, ldx, y, ldy, nfield, diag, jpre, t1, t2, p.twxps, p.twyps, num_sms(), st, done};
-      cudaError_t e = cudaSuccess;
-      const bool ok = launch_tile_static(pass, a, &e);
-      if (ok && e != cudaSuccess) serr = e;
-      return ok;
-    } else {
-      (void)pass;
-      return false;
-    }
+    const TileArgs a{&g, x, ldx, y, ldy, nfield, diag, jpre, t1, t2, p.twxps, p.twyps, num_sms(), st, done};
+    cudaError_t e = cudaSuccess;
+    const bool ok = launch_tile_static(pass, a, &e);
+    if (ok && e != cudaSuccess) serr = e;
+    return ok;
   };
   // A
-  if (runA && timer) timer->begin(kPassA + pbase, st);
+  if (runA && timer) timer->begin(kPassA, st);
   if (runA && !static_tile(kTileA))
     tile::k_pass_a<T><<<xgrid, kTileThreads, xsm, st>>>(
         x, ldx, nfield, xfpg, g.f, g.occ, g.tiles, g.nx, g.ny, g.nz, g.nzp, g.nzt, lx, p.twx, t1, xbuf, done);
-  if (runA && timer) timer->end(kPassA + pbase, st);
+  if (runA && timer) timer->end(kPassA, st);
   if (serr != cudaSuccess) return serr;
   // B
-  if (runB && timer) timer->begin(kPassB + pbase, st);
+  if (runB && timer) timer->begin(kPassB, st);
   if (runB && !static_tile(kTileB))
     tile::k_pass_y<T, false><<<grid_y(tile::k_pass_y<T, false, tile::RtLine<C>>, ysm), kTileThreads, ysm, st>>>(
         t1, t2, g.tmask, g.ny, g.nz, g.nzp, g.nzt, ntask_y, ly, p.twy, ybuf, done);
-  if (runB && timer) timer->end(kPassB + pbase, st);
+  if (runB && timer) timer->end(kPassB, st);
   if (serr != cudaSuccess) return serr;
   // C
   if (runC) {
     const long long ntask = (long long)g.Px * g.Py * L;
-    if (timer) timer->begin(kPassC + pbase, st);
-    bool launched = false;
-    if constexpr (std::is_same<T, float>::value) {
-      cudaError_t e = cudaSuccess;
-      launched = launch_pass_c_static(g, t2, L, p.twzs, p.twzc, p.ghat, st, done, &e);
-      if (launched && e != cudaSuccess) return e;
-    }
+    if (timer) timer->begin(kPassC, st);
+    cudaError_t e = cudaSuccess;
+    const bool launched = launch_pass_c_static(g, t2, L, p.twzs, p.twzc, p.ghat, st, done, &e);
+    if (launched && e != cudaSuccess) return e;
     if (!launched) {
       const int per_warp = g.f * plan_lw<C>(g.pz) * (int)sizeof(C);
       const int wpc = z_warps_per_cta(per_warp);
@@ -179,22 +168,22 @@ cudaError_t launch_block_mvp(const MvpGeom& g, const MvpPrec<T>& p, const typena
       k_pass_c<T><<<grid, wpc * 32, wpc * per_warp, st>>>(t2, L, g.f, g.Px, g.Py, g.nz, g.nzp, g.pz, p.twz, p.ghat,
                                                            g.gperm, done);
     }
-    if (timer) timer->end(kPassC + pbase, st);
+    if (timer) timer->end(kPassC, st);
   }
   // D
-  if (runD && timer) timer->begin(kPassD + pbase, st);
+  if (runD && timer) timer->begin(kPassD, st);
   if (runD && !static_tile(kTileD))
     tile::k_pass_y<T, true><<<grid_y(tile::k_pass_y<T, true, tile::RtLine<C>>, ysm), kTileThreads, ysm, st>>>(
         t2, t1, g.tmask, g.ny, g.nz, g.nzp, g.nzt, ntask_y, ly, p.twy, ybuf, done);
-  if (runD && timer) timer->end(kPassD + pbase, st);
+  if (runD && timer) timer->end(kPassD, st);
   if (serr != cudaSuccess) return serr;
   // E
-  if (runE && timer) timer->begin(kPassE + pbase, st);
+  if (runE && timer) timer->begin(kPassE, st);
   if (runE && !static_tile(kTileE))
     tile::k_pass_e<T><<<xgrid, kTileThreads, xsm, st>>>(
         t1, nfield, xfpg, g.f, g.occ, g.tiles, g.nx, g.ny, g.nz, g.nzp, g.nzt, lx, p.twx, x, ldx, diag, jpre, y, ldy, xbuf,
         done);
-  if (runE && timer) timer->end(kPassE + pbase, st);
+  if (runE && timer) timer->end(kPassE, st);
   if (serr != cudaSuccess) return serr;
   return cudaGetLastError();
 }

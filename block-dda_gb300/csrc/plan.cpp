@@ -153,7 +153,8 @@ constexpr PlanRow kZPlans[] = {
 #include "zplans.inc"
 #undef BDDA_ZPLAN
 };
-// ... the 16-byte (FP64 / double-float) z passes (radices <= 16) ...
+// ... FP64 and double-float z lines of the host line transform (radices <= 16; the MVPs of these precisions run in fixed
+// point, make_fx_plan) ...
 constexpr PlanRow kZWPlans[] = {
 #define BDDA_ZWPLAN(I, N, S, LW, ...) {N, S, LW, {__VA_ARGS__}},
 #include "zwplans.inc"
@@ -426,8 +427,8 @@ extern "C" {
 // transform reads only the first nvalid inputs and takes the rest as zero
 // (the pad slots hold poison values to prove it).  radix[0] > 8 on input: the
 // z-axis schedule, else the x / y one, each for the element width of prec;
-// radix[1] = 1 on input: the complex FP32 schedule in any arithmetic (its
-// Green spectrum is transformed in FP64).  Returns the number of stages, or a
+// radix[1] = 1 on input: the complex FP32 schedule in any arithmetic.  Of 1 to 3 the
+// MVP runs FP32; FP64 and double-float are here to compare with.  Returns the number of stages, or a
 // negative value for an unsupported N.  Radices are written to radix (<= 32).
 int bdda_host_fft_line(int N, int inverse, int prec, int nvalid, double* data, int* radix) {
   if (prec == 4) {
@@ -492,7 +493,7 @@ int bdda_host_fft_line(int N, int inverse, int prec, int nvalid, double* data, i
       const double2 v = s[bdda::skw(i, sh)];
       data[2 * i] = v.x; data[2 * i + 1] = v.y;
     }
-  } else if (prec == 3) {  // the double-float MVP's arithmetic (dfz)
+  } else if (prec == 3) {  // double-float arithmetic without renormalisation (dfz)
     const int sh = bdda::plan_sk<bdda::dfzc>(p);
     std::vector<bdda::dfzc> s(bdda::plan_lw<bdda::dfzc>(p), bdda::cmake(bdda::dfz(1e30), bdda::dfz(1e30))), t(N);
     for (int i = 0; i < N; ++i) {

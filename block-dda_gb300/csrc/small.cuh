@@ -112,22 +112,13 @@ __device__ __forceinline__ dfc m_over(dfc a, dfl b) {
   const dfl q = df_recip(b);
   return cmake(a.x * q, -(a.y * q));
 }
-// a / b; operands are O(1) pivots (no scaling against overflow)
-__device__ __forceinline__ double2 m_div(double2 a, double2 b) {
+// complex FP64 helpers used outside the templated routines
+__device__ __forceinline__ double cabs2(double2 a) { return a.x * a.x + a.y * a.y; }
+// a / b, no scaling against overflow of |b|^2
+__device__ __forceinline__ double2 cdiv(double2 a, double2 b) {
   const double d = b.x * b.x + b.y * b.y;
   return make_double2((a.x * b.x + a.y * b.y) / d, (a.y * b.x - a.x * b.y) / d);
 }
-__device__ __forceinline__ dfc m_div(dfc a, dfc b) {
-  const dfl di = df_recip(b.x * b.x + b.y * b.y);
-  return cmake((a.x * b.x + a.y * b.y) * di, (a.y * b.x - a.x * b.y) * di);
-}
-template <typename R> __device__ __forceinline__ typename SmallMat<R>::M m_one() {
-  return cmake(r_const<R>(1.0f), r_const<R>(0.0f));
-}
-
-// complex FP64 helpers used outside the templated routines
-__device__ __forceinline__ double cabs2(double2 a) { return a.x * a.x + a.y * a.y; }
-__device__ __forceinline__ double2 cdiv(double2 a, double2 b) { return m_div(a, b); }
 __device__ __forceinline__ bool cfinite(double2 a) { return isfinite(a.x) && isfinite(a.y); }
 
 // A Gram matrix as the row kernels leave it: n = 0: reduced, complex FP64 at p; else n partial matrices of type P (FP64 or

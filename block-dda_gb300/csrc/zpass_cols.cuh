@@ -46,7 +46,7 @@ namespace zcol {
 template <class P> constexpr bool supported() { return P::N < kFusedWideMinN && fused_z(P::N, P::nst, P::Rl); }
 
 // The plan of these kernels: the operator's, but two-stage lines take the
-// radices of z_col_radices (mvp.hpp).  The last-radix-major spectrum of a
+// radices that z_col_last_radix (mvp.hpp) gives.  The last-radix-major spectrum of a
 // two-stage line is in natural order (frequency b + R0 i at i R0 + b), so it
 // does not depend on which two radices the kernel uses.
 template <class P, bool TWO = P::nst == 2> struct Own { using type = P; };
