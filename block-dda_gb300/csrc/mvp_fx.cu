@@ -431,7 +431,7 @@ k_fx_c(Val* __restrict__ t2, int L, int Px, int Py, int nz, int nzp, fx::Plan p,
     for (int h = 0; h < halves; ++h) {
 #pragma unroll
       for (int r = 0; r < 3; ++r) {
-        Acc acc;
+        Acc acc = Acc::start<fx::kRowBits<SIX>>();
         const unsigned q = SIX && h ? sown[fc - 3 + r] : sown[r];
 #pragma unroll
         for (int c = 0; c < 3; ++c) acc.mad(g[fx::green_a(r, c)], fx::split(fx::align(e[c], (int)(q >> (8 * c) & 255u))));
@@ -449,7 +449,7 @@ k_fx_c(Val* __restrict__ t2, int L, int Px, int Py, int nz, int nzp, fx::Plan p,
           if (h) acc.sub(t);
           else acc.add(t);
         }
-        const Val v = acc.get();
+        const Val v = acc.get<fx::kRowBits<SIX>>();
         const int b = fx::bits_of(v);
         used[r] |= SIX && h ? 0 : b;
         if constexpr (SIX) used[3 + r] |= h ? b : 0;
@@ -477,7 +477,7 @@ k_fx_c(Val* __restrict__ t2, int L, int Px, int Py, int nz, int nzp, fx::Plan p,
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
       const int t = fx::store_shift((int)__reduce_or_sync(0xffffffffu, (unsigned)ou[c]));
-      if (lane == 3 * (3 * h + c)) eo[(3 * h + c) * eostride] = er > fx::kZeroExp ? er + rsh[c] + p.D - t : fx::kZeroExp;
+      if (lane == 3 * (3 * h + c)) eo[(3 * h + c) * eostride] = er > fx::kZeroExp ? er - fx::kRowBits<SIX> + rsh[c] + p.D - t : fx::kZeroExp;
 #pragma unroll
       for (int k = c; k < fc; k += 3) s[k] = k == 3 * h + c ? t : s[k];
     }

@@ -8,9 +8,9 @@ using namespace bdda;
 
 extern "C" {
 
-// Sum of n products of Q62 factors g (re, im) and values z, those with sub[i] subtracted.
-void fx_products(int n, const long long* g, const long long* z, const int* sub, long long* out) {
-  fx::Acc acc;
+// Sum of n products of Q62 factors g (re, im) and values z, those with sub[i] subtracted, times 2^up (0 or 1).
+void fx_products(int n, const long long* g, const long long* z, const int* sub, int up, long long* out) {
+  fx::Acc acc = up ? fx::Acc::start<1>() : fx::Acc::start<0>();
   for (int i = 0; i < n; ++i) {
     fx::Fac f;
     fx::split(g[2 * i], f.rh, f.rl);
@@ -19,7 +19,7 @@ void fx_products(int n, const long long* g, const long long* z, const int* sub, 
     if (sub[i]) acc.msub(f, s);
     else acc.mad(f, s);
   }
-  const fx::Val v = acc.get();
+  const fx::Val v = up ? acc.get<1>() : acc.get<0>();
   out[0] = v.x;
   out[1] = v.y;
 }
