@@ -13,7 +13,8 @@ namespace bdda {
 
 constexpr int kMaxL = 32;          // largest block width (nrhs) supported
 constexpr int kGramThreads = 256;
-constexpr int kGramSlices = 8;     // threads that share the rows of a sub-tile for one Gram entry, at most
+constexpr int kGramSlices = 8;     // threads that share the rows of a sub-tile for one Gram entry, at most (8 to 32 take the
+                                   // same time; the order of the sums moves loosely converged BiCGSTAB results by rounding)
 constexpr int kGramRows = 32;      // rows per shared-memory sub-tile
 constexpr int kRowRows = 64;       // rows per CTA of the row-transform kernel
 constexpr int kRowThreads = 256;   // its threads: kRowRows rows x 4 column groups

@@ -105,6 +105,9 @@ int bdda_mbt_fft_mvp(bdda_op* op, const double* p_hat, double* q_hat);
  *   diag      f*nocc complex or null (off-diagonal part only)
  *   jpre      f*nocc complex or null (no Jacobi scaling)
  *   stream    cudaStream_t or null (the operator's stream)
+ * Asynchronous on the stream.  The operator has one workspace per precision:
+ * calls of one precision on different streams must be ordered by the caller,
+ * calls of different precisions need not be.
  */
 int bdda_op_mvp_device(bdda_op* op, int prec, const void* x, int ldx, void* y, int ldy, int L,
                        const void* diag, const void* jpre, void* stream);
@@ -116,14 +119,15 @@ int bdda_op_mvp_device(bdda_op* op, int prec, const void* x, int ldx, void* y, i
  * serving loops that must never enter the CUDA allocator (which can
  * synchronise the device).  Same arguments and result as bdda_op_mvp_device
  * for prec BDDA_PREC_FP64 and BDDA_PREC_FP32 (BDDA_PREC_DF64 is rejected with
- * BDDA_ERR_INVALID), but the two FFT workspaces come from a fixed 64 MiB
- * __device__ array; boxes and nrhs whose workspace exceeds it are rejected with
+ * BDDA_ERR_INVALID), but the two FFT workspaces come from a fixed __device__
+ * array: 64 MiB for them, and 11 MiB for the exponents of the FP64 path's
+ * lines; boxes and nrhs whose workspace exceeds 64 MiB are rejected with
  * BDDA_ERR_INVALID and a message.  The array is reserved on a device when the
  * library's code holding it is loaded there -- with CUDA's default lazy module
  * loading, at the first call of this entry point on that device -- and kept
  * until the process exits; that first call also looks up the array's device
  * address.  Make the first call at set-up, before any stream capture and
- * while the device still has 64 MiB free.  The address is kept for the life
+ * while the device still has 75 MiB free.  The address is kept for the life
  * of the process: a cudaDeviceReset after the first call is not supported.
  * All calls share the array: calls that overlap on the GPU race and must be
  * ordered by the caller.
