@@ -107,8 +107,7 @@ template <int D, bool CJ> BDDA_FX_FN Val cmul(Val z, int rh, int rl, int ih, int
   else return {(mr + (cr >> 32) + (1ll << (D - 3))) >> (D - 2), (mi + (ci >> 32) + (1ll << (D - 3))) >> (D - 2)};
 }
 
-// Sum of complex products Fac x Val, scaled as its Val operands over 2^K (get<K> of a sum from start<K>); one shift and
-// rounding at the end.
+// Sum of complex products Fac x Val, scaled as its Val operands; one shift and rounding at the end.
 struct Split { int xh, xl, yh, yl; };
 BDDA_FX_FN Split split(Val v) {
   Split s;
@@ -117,8 +116,7 @@ BDDA_FX_FN Split split(Val v) {
   return s;
 }
 struct Acc {
-  long long cr, ci, mr, mi;
-  template <int K> static BDDA_FX_FN Acc start() { return {1ll << (29 - K), 1ll << (29 - K), 0, 0}; }
+  long long cr = 1ll << 29, ci = 1ll << 29, mr = 0, mi = 0;
   BDDA_FX_FN void mad(const Fac& g, const Split& s) {
     cr += (mw(s.xh, g.rl) + mw(s.xl, g.rh)) - (mw(s.yh, g.il) + mw(s.yl, g.ih));
     mr += mw(s.xh, g.rh) - mw(s.yh, g.ih);
@@ -132,23 +130,24 @@ struct Acc {
     ci -= (mw(s.xh, g.il) + mw(s.xl, g.ih)) + (mw(s.yh, g.rl) + mw(s.yl, g.rh));
     mi -= mw(s.xh, g.ih) + mw(s.yh, g.rh);
   }
-  BDDA_FX_FN void add(const Acc& o) { cr += o.cr; ci += o.ci; mr += o.mr; mi += o.mi; }
-  BDDA_FX_FN void sub(const Acc& o) { cr -= o.cr; ci -= o.ci; mr -= o.mr; mi -= o.mi; }
-  template <int K> BDDA_FX_FN Val get() const { return {shl(mr, 2 + K) + (cr >> (30 - K)), shl(mi, 2 + K) + (ci >> (30 - K))}; }
+  BDDA_FX_FN Val get() const { return {shl(mr, 2) + (cr >> 30), shl(mi, 2) + (ci >> 30)}; }
+  // this sum plus or minus another one (of no rounding half), whose middle sums together may pass 2^63
+  BDDA_FX_FN Val get(const Acc& o, bool sub) const {
+    const long long hr = o.cr >> 1, hi = o.ci >> 1;
+    return {shl(sub ? mr - o.mr : mr + o.mr, 2) + (((cr >> 1) + (sub ? -hr : hr)) >> 29),
+            shl(sub ? mi - o.mi : mi + o.mi, 2) + (((ci >> 1) + (sub ? -hi : hi)) >> 29)};
+  }
 };
 
 // Index of the spectrum components that couple component c to row r, r and c < 3: of the symmetric block A (xx xy xz yy yz
 // zz), and with f = 6, [A B; -B A], of the antisymmetric B (xy xz yz, -1 on its diagonal; subtracted where r > c).
 BDDA_FX_FN constexpr int green_a(int r, int c) { return r + c + (r != 0 && c != 0 ? 1 : 0); }
 BDDA_FX_FN constexpr int green_b(int r, int c) { return r == c ? -1 : 5 + r + c; }
-// Bits that a spectrum component stays below 1, and that values are shifted for the products at least: with the 3 (SIX: 5)
-// terms of a row the middle sums of Acc stay below 7.3 (6.1) 2^60 and its result below 2^62.  Both cost precision, the
-// first against the elements far below a line's peak: SIX with 3 and 2 bits had errors of 2.8e-16 (N=568, extended
-// precision) where 2 and 2, 1 and 3 have 1.7e-16.
-template <bool SIX> constexpr int kGreenBits = SIX ? 2 : 1;
-template <bool SIX> constexpr int kProductBits = SIX ? 2 : 1;
-// Bits that a row's sum is scaled up by, as far as its bound allows (5 terms of 2^60 by kGreenBits).
-template <bool SIX> constexpr int kRowBits = SIX ? 1 : 0;
+// Bits that a spectrum component stays below 1, and that values are shifted for the products at least: the middle sums of
+// three terms stay below 7.3 2^60, of f = 6's other two below 4.9, and a row of five below 5 2^60, which the shift to the
+// inverse transform's headroom takes.  Each bit costs precision, the first against elements far below a line's peak: with
+// 3 and 2 bits f = 6 had errors of 2.8e-16 (N=568, extended precision), with 2 and 2 1.7e-16.
+constexpr int kGreenBits = 1, kProductBits = 1;
 
 // ---- butterflies: forward exp(-2 pi i / R), INV exp(+2 pi i / R) --------------
 constexpr long long kS60 = 3993837246235628775ll;   // sin 60, Q62

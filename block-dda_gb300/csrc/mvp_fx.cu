@@ -401,7 +401,7 @@ k_fx_c(Val* __restrict__ t2, int L, int Px, int Py, int nz, int nzp, fx::Plan p,
   int er = max(own, oth);
   er = max(er, max(__shfl_down_sync(0xffffffffu, er, 1), __shfl_down_sync(0xffffffffu, er, 2)));
   er = __shfl_sync(0xffffffffu, er, lane - tc);
-  if (er > fx::kZeroExp) er += fx::kProductBits<SIX>;
+  if (er > fx::kZeroExp) er += fx::kProductBits;
   auto shifts = [&](int e) {
     const unsigned s = (unsigned)min(max(er - e, 1), 62) << (8 * tc);
     return s | __shfl_down_sync(0xffffffffu, s, 1) | __shfl_down_sync(0xffffffffu, s, 2);
@@ -431,10 +431,11 @@ k_fx_c(Val* __restrict__ t2, int L, int Px, int Py, int nz, int nzp, fx::Plan p,
     for (int h = 0; h < halves; ++h) {
 #pragma unroll
       for (int r = 0; r < 3; ++r) {
-        Acc acc = Acc::start<fx::kRowBits<SIX>>();
+        Acc acc;
         const unsigned q = SIX && h ? sown[fc - 3 + r] : sown[r];
 #pragma unroll
         for (int c = 0; c < 3; ++c) acc.mad(g[fx::green_a(r, c)], fx::split(fx::align(e[c], (int)(q >> (8 * c) & 255u))));
+        Val v;
         if constexpr (SIX) {  // E' = A E + B M, M' = A M - B E
           Acc t{0, 0, 0, 0};
           const unsigned u = h ? soth[fc - 3 + r] : soth[r];
@@ -446,10 +447,10 @@ k_fx_c(Val* __restrict__ t2, int L, int Px, int Py, int nz, int nzp, fx::Plan p,
             if (r > c) t.msub(g[i], s);
             else t.mad(g[i], s);
           }
-          if (h) acc.sub(t);
-          else acc.add(t);
+          v = acc.get(t, h != 0);
+        } else {
+          v = acc.get();
         }
-        const Val v = acc.get<fx::kRowBits<SIX>>();
         const int b = fx::bits_of(v);
         used[r] |= SIX && h ? 0 : b;
         if constexpr (SIX) used[3 + r] |= h ? b : 0;
@@ -477,7 +478,7 @@ k_fx_c(Val* __restrict__ t2, int L, int Px, int Py, int nz, int nzp, fx::Plan p,
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
       const int t = fx::store_shift((int)__reduce_or_sync(0xffffffffu, (unsigned)ou[c]));
-      if (lane == 3 * (3 * h + c)) eo[(3 * h + c) * eostride] = er > fx::kZeroExp ? er - fx::kRowBits<SIX> + rsh[c] + p.D - t : fx::kZeroExp;
+      if (lane == 3 * (3 * h + c)) eo[(3 * h + c) * eostride] = er > fx::kZeroExp ? er + rsh[c] + p.D - t : fx::kZeroExp;
 #pragma unroll
       for (int k = c; k < fc; k += 3) s[k] = k == 3 * h + c ? t : s[k];
     }
@@ -585,7 +586,7 @@ k_fx_pack(const double2* __restrict__ g, Fac* __restrict__ out, int* __restrict_
   }
   if (lane < NC && m[0] * scale > 0.0) {
     frexp(m[0] * scale, &e);  // below 2^e
-    e += fx::kGreenBits<NC == 9>;
+    e += fx::kGreenBits;
     mul = ldexp(scale, min(62 - e, 1000));
     more = ldexp(1.0, max(62 - e - 1000, 0));
   }

@@ -8,18 +8,20 @@ using namespace bdda;
 
 extern "C" {
 
-// Sum of n products of Q62 factors g (re, im) and values z, those with sub[i] subtracted, times 2^up (0 or 1).
-void fx_products(int n, const long long* g, const long long* z, const int* sub, int up, long long* out) {
-  fx::Acc acc = up ? fx::Acc::start<1>() : fx::Acc::start<0>();
+// Sum of n products of Q62 factors g (re, im) and values z, those with sub[i] subtracted; from the fourth on in a sum of
+// their own that is added at the end (minus: subtracted).
+void fx_products(int n, const long long* g, const long long* z, const int* sub, int minus, long long* out) {
+  fx::Acc acc, rest{0, 0, 0, 0};
   for (int i = 0; i < n; ++i) {
     fx::Fac f;
     fx::split(g[2 * i], f.rh, f.rl);
     fx::split(g[2 * i + 1], f.ih, f.il);
     const fx::Split s = fx::split(fx::Val{z[2 * i], z[2 * i + 1]});
-    if (sub[i]) acc.msub(f, s);
-    else acc.mad(f, s);
+    fx::Acc& a = i < 3 ? acc : rest;
+    if (sub[i]) a.msub(f, s);
+    else a.mad(f, s);
   }
-  const fx::Val v = up ? acc.get<1>() : acc.get<0>();
+  const fx::Val v = n > 3 ? acc.get(rest, minus != 0) : acc.get();
   out[0] = v.x;
   out[1] = v.y;
 }

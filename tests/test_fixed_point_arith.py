@@ -45,10 +45,11 @@ def test_products_at_the_ends_of_the_low_half(fx, low, sub):
             assert abs(int(out[1]) * 2 ** 62 - im) <= 5 * 2 ** 62
 
 
-# The largest terms of a row: 3 with |re| + |im| <= 2^61 and |z| <= 2^61, or 5 with 2^60 and 2^60; no sum may wrap.
-# f = 6 scales its sums up by one bit.
-@pytest.mark.parametrize("terms, gbits, zbits, up", [(3, 61, 61, 0), (5, 60, 60, 1)])
-def test_largest_rows_do_not_wrap(fx, terms, gbits, zbits, up):
+# The largest terms of a row: 3 (f = 6: and 2 in a sum of their own) with |re| + |im| <= 2^61 and |z| <= 2^61; no sum may
+# wrap.
+@pytest.mark.parametrize("terms, minus", [(3, 0), (5, 0), (5, 1)])
+def test_largest_rows_do_not_wrap(fx, terms, minus):
+    gbits = zbits = 61
     rng = np.random.default_rng(terms)
     for _ in range(400):
         g, z, s = [], [], []
@@ -61,12 +62,12 @@ def test_largest_rows_do_not_wrap(fx, terms, gbits, zbits, up):
             for i in range(len(v)):
                 v[i] = ((v[i] >> 32 << 32) | int(rng.choice([0x7FFFFFFF, 0x80000001, v[i] & 0xFFFFFFFF]))) * int(rng.choice([-1, 1]))
         out = np.zeros(2, np.int64)
-        fx.fx_products(terms, _ll(g), _ll(z), np.array(s, np.int32).ctypes.data_as(ct.POINTER(ct.c_int)), up, _ll(out))
-        re = sum((-1 if s[i] else 1) * (g[2 * i] * z[2 * i] - g[2 * i + 1] * z[2 * i + 1]) for i in range(terms))
-        im = sum((-1 if s[i] else 1) * (g[2 * i] * z[2 * i + 1] + g[2 * i + 1] * z[2 * i]) for i in range(terms))
-        tol = (2 * terms + 1) * 2 ** (62 + up)
-        assert abs(int(out[0]) * 2 ** 62 - re * 2 ** up) <= tol
-        assert abs(int(out[1]) * 2 ** 62 - im * 2 ** up) <= tol
+        fx.fx_products(terms, _ll(g), _ll(z), np.array(s, np.int32).ctypes.data_as(ct.POINTER(ct.c_int)), minus, _ll(out))
+        sg = [(-1 if s[i] else 1) * (-1 if minus and i > 2 else 1) for i in range(terms)]
+        re = sum(sg[i] * (g[2 * i] * z[2 * i] - g[2 * i + 1] * z[2 * i + 1]) for i in range(terms))
+        im = sum(sg[i] * (g[2 * i] * z[2 * i + 1] + g[2 * i + 1] * z[2 * i]) for i in range(terms))
+        assert abs(int(out[0]) * 2 ** 62 - re) <= (2 * terms + 1) * 2 ** 62
+        assert abs(int(out[1]) * 2 ** 62 - im) <= (2 * terms + 1) * 2 ** 62
 
 
 # Elements are shifted right by e + s - ex: e the largest exponent of their line, ex their own, s from 1 to 64.
